@@ -24,6 +24,7 @@
 #include "edgelist.cuh"
 #include "eigen.cuh"
 #include "handle.cuh"
+#include "pool.cuh"
 #include "ppr_batch.cuh"
 #include "solver.cuh"
 
@@ -187,10 +188,9 @@ void destroy(prg_graph *h);
 int32_t create_from_host(uint32_t n, uint64_t m, const uint32_t *from, const uint32_t *to, const double *w,
                          int32_t directed, prg_graph **out, int relabel = -1) {
     if (!ensure_pool_config()) return fail(PRG_ERR_CUDA, "cuda: no usable device");
-    cudaStream_t s;
-    PRG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    cudaStream_t s = prg::stream_acquire();
     if (m > 0xFFFFFFFFull) {
-        cudaStreamDestroy(s);
+        prg::stream_release(s);
         return fail(PRG_ERR_INTERNAL, "ecount overflows u32");
     }
     if (m >= prg::kStreamMinEdges && !(w && directed)) {
@@ -213,8 +213,7 @@ int32_t create_from_host(uint32_t n, uint64_t m, const uint32_t *from, const uin
             destroy(h);  // what was built, and the stream
             return fail(PRG_ERR_VERTEX_OUT_OF_RANGE, range_message(mx, n));
         }
-        cudaStreamSynchronize(s);
-        cudaStreamDestroy(s);
+        prg::stream_release(s);
         return rc;
     }
     uint32_t *d_f = nullptr, *d_t = nullptr;
@@ -235,8 +234,7 @@ int32_t create_from_host(uint32_t n, uint64_t m, const uint32_t *from, const uin
     cudaFreeAsync(d_t, s);
     if (d_w) cudaFreeAsync(d_w, s);
     if (rc != PRG_OK) {
-        cudaStreamSynchronize(s);
-        cudaStreamDestroy(s);
+        prg::stream_release(s);
     }
     return rc;
 }
@@ -276,8 +274,7 @@ void destroy(prg_graph *h) {
     f(h->d_reset);
     f(h->d_out);
     f(h->d_start);
-    cudaStreamSynchronize(s);
-    cudaStreamDestroy(s);
+    prg::stream_release(s);
     delete h;
 }
 
@@ -897,10 +894,9 @@ int32_t prg_graph_create_device(uint32_t n, uint64_t m, const uint32_t *d_from, 
     if (!out) return fail(PRG_ERR_INVALID_ARGUMENT, "null output handle");
     *out = nullptr;
     if (!ensure_pool_config()) return fail(PRG_ERR_CUDA, "cuda: no usable device");
-    cudaStream_t s;
-    PRG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    cudaStream_t s = prg::stream_acquire();
     int32_t rc = create_from_device(n, m, d_from, d_to, d_weights, directed, s, out);
-    if (rc != PRG_OK) cudaStreamDestroy(s);
+    if (rc != PRG_OK) prg::stream_release(s);
     else prepare_handle(*out);
     return rc;
     PRG_GUARD_END
@@ -938,8 +934,7 @@ int32_t prg_parse_edgelist(const char *text, uint64_t len, uint32_t *from, uint3
     if (m) *m = 0;
     if (n) *n = 0;
     if (!ensure_pool_config()) return fail(PRG_ERR_CUDA, "cuda: no usable device");
-    cudaStream_t s;
-    PRG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    cudaStream_t s = prg::stream_acquire();
     prg::el::ParseResult r;
     int32_t rc = PRG_OK;
     try {
@@ -963,11 +958,10 @@ int32_t prg_parse_edgelist(const char *text, uint64_t len, uint32_t *from, uint3
         PRG_CUDA(cudaStreamSynchronize(s));
     } catch (...) {
         prg::el::free_result(r, s);
-        cudaStreamSynchronize(s);
-        cudaStreamDestroy(s);
+        prg::stream_release(s);
         throw;
     }
-    cudaStreamDestroy(s);
+    prg::stream_release(s);
     return rc;
     PRG_GUARD_END
 }
@@ -981,8 +975,7 @@ int32_t prg_read_edgelist(const char *text, uint64_t len, prg_graph **out, uint3
     if (m) *m = 0;
     if (n) *n = 0;
     if (!ensure_pool_config()) return fail(PRG_ERR_CUDA, "cuda: no usable device");
-    cudaStream_t s;
-    PRG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    cudaStream_t s = prg::stream_acquire();
     prg::el::ParseResult r;
     int32_t rc = PRG_OK;
     try {
@@ -1003,11 +996,10 @@ int32_t prg_read_edgelist(const char *text, uint64_t len, prg_graph **out, uint3
         PRG_CUDA(cudaStreamSynchronize(s));
     } catch (...) {
         prg::el::free_result(r, s);
-        cudaStreamSynchronize(s);
-        cudaStreamDestroy(s);
+        prg::stream_release(s);
         throw;
     }
-    cudaStreamDestroy(s);
+    prg::stream_release(s);
     return rc;
     PRG_GUARD_END
 }

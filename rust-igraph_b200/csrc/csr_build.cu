@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "graph.cuh"
+#include "pool.cuh"
 #include "prims.cuh"
 
 namespace prg {
@@ -871,8 +872,7 @@ bool build_graph_host(DeviceGraph &g, const uint32_t *h_from, const uint32_t *h_
     uint32_t *ka = dalloc<uint32_t>(chunk_arcs, s), *va = dalloc<uint32_t>(chunk_arcs, s);
     uint32_t *kb = dalloc<uint32_t>(chunk_arcs, s), *vb = dalloc<uint32_t>(chunk_arcs, s);
 
-    cudaStream_t cs;
-    PRG_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
+    cudaStream_t cs = stream_acquire();
     std::vector<cudaEvent_t> ev(nchunks + 1);
     for (cudaEvent_t &e : ev) PRG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     // the copy stream starts once the allocations above are usable
@@ -909,9 +909,8 @@ bool build_graph_host(DeviceGraph &g, const uint32_t *h_from, const uint32_t *h_
     uint32_t mx = 0;
     PRG_CUDA(cudaMemcpyAsync(&mx, d_mx, 4, cudaMemcpyDeviceToHost, s));
     PRG_CUDA(cudaStreamSynchronize(s));
-    PRG_CUDA(cudaStreamSynchronize(cs));
     for (cudaEvent_t &e : ev) cudaEventDestroy(e);
-    cudaStreamDestroy(cs);
+    stream_release(cs);
     dfree(ka, s);
     dfree(va, s);
     dfree(kb, s);

@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "eigen.cuh"
+#include "pool.cuh"
 #include "prims.cuh"
 #include "solver.cuh"
 
@@ -544,7 +545,8 @@ Result eigenvector_centrality(const DeviceGraph &g, Workspace &ws, double *d_out
     double4 *recs = alloc<double4>(std::max(grid, kNB), s), *part = alloc<double4>(kNB, s);
     double4 *pvrec = alloc<double4>(kNB, s);
     State *d_st = alloc<State>(1, s), *h_st = nullptr;
-    PRG_CUDA(cudaMallocHost((void **)&h_st, 2 * sizeof(State)));
+    static_assert(2 * sizeof(State) <= kSlabBytes, "iteration state slab");
+    h_st = static_cast<State *>(pinned_acquire());
     try {
         State init;
         std::memset(&init, 0, sizeof(init));
@@ -589,10 +591,10 @@ Result eigenvector_centrality(const DeviceGraph &g, Workspace &ws, double *d_out
         PRG_CUDA(cudaStreamSynchronize(s));
     } catch (...) {
         cudaStreamSynchronize(s);
-        cudaFreeHost(h_st);
+        pinned_release(h_st);
         throw;
     }
-    cudaFreeHost(h_st);
+    pinned_release(h_st);
     release(x[0], s);
     release(x[1], s);
     release(recs, s);
@@ -672,7 +674,8 @@ Result infomap_flow(const DeviceGraph &g, Workspace &ws, const double *d_t, doub
     double4 *recs = alloc<double4>(std::max(grid, kNB), s), *spart = alloc<double4>(kNB, s);
     double4 *dpart = alloc<double4>(kNB, s);
     State *d_st = alloc<State>(1, s), *h_st = nullptr;
-    PRG_CUDA(cudaMallocHost((void **)&h_st, 2 * sizeof(State)));
+    static_assert(2 * sizeof(State) <= kSlabBytes, "iteration state slab");
+    h_st = static_cast<State *>(pinned_acquire());
     try {
         State init;
         std::memset(&init, 0, sizeof(init));
@@ -696,10 +699,10 @@ Result infomap_flow(const DeviceGraph &g, Workspace &ws, const double *d_t, doub
         PRG_CUDA(cudaStreamSynchronize(s));
     } catch (...) {
         cudaStreamSynchronize(s);
-        cudaFreeHost(h_st);
+        pinned_release(h_st);
         throw;
     }
-    cudaFreeHost(h_st);
+    pinned_release(h_st);
     release(pr[0], s);
     release(pr[1], s);
     release(xt, s);
@@ -728,7 +731,8 @@ Result hits_directed(const DeviceGraph &g, Workspace &ws, const DeviceGraph &rev
     double4 *rin = alloc<double4>(std::max(gin, kNB), s), *rout = alloc<double4>(std::max(gout, kNB), s);
     double4 *part = alloc<double4>(kNB, s), *pvrec = alloc<double4>(kNB, s);
     State *d_st = alloc<State>(1, s), *h_st = nullptr;
-    PRG_CUDA(cudaMallocHost((void **)&h_st, 2 * sizeof(State)));
+    static_assert(2 * sizeof(State) <= kSlabBytes, "iteration state slab");
+    h_st = static_cast<State *>(pinned_acquire());
     try {
         State init;
         std::memset(&init, 0, sizeof(init));
@@ -769,10 +773,10 @@ Result hits_directed(const DeviceGraph &g, Workspace &ws, const DeviceGraph &rev
         PRG_CUDA(cudaStreamSynchronize(s));
     } catch (...) {
         cudaStreamSynchronize(s);
-        cudaFreeHost(h_st);
+        pinned_release(h_st);
         throw;
     }
-    cudaFreeHost(h_st);
+    pinned_release(h_st);
     release(h[0], s);
     release(h[1], s);
     release(tmp, s);

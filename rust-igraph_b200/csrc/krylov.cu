@@ -35,6 +35,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "pool.cuh"
 #include "solver.cuh"
 
 namespace prg {
@@ -113,7 +114,7 @@ void krylov_free(KrylovWs *&k, cudaStream_t s) {
     kbuf_free(k->d, s);
     for (double4 **q : {&k->part1, &k->part2, &k->part3, &k->part4, &k->part5}) kfree(*q, s);
     kfree(k->st, s);
-    if (k->h_st) cudaFreeHost(k->h_st);
+    if (k->h_st) pinned_release(k->h_st);
     for (cudaEvent_t &e : k->ev)
         if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : k->mv_ev) cudaEventDestroy(e);
@@ -130,7 +131,8 @@ static KrylovWs &krylov_ws(Workspace &ws, const DeviceGraph &g, unsigned spmv_gr
         const unsigned np = std::max(kVB, spmv_grid);
         for (double4 **q : {&k.part1, &k.part2, &k.part3, &k.part4, &k.part5}) kalloc(*q, np, s);
         kalloc(k.st, 1, s);
-        PRG_CUDA(cudaMallocHost((void **)&k.h_st, 2 * sizeof(KState)));
+        static_assert(2 * sizeof(KState) <= kSlabBytes, "Krylov state slab");
+        k.h_st = static_cast<KState *>(pinned_acquire());
         for (cudaEvent_t &e : k.ev) PRG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     return *ws.kry;

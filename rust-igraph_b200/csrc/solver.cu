@@ -20,6 +20,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "pool.cuh"
 #include "solver.cuh"
 
 namespace prg {
@@ -37,6 +38,7 @@ static void wfree(T *&p, cudaStream_t s) {
 constexpr uint32_t kPrepParts = 148u * 4u;
 
 void workspace_free(Workspace &ws, cudaStream_t s) {
+    if (ws.h_ctl || ws.kry) cudaStreamSynchronize(s);  // no copy into a pinned slab is left in flight
     for (auto &kv : ws.graphs) cudaGraphExecDestroy(kv.second);
     ws.graphs.clear();
     krylov_free(ws.kry, s);
@@ -56,7 +58,7 @@ void workspace_free(Workspace &ws, cudaStream_t s) {
     wfree(ws.hub_rec, s);
     wfree(ws.chunk_part, s);
     wfree(ws.hub_ticket, s);
-    if (ws.h_ctl) cudaFreeHost(ws.h_ctl);
+    if (ws.h_ctl) pinned_release(ws.h_ctl);
     ws.h_ctl = nullptr;
     for (cudaEvent_t *e : {&ws.ev0, &ws.ev1, &ws.eva, &ws.evb}) {
         if (*e) cudaEventDestroy(*e);
@@ -117,7 +119,8 @@ void workspace_ensure(Workspace &ws, const DeviceGraph &g, cudaStream_t s) {
     walloc(ws.hub_ticket, g.nhub, s);
     PRG_CUDA(cudaMemsetAsync(ws.hub_ticket, 0, std::max<uint64_t>(g.nhub, 1) * 4, s));
     PRG_CUDA(cudaMemsetAsync(ws.hub_rec, 0, std::max<uint64_t>(g.nhub, 1) * sizeof(double4), s));
-    PRG_CUDA(cudaMallocHost((void **)&ws.h_ctl, sizeof(Ctl)));
+    static_assert(sizeof(Ctl) <= kSlabBytes, "control block slab");
+    ws.h_ctl = static_cast<Ctl *>(pinned_acquire());
     PRG_CUDA(cudaEventCreate(&ws.ev0));
     PRG_CUDA(cudaEventCreate(&ws.ev1));
     PRG_CUDA(cudaEventCreate(&ws.eva));
