@@ -144,6 +144,7 @@ static prg_graph *new_handle(uint32_t n, uint64_t m, int32_t directed, cudaStrea
     h->g.seg_hot64 = t.seg_hot64;
     h->g.seg_plain64 = t.seg_plain64;
     h->g.seg_eig64 = t.seg_eig64;
+    h->g.resident = t.resident;
     h->g.seg_prefetch = t.seg_prefetch;
     h->g.seg_threads = t.seg_threads;
     h->g.seg_pipe = t.seg_pipe;
@@ -378,6 +379,9 @@ int32_t dropin(uint32_t n, uint64_t m, const uint32_t *from, const uint32_t *to,
     }                                                                   \
     catch (const prg::CudaError &e) {                                   \
         return from_cuda(e);                                            \
+    }                                                                   \
+    catch (const prg::TimeoutError &e) {                                \
+        return fail(PRG_ERR_TIMEOUT, e.what);                           \
     }                                                                   \
     catch (const std::bad_alloc &) {                                    \
         return fail(PRG_ERR_OUT_OF_MEMORY, "host: out of memory");      \
@@ -1403,6 +1407,9 @@ int32_t prg_set_tuning(const char *key, int64_t value) {
     } else if (k == "seg_eig64") {
         if (value > 1) return fail(PRG_ERR_INVALID_ARGUMENT, "seg_eig64 must be 0 or 1");
         t.seg_eig64 = (uint32_t)value;
+    } else if (k == "resident") {
+        if (value > 1) return fail(PRG_ERR_INVALID_ARGUMENT, "resident must be 0 or 1");
+        t.resident = (uint32_t)value;
     } else if (k == "seg_threads") {
         if (value != 1024 && value != 768 && value != 512)
             return fail(PRG_ERR_INVALID_ARGUMENT, "seg_threads must be 1024, 768 or 512");

@@ -524,6 +524,37 @@ static double seed(const DeviceGraph &g, bool keep_sign, bool neg, double *x, do
     return norm;
 }
 
+// The iterations and the Rayleigh quotient as one block-resident launch from
+// x[0], the last iterate left there; false (nothing done) when the device
+// cannot hold the grid at once.
+static bool resident_iterations(const DeviceGraph &g, Workspace &ws, const ResPlan &p, double *const (&x)[2],
+                                double shift, double eps, uint32_t max_iter, Result &r, cudaStream_t s) {
+    ResArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.row_ptr = g.row_ptr;
+    a.col = g.col;
+    a.w64 = g.weighted ? g.w64 : nullptr;
+    a.start = x[0];
+    a.x_out = x[0];
+    a.xt[0] = x[1];
+    a.xt[1] = ws.x64[0];
+    a.total = g.arcs + (uint64_t)p.alpha * g.n;
+    a.n = g.n;
+    a.alpha = p.alpha;
+    a.l1hot = g.perm != nullptr && g.l1_hot64 ? kResL1Hot : 0xFFFFFFFFu;
+    a.max_iter = max_iter;
+    a.thr = eps;
+    a.shift = shift;
+    resident_scratch(ws, p, a, s);
+    PRG_CUDA(cudaMemsetAsync(ws.ctl, 0, sizeof(Ctl), s));
+    if (!launch_resident(RES_EIG, p, a, s)) return false;
+    read_ctl(ws, s);
+    if (ws.h_ctl->status != 0) throw TimeoutError{"eigenvector iteration: a grid barrier timed out"};
+    r.iterations = ws.h_ctl->iters;
+    r.eigenvalue = ws.h_ctl->dsum[1] > 0.0 ? ws.h_ctl->dsum[0] / ws.h_ctl->dsum[1] : 0.0;
+    return true;
+}
+
 Result eigenvector_centrality(const DeviceGraph &g, Workspace &ws, double *d_out, cudaStream_t s,
                               bool strength_seed, double eps) {
     EigOpts o;
@@ -537,7 +568,8 @@ Result eigenvector_centrality(const DeviceGraph &g, Workspace &ws, double *d_out
     const double eps = o.eps;
     Result r;
     const uint32_t n = g.n;
-    workspace_ensure(ws, g, s);
+    const ResPlan rp = o.negative ? ResPlan{} : resident_plan(ws, g, RES_EIG, s);
+    workspace_ensure(ws, g, s, rp.grid == 0);
     PRG_CUDA(cudaMemsetAsync(ws.hub_ticket, 0, std::max<uint64_t>(g.nhub, 1) * 4, s));
     const Product pr{&g, &ws};
     const unsigned grid = ws.cfg[MODE_EIG64].grid;
@@ -561,7 +593,10 @@ Result eigenvector_centrality(const DeviceGraph &g, Workspace &ws, double *d_out
             fill_kernel<<<kNB, kNT, 0, s>>>(x[0], n, 1.0);
             PRG_CUDA(cudaGetLastError());
         }
-        run_until_done(d_st, h_st, init.max_iter, s, [&](uint32_t it) {
+        const double *xf = nullptr;
+        if (rp.grid && resident_iterations(g, ws, rp, x, shift, eps, init.max_iter, r, s)) xf = x[0];
+        else workspace_ensure(ws, g, s);
+        if (!xf) run_until_done(d_st, h_st, init.max_iter, s, [&](uint32_t it) {
             const int q = (int)(it & 1u);
             product(pr, x[q], x[q ^ 1], shift, recs, &d_st->done, s);
             if (o.negative) {
@@ -574,10 +609,12 @@ Result eigenvector_centrality(const DeviceGraph &g, Workspace &ws, double *d_out
             check_kernel<<<1, 256, 0, s>>>(part, kNB, d_st, q ^ 1);
             PRG_CUDA(cudaGetLastError());
         });
-        r.iterations = h_st[0].iters;
-        const double *xf = h_st[0].iters ? x[h_st[0].final_buf] : x[0];
-        double *other = xf == x[0] ? x[1] : x[0];
-        r.eigenvalue = rayleigh(pr, xf, other, recs, s);
+        if (!xf) {
+            r.iterations = h_st[0].iters;
+            xf = h_st[0].iters ? x[h_st[0].final_buf] : x[0];
+            double *other = xf == x[0] ? x[1] : x[0];
+            r.eigenvalue = rayleigh(pr, xf, other, recs, s);
+        }
         if (o.zero_fallback && !o.negative && r.eigenvalue <= 1e-12) {
             // eigenvector.rs:695-699: a (numerically) nilpotent matrix gives zeros
             r.eigenvalue = 0.0;

@@ -55,6 +55,9 @@ struct DeviceGraph {
     uint32_t seg_plain64 = 1;
     // ... and the adjacency product of the eigenvector and HITS iterations
     uint32_t seg_eig64 = 1;
+    // graphs whose arcs fit the SMs' shared memory: FP64 power and eigenvector
+    // iterations as one persistent launch (resident.cu)
+    uint32_t resident = 1;
     uint32_t seg_prefetch = 1;  // segmented passes: prefetch each warp's next index tile into L2
     // their tile kernel: threads of its one block per SM (1024, 768 or 512)
     // and, in the FP32 matvec, whether each warp loads its next tile while
@@ -105,6 +108,7 @@ struct Tuning {
     uint32_t seg_plain64 = 1;    // unweighted graphs: tile-segmented FP64 power step and Krylov matvec
                                  // (0 = row-block kernels)
     uint32_t seg_eig64 = 1;      // unweighted graphs: tile-segmented eigenvector / HITS product
+    uint32_t resident = 1;       // small graphs: block-resident persistent iterations (resident.cu)
     uint32_t seg_prefetch = 1;   // segmented passes: L2 prefetch of each warp's next index tile
     uint32_t seg_threads = 1024;  // segmented passes: tile-kernel block size (1024, 768 or 512)
     uint32_t seg_pipe = 1;        // segmented FP32 matvec: load each warp's next tile ahead

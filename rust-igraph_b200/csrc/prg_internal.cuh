@@ -71,4 +71,8 @@ struct CudaError {
     const char *what;
     CudaError(cudaError_t e, const char *w) : err(e), what(w) {}
 };
+// A bounded device wait expired (PRG_ERR_TIMEOUT).
+struct TimeoutError {
+    const char *what;
+};
 }  // namespace prg

@@ -1,0 +1,52 @@
+// resident.cuh — launch interface of the block-resident persistent iteration
+// (resident.cu) for graphs whose arcs fit the SMs' shared memory.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "graph.cuh"
+
+namespace prg {
+
+constexpr uint32_t kResL1Hot = 8192;
+
+enum ResKind : int {
+    RES_POWER = 0,  // damped FP64 power iteration (uniform or personalised teleport)
+    RES_EIG = 1,    // max-normalised iteration x' = (shift I + A) x / max
+};
+
+struct ResPlan {
+    unsigned grid = 0;   // 0: the graph does not fit, use the other kernels
+    size_t smem = 0;     // dynamic shared memory per block
+    bool stream = false; // column indices and weights are read from memory every iteration, not kept in shared memory
+    uint32_t alpha = 0;  // a row weighs as much as alpha arcs in the split over the blocks
+};
+
+struct ResArgs {
+    const uint32_t *row_ptr;
+    const uint32_t *col;
+    const double *w64;    // null: unweighted
+    const double *dval;   // RES_POWER
+    const double *t64;    // RES_POWER: teleport vector (null: uniform)
+    const double *start;  // start vector (RES_POWER: null = the teleport vector; not an xt[])
+    double *x_out;        // the last iterate; RES_EIG: the start itself
+    double *xt[2];        // gathered vectors, rewritten in turn (RES_EIG: xt[0] is not the start)
+    double2 *rec;         // 2 x grid records
+    uint32_t *bar;        // arrival counter, zero at launch
+    Ctl *ctl;             // out: iters, diff, done, status; RES_EIG: dsum = (x.Ax, x.x)
+    uint64_t total;       // arcs + alpha n
+    uint32_t n, alpha, max_iter;
+    uint32_t l1hot;       // sources at or above this id are gathered without L1 allocation
+    double damping, thr, shift;
+};
+
+// Launch shape for graph g, or grid = 0 where it does not apply (reads the
+// rows' split back from the device when the sizes alone do not decide).
+ResPlan res_plan(const DeviceGraph &g, int kind, cudaStream_t s);
+// Bytes of scratch the launch needs (records and arrival counter).
+size_t res_scratch_bytes(const ResPlan &p);
+// Iterates until the stop rule holds or max_iter iterations ran; false when
+// the device cannot hold the grid at once (nothing was launched).
+bool launch_resident(int kind, const ResPlan &p, const ResArgs &a, cudaStream_t s);
+
+}  // namespace prg

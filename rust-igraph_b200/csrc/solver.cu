@@ -31,7 +31,7 @@ static void walloc(T *&p, uint64_t count, cudaStream_t s) {
 }
 template <class T>
 static void wfree(T *&p, cudaStream_t s) {
-    if (p) cudaFreeAsync(p, s);
+    if (p) cudaFreeAsync((void *)p, s);
     p = nullptr;
 }
 
@@ -58,6 +58,8 @@ void workspace_free(Workspace &ws, cudaStream_t s) {
     wfree(ws.hub_rec, s);
     wfree(ws.chunk_part, s);
     wfree(ws.hub_ticket, s);
+    wfree(ws.res_buf, s);
+    ws.res_bytes = 0;
     if (ws.h_ctl) pinned_release(ws.h_ctl);
     ws.h_ctl = nullptr;
     for (cudaEvent_t *e : {&ws.ev0, &ws.ev1, &ws.eva, &ws.evb}) {
@@ -67,14 +69,23 @@ void workspace_free(Workspace &ws, cudaStream_t s) {
     ws.ready = false;
 }
 
-void workspace_ensure(Workspace &ws, const DeviceGraph &g, cudaStream_t s) {
+// The tile-segmented passes' index, when this graph uses one.
+static void seg_ensure(Workspace &ws, const DeviceGraph &g, cudaStream_t s) {
+    const bool any = g.seg_kry32 != 0 || g.seg_res64 != 0 || g.seg_plain64 != 0 || g.seg_eig64 != 0;
+    if (!g.weighted && any && g.arcs > 0 && ws.seg.mask == nullptr) seg_build(g, ws.seg, s);
+}
+
+void workspace_ensure(Workspace &ws, const DeviceGraph &g, cudaStream_t s, bool need_seg) {
     if (ws.ready && ws.graphs_rb != (const void *)g.rb) {
         // row-blocks were rebuilt (autotuner): captured graphs hold the old list
         for (auto &kv : ws.graphs) cudaGraphExecDestroy(kv.second);
         ws.graphs.clear();
         ws.graphs_rb = g.rb;
     }
-    if (ws.ready && ws.n == g.n && ws.nrb == g.nrb && ws.nhub == g.nhub) return;
+    if (ws.ready && ws.n == g.n && ws.nrb == g.nrb && ws.nhub == g.nhub) {
+        if (need_seg) seg_ensure(ws, g, s);
+        return;
+    }
     if (ws.ready) workspace_free(ws, s);
     ws.n = g.n;
     ws.nrb = g.nrb;
@@ -86,7 +97,8 @@ void workspace_ensure(Workspace &ws, const DeviceGraph &g, cudaStream_t s) {
     const bool seg_eig = !g.weighted && g.seg_eig64 != 0 && g.arcs > 0;
     for (int m = 0; m < kModes; m++) {
         const bool fp32 = m == MODE_CORR32 || m == MODE_KRY32;
-        const uint32_t hot = g.perm != nullptr ? (fp32 ? g.hot_cache : g.hot_cache64) : 0u;
+        // (a hot prefix holds whole quads, so fewer than 4 vertices have none)
+        const uint32_t hot = g.perm != nullptr && g.n >= 4 ? (fp32 ? g.hot_cache : g.hot_cache64) : 0u;
         if (m == MODE_KRY32 && seg) ws.cfg[m] = seg_config(g, g.perm != nullptr ? g.seg_hot : 0u, (int)g.seg_kry32);
         else if (m == MODE_KRES64 && seg_res)
             ws.cfg[m] = seg_config(g, g.perm != nullptr ? g.seg_hot64 : 0u, 2, MODE_KRES64);
@@ -100,7 +112,7 @@ void workspace_ensure(Workspace &ws, const DeviceGraph &g, cudaStream_t s) {
         if (g.perm != nullptr && l1) ws.cfg[m].l1hot = l1;
         gmax = std::max(gmax, ws.cfg[m].grid);
     }
-    if (seg || seg_res || seg_plain || seg_eig) seg_build(g, ws.seg, s);
+    if (need_seg) seg_ensure(ws, g, s);
     const uint64_t n = g.n;
     for (int i = 0; i < 2; i++) {
         walloc(ws.x64[i], n, s);
@@ -229,12 +241,89 @@ void to_f32(const double *a, float *b, uint32_t n, cudaStream_t s) {
     PRG_CUDA(cudaGetLastError());
 }
 
+ResPlan resident_plan(Workspace &ws, const DeviceGraph &g, int kind, cudaStream_t s) {
+    const bool on = g.resident != 0 && (g.weighted || (kind == RES_EIG ? g.seg_eig64 : g.seg_plain64) != 0);
+    if (!on) return ResPlan{};
+    if (!ws.res_planned[kind]) {
+        ws.res_plan[kind] = res_plan(g, kind, s);
+        ws.res_planned[kind] = true;
+    }
+    return ws.res_plan[kind];
+}
+
+void resident_scratch(Workspace &ws, const ResPlan &p, ResArgs &a, cudaStream_t s) {
+    const size_t bytes = res_scratch_bytes(p);
+    if (ws.res_bytes < bytes) {
+        wfree(ws.res_buf, s);
+        PRG_CUDA(cudaMallocAsync(&ws.res_buf, bytes, s));
+        ws.res_bytes = bytes;
+    }
+    a.bar = static_cast<uint32_t *>(ws.res_buf);
+    a.rec = reinterpret_cast<double2 *>(static_cast<unsigned char *>(ws.res_buf) + 256);
+    a.ctl = ws.ctl;
+}
+
+// Iterations of one block-resident launch of the power iteration: a solve
+// with a larger max_iter continues in further launches, so that a tolerance
+// out of reach does not hold the device in one kernel.
+constexpr uint32_t kResidentIters = 4096;
+
+// The FP64 power iteration as block-resident launches; false (nothing done)
+// when the device cannot hold the grid at once.
+static bool resident_loop(const DeviceGraph &g, Workspace &ws, const ResPlan &p, const SolveOpts &o, const double *d_t,
+                          double thr, uint32_t max_iter, SolveStats &st, cudaStream_t s) {
+    ResArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.row_ptr = g.row_ptr;
+    a.col = g.col;
+    a.w64 = g.weighted ? g.w64 : nullptr;
+    a.dval = g.dval;
+    a.t64 = d_t;
+    a.start = o.d_start;
+    a.x_out = ws.x64[0];
+    a.xt[0] = ws.xt64[0];
+    a.xt[1] = ws.xt64[1];
+    a.total = g.arcs + (uint64_t)p.alpha * g.n;
+    a.n = g.n;
+    a.alpha = p.alpha;
+    a.l1hot = g.perm != nullptr && g.l1_hot64 ? kResL1Hot : 0xFFFFFFFFu;
+    a.damping = o.damping;
+    a.thr = thr;
+    resident_scratch(ws, p, a, s);
+    uint32_t done_iters = 0;
+    for (;;) {
+        a.max_iter = std::min(max_iter - done_iters, kResidentIters);
+        PRG_CUDA(cudaMemsetAsync(ws.ctl, 0, sizeof(Ctl), s));
+        PRG_CUDA(cudaEventRecord(ws.eva, s));
+        if (!launch_resident(RES_POWER, p, a, s)) return false;
+        PRG_CUDA(cudaEventRecord(ws.evb, s));
+        read_ctl(ws, s);
+        float t = 0.f;
+        PRG_CUDA(cudaEventElapsedTime(&t, ws.eva, ws.evb));
+        st.fp64_ms += t;
+        st.spmv_ms += t;
+        st.kernel_launches += 1u;
+        if (ws.h_ctl->status != 0) throw TimeoutError{"power iteration: a grid barrier timed out"};
+        done_iters += ws.h_ctl->iters;
+        st.last_diff = ws.h_ctl->diff;
+        if (ws.h_ctl->diff < thr || done_iters >= max_iter) break;
+        a.start = ws.x64[0];
+    }
+    st.spmv_launches += done_iters;
+    st.fp64_passes += done_iters;
+    st.iterations += done_iters;
+    return true;
+}
+
 // FP64 power iteration (PLAIN64 / PPR64) from the start vector until the
 // successive L1 change is < thr or max_iter iterations ran.  Returns the
 // buffer holding the newest iterate.
 const double *fp64_loop(const DeviceGraph &g, Workspace &ws, const SolveOpts &o, const double *d_t, double thr,
                         uint32_t max_iter, SolveStats &st, cudaStream_t s) {
     const bool ppr = d_t != nullptr;
+    const ResPlan rp = max_iter > 0 ? resident_plan(ws, g, RES_POWER, s) : ResPlan{};
+    if (rp.grid && resident_loop(g, ws, rp, o, d_t, thr, max_iter, st, s)) return ws.x64[0];
+    seg_ensure(ws, g, s);
     if (o.d_start) {
         if (o.d_start != ws.x64[0])
             PRG_CUDA(cudaMemcpyAsync(ws.x64[0], o.d_start, (uint64_t)g.n * 8, cudaMemcpyDeviceToDevice, s));
@@ -435,7 +524,7 @@ double time_iterations(const DeviceGraph &g, Workspace &ws, int mode, uint32_t i
 void solve(const DeviceGraph &g, Workspace &ws, const SolveOpts &o_in, const double *d_t, double *d_out,
            SolveStats &st, cudaStream_t s) {
     st = SolveStats{};
-    workspace_ensure(ws, g, s);
+    workspace_ensure(ws, g, s, o_in.precision != 0 || resident_plan(ws, g, RES_POWER, s).grid == 0);
     PRG_CUDA(cudaMemsetAsync(ws.hub_ticket, 0, std::max<uint64_t>(g.nhub, 1) * 4, s));
     PRG_CUDA(cudaEventRecord(ws.ev0, s));
     // Vectors cross into internal ids here: the teleport vector always lives

@@ -6,6 +6,7 @@
 #include <map>
 
 #include "graph.cuh"
+#include "resident.cuh"
 #include "spmv.cuh"
 
 namespace prg {
@@ -57,10 +58,19 @@ struct Workspace {
     const void *graphs_rb = nullptr;  // row-block list the cached graphs were captured with
     int unroll = 8;  // iteration pairs per graph launch
     KrylovWs *kry = nullptr;  // Krylov vectors, allocated on first use
-    SegIndex seg;             // row-end index of the tile-segmented FP32 Krylov matvec (when used)
+    SegIndex seg;             // row-end index of the tile-segmented passes, built on first use
+    void *res_buf = nullptr;  // records of the block-resident iteration, allocated on first use
+    size_t res_bytes = 0;
+    ResPlan res_plan[2];      // by ResKind, once planned
+    bool res_planned[2] = {false, false};
 };
 
-void workspace_ensure(Workspace &ws, const DeviceGraph &g, cudaStream_t s);
+// need_seg = false leaves the tile-segmented passes' index for a later call.
+void workspace_ensure(Workspace &ws, const DeviceGraph &g, cudaStream_t s, bool need_seg = true);
+// The block-resident launch on g (grid 0: not for this graph or tuning) and
+// its scratch in ws.
+ResPlan resident_plan(Workspace &ws, const DeviceGraph &g, int kind, cudaStream_t s);
+void resident_scratch(Workspace &ws, const ResPlan &p, ResArgs &a, cudaStream_t s);
 
 // Device time of one iteration of `mode` (ms), averaged over `iters`
 // back-to-back launches that never converge (autotuner probe).
