@@ -26,6 +26,7 @@
 #include "handle.cuh"
 #include "pool.cuh"
 #include "ppr_batch.cuh"
+#include "small_call.cuh"
 #include "solver.cuh"
 
 namespace {
@@ -353,9 +354,74 @@ int32_t check_options(const prg_options &o) {
     return PRG_OK;
 }
 
+// pagerank_weighted.rs:69-76
+int32_t bad_weight(uint64_t e, double w) {
+    return fail(PRG_ERR_INVALID_ARGUMENT, "weight at edge " + std::to_string(e) +
+                                              " must be non-negative and finite (got " + rust_f64(w) + ")");
+}
+int32_t check_weights(const double *w, uint64_t m) {
+    for (uint64_t e = 0; e < m; e++)
+        if (std::isnan(w[e]) || w[e] < 0.0 || !std::isfinite(w[e])) return bad_weight(e, w[e]);
+    return PRG_OK;
+}
+
+// A drop-in on a small graph in two launches (small_call.cu): true when it
+// ran, with the call's status in *rc and the eigenvalue in *eigenvalue; false
+// sends the call to the general path.
+bool small_dropin(prg::SmallCall &c, double *out, int32_t *rc, double *eigenvalue = nullptr) {
+    const prg::Tuning &t = prg::tuning();
+    const bool seg = c.kind == prg::RES_EIG ? t.seg_eig64 != 0 : t.seg_plain64 != 0;
+    if (!t.resident || !(c.w || seg) || c.m > 0xFFFFFFFFull || check_sizes(c.n, c.m, c.directed) != PRG_OK) return false;
+    if (!ensure_pool_config()) return false;
+    cudaStream_t s = prg::stream_acquire();
+    prg::SmallResult r;
+    prg::SmallStatus st;
+    try {
+        st = prg::small_call(c, out, r, s);
+    } catch (...) {
+        prg::stream_release(s);
+        throw;
+    }
+    prg::stream_release(s);
+    if (st == prg::SMALL_NOT_HERE) return false;
+    if (st == prg::SMALL_BAD_WEIGHT) {
+        *rc = bad_weight(r.bad_edge, c.w[r.bad_edge]);
+        return true;
+    }
+    *rc = st == prg::SMALL_OUT_OF_RANGE ? fail(PRG_ERR_VERTEX_OUT_OF_RANGE, range_message(r.max_endpoint, c.n)) : PRG_OK;
+    if (eigenvalue && st == prg::SMALL_DONE) *eigenvalue = r.eigenvalue;
+    return true;
+}
+
 // One-shot drop-in: build, solve with the reference's constants, download.
+// The weights are checked on the device where the small-graph path runs, else
+// here (and before any device error is reported).
 int32_t dropin(uint32_t n, uint64_t m, const uint32_t *from, const uint32_t *to, int32_t directed, const double *w,
                const double *norm_reset, double damping, double *out, int precision = PRG_PRECISION_FP64) {
+    if (precision == PRG_PRECISION_FP64) {
+        prg::SmallCall c;
+        const prg::SolveOpts d;  // the reference's eps and max_iter
+        c.n = n;
+        c.m = m;
+        c.from = from;
+        c.to = to;
+        c.w = w;
+        c.check_weights = true;
+        c.directed = directed != 0;
+        c.reset = norm_reset;
+        c.damping = damping;
+        c.thr = d.eps;
+        c.max_iter = d.max_iter;
+        int32_t rc = PRG_OK;
+        try {
+            if (small_dropin(c, out, &rc)) return rc;
+        } catch (...) {
+            if (w && (rc = check_weights(w, m)) != PRG_OK) return rc;
+            throw;
+        }
+    }
+    if (w)
+        if (int32_t bad = check_weights(w, m)) return bad;
     prg_graph *h = nullptr;
     int32_t rc = create_from_host(n, m, from, to, w, directed, &h);
     if (rc != PRG_OK) return rc;
@@ -421,6 +487,27 @@ int32_t prg_pagerank(uint32_t n, uint64_t m, const uint32_t *from, const uint32_
     PRG_GUARD_END
 }
 
+// The undirected eigenvector iterations without negative weights
+// (eigenvector.rs:286-372, 375-538) on a small graph.
+static bool small_eigenvector(uint32_t n, uint64_t m, const uint32_t *from, const uint32_t *to, const double *w,
+                              double eps, double *out, double *eigenvalue, int32_t *rc) {
+    for (uint64_t e = 0; w && e < m; e++)
+        if (!std::isfinite(w[e])) return false;
+    prg::SmallCall c;
+    c.n = n;
+    c.m = m;
+    c.from = from;
+    c.to = to;
+    c.w = w;
+    c.directed = false;
+    c.kind = prg::RES_EIG;
+    c.thr = eps;
+    c.shift = 1.0;
+    c.max_iter = 5000;
+    c.strength_seed = w != nullptr;
+    return small_dropin(c, out, rc, eigenvalue);
+}
+
 int32_t prg_eigenvector_centrality(uint32_t n, uint64_t m, const uint32_t *from, const uint32_t *to, int32_t directed,
                                    double *out, double *eigenvalue) {
     g_err.clear();
@@ -434,8 +521,10 @@ int32_t prg_eigenvector_centrality(uint32_t n, uint64_t m, const uint32_t *from,
         for (uint32_t i = 0; i < n; i++) out[i] = 1.0;
         return PRG_OK;
     }
+    int32_t rc = PRG_OK;
+    if (small_eigenvector(n, m, from, to, nullptr, 1e-14, out, eigenvalue, &rc)) return rc;
     prg_graph *h = nullptr;
-    int32_t rc = create_from_host(n, m, from, to, nullptr, 0, &h);
+    rc = create_from_host(n, m, from, to, nullptr, 0, &h);
     if (rc != PRG_OK) return rc;
     try {
         cudaStream_t s = h->stream;
@@ -540,8 +629,10 @@ int32_t prg_eigenvector_centrality_weighted(uint32_t n, uint64_t m, const uint32
     o.rowsum_seed = true;
     o.eps = 1e-12;
     o.negative = any_negative(weights, m);
+    int32_t rc = PRG_OK;
+    if (!o.negative && small_eigenvector(n, m, from, to, weights, o.eps, out, eigenvalue, &rc)) return rc;
     prg_graph *h = nullptr;
-    int32_t rc = create_from_host(n, m, from, to, weights, 0, &h);
+    rc = create_from_host(n, m, from, to, weights, 0, &h);
     if (rc != PRG_OK) return rc;
     try {
         cudaStream_t s = h->stream;
@@ -637,8 +728,16 @@ int32_t prg_hub_and_authority_scores_weighted(uint32_t n, uint64_t m, const uint
         o.signed_seed = true;
         o.eps = 1e-12;
         o.negative = neg;
+        int32_t rc = PRG_OK;
+        double lam = 0.0;
+        if (!neg && small_eigenvector(n, m, from, to, weights, o.eps, hub, &lam, &rc)) {
+            if (rc != PRG_OK) return rc;
+            for (uint32_t i = 0; i < n; i++) authority[i] = hub[i];
+            if (eigenvalue) *eigenvalue = lam * lam;
+            return PRG_OK;
+        }
         prg_graph *h = nullptr;
-        int32_t rc = create_from_host(n, m, from, to, weights, 0, &h);
+        rc = create_from_host(n, m, from, to, weights, 0, &h);
         if (rc != PRG_OK) return rc;
         try {
             cudaStream_t s = h->stream;
@@ -788,12 +887,6 @@ int32_t prg_pagerank_weighted(uint32_t n, uint64_t m, const uint32_t *from, cons
     if (weights_len != m)  // :62-68
         return fail(PRG_ERR_INVALID_ARGUMENT, "weights vector size (" + std::to_string(weights_len) +
                                                   ") differs from edge count (" + std::to_string(m) + ")");
-    for (uint64_t e = 0; e < m; e++) {  // :69-76
-        const double w = weights[e];
-        if (std::isnan(w) || w < 0.0 || !std::isfinite(w))
-            return fail(PRG_ERR_INVALID_ARGUMENT, "weight at edge " + std::to_string(e) +
-                                                      " must be non-negative and finite (got " + rust_f64(w) + ")");
-    }
     return dropin(n, m, from, to, directed, weights, nullptr, 0.85, out);
     PRG_GUARD_END
 }
@@ -876,15 +969,8 @@ int32_t prg_graph_create(uint32_t n, uint64_t m, const uint32_t *from, const uin
     PRG_GUARD_BEGIN
     if (!out) return fail(PRG_ERR_INVALID_ARGUMENT, "null output handle");
     *out = nullptr;
-    if (weights) {
-        for (uint64_t e = 0; e < m; e++) {
-            const double w = weights[e];
-            if (std::isnan(w) || w < 0.0 || !std::isfinite(w))
-                return fail(PRG_ERR_INVALID_ARGUMENT, "weight at edge " + std::to_string(e) +
-                                                          " must be non-negative and finite (got " + rust_f64(w) +
-                                                          ")");
-        }
-    }
+    if (weights)
+        if (int32_t bad = check_weights(weights, m)) return bad;
     const int32_t rc = create_from_host(n, m, from, to, weights, directed, out);
     if (rc == PRG_OK) prepare_handle(*out);
     return rc;

@@ -52,7 +52,7 @@ constexpr uint32_t kResOpen = 0xFFFFFFFFu;   // no row end
 // launched: 0.1 M arcs 4.7 / 18, 1 M 8.1 / 21, 4 M 23 / 38, 8 M 38 / 56 on
 // uniform random graphs (weighted 4.7 / 13, 8.3 / 20, 26 / 48, 49 / 79);
 // R-MAT 4 M 15 / 28, 8 M 27 / 37 (weighted 17 / 136, 38 / 151).
-constexpr uint64_t kResMaxArcs = 10u << 20;
+// Hence kResMaxArcs.
 constexpr int kResTiles = 32;                // tiles of 8192 arcs a block can take
 // Shared memory of a block (dynamic): L1 needs the rest for the gathers in
 // flight and the hot sources.  R-MAT passes of 8 M arcs took 72-84 us with
@@ -67,7 +67,7 @@ constexpr size_t kResStatic = 2048;          // shared memory kept for the kerne
 // graphs of many short rows need 6 or 12 to fit shared memory.
 constexpr unsigned kResSplits = 3;
 __host__ __device__ constexpr uint32_t res_alpha(unsigned k) { return k == 0 ? 3u : k == 1 ? 6u : 12u; }
-constexpr int kResRecs = 5;                  // records a lane adds: at most 160 blocks
+constexpr int kResRecs = kResBlocks / 32;     // records a lane adds
 constexpr uint32_t kResMinShare = 1024;      // arcs + alpha rows a block takes at least
 constexpr uint32_t kResSpins = 1u << 21;     // polls before a barrier gives up (~0.7 us each)
 
@@ -140,7 +140,16 @@ __host__ __device__ inline size_t res_bytes(uint32_t rows, uint32_t chunks, int 
            (size_t)((chunks + kResNT - 1) / kResNT) * kResWarps * 12 + 16;
 }
 
-// For the splits kResAlphas[k]: out[3k ..] = (largest shared bytes of a block,
+// Bound on a block's shared bytes: its arcs + alpha rows exceed the equal share
+// by less than one row.
+__host__ __device__ inline double res_bound(uint64_t total, unsigned nb, uint32_t alpha, uint32_t longest, bool w,
+                                            int kind) {
+    const double share = (double)(total / nb + 2) + longest + alpha;
+    const double per_arc = 4.43 + (w ? 8.0 : 0.0), per_row = (kind == RES_EIG ? 26.0 : 18.0) / alpha;
+    return share * (per_arc > per_row ? per_arc : per_row) + 16.0 * per_arc + 1024.0;
+}
+
+// For the splits res_alpha(k): out[3k ..] = (largest shared bytes of a block,
 // the same with indices and weights streamed, most chunks of a block)
 __global__ void __launch_bounds__(1024) res_plan_kernel(const uint32_t *rp, uint32_t n, uint64_t arcs, unsigned nb,
                                                         int kind, bool w, uint32_t *out) {
@@ -194,6 +203,13 @@ __global__ void __launch_bounds__(kResNT, 1) res_kernel(const ResArgs a) {
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const unsigned nb = gridDim.x, blk = blockIdx.x;
 
+    if (a.longest) {
+        if (a.ctl->status != 0) return;
+        if (res_bound(a.total, nb, a.alpha, *a.longest, W, KIND) > (double)a.smem) {
+            if (blk == 0 && tid == 0) a.ctl->status = 1;
+            return;
+        }
+    }
     if (warp < 2) {
         const unsigned k = blk + warp;
         const uint32_t c = k >= nb ? a.n : k == 0 ? 0u : res_cut(a.row_ptr, a.n, a.alpha, a.total * k / nb);
@@ -542,27 +558,46 @@ __global__ void __launch_bounds__(kResNT, 1) res_kernel(const ResArgs a) {
 
 // ------------------------------------------------------------------ host side
 
+// Shared memory a block may take, and the blocks of a launch.
+static size_t res_limits(uint64_t arcs, uint32_t n, unsigned &nb) {
+    static int sms = 0, optin = 0;
+    if (sms == 0) {
+        int dev = 0, o = 0;
+        PRG_CUDA(cudaGetDevice(&dev));
+        PRG_CUDA(cudaDeviceGetAttribute(&o, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+        optin = o;
+        PRG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    }
+    nb = (unsigned)std::max<uint64_t>(
+        1, std::min<uint64_t>(std::min<unsigned>(sms, kResBlocks), (arcs + (uint64_t)res_alpha(0) * n) / kResMinShare));
+    return std::min(kResSmem, (size_t)optin - kResStatic);
+}
+
+ResPlan res_plan_blind(uint32_t n, uint64_t arcs, bool weighted, int kind) {
+    ResPlan p;
+    if (n < 2 || arcs == 0 || arcs > kResMaxArcs) return p;
+    unsigned nb = 0;
+    const size_t most = res_limits(arcs, n, nb);
+    p.alpha = res_alpha(0);
+    const uint64_t total = arcs + (uint64_t)p.alpha * n;
+    // room for rows of up to 8192 arcs, or what shared memory leaves
+    if (res_bound(total, nb, p.alpha, 512, weighted, kind) > (double)most) return p;
+    p.smem = std::min(most, ((size_t)res_bound(total, nb, p.alpha, 8192, weighted, kind) + 15) & ~(size_t)15);
+    p.grid = nb;
+    return p;
+}
+
 ResPlan res_plan(const DeviceGraph &g, int kind, cudaStream_t s) {
     ResPlan p;
     if (g.n < 2 || g.arcs == 0 || g.arcs > kResMaxArcs) return p;
-    static int sms = 0, optin = 0;
-    if (sms == 0) {
-        int dev = 0;
-        PRG_CUDA(cudaGetDevice(&dev));
-        PRG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        PRG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    }
-    const size_t most = std::min(kResSmem, (size_t)optin - kResStatic);
+    unsigned nb = 0;
+    const size_t most = res_limits(g.arcs, g.n, nb);
     const uint32_t max_chunks = kResTiles * kResNT;
-    const unsigned nb = (unsigned)std::max<uint64_t>(
-        1, std::min<uint64_t>(std::min(sms, 32 * kResRecs), (g.arcs + 3ull * g.n) / kResMinShare));
-    // A block's arcs + alpha rows exceed the equal share by less than one row,
-    // so small graphs fit whatever their rows look like.
+    // small graphs fit whatever their rows look like
     p.alpha = res_alpha(0);
-    const uint64_t share = (g.arcs + (uint64_t)p.alpha * g.n) / nb + 2 + g.max_in_degree + p.alpha;
-    const double per_arc = 4.43 + (g.weighted ? 8.0 : 0.0), per_row = kind == RES_EIG ? 26.0 : 18.0;
-    const double bound = (double)share * std::max(per_arc, per_row / p.alpha) + 16.0 * per_arc + 1024.0;
-    if (bound <= (double)most && share / 8 + 2 <= max_chunks) {
+    const uint64_t total = g.arcs + (uint64_t)p.alpha * g.n;
+    const double bound = res_bound(total, nb, p.alpha, g.max_in_degree, g.weighted, kind);
+    if (bound <= (double)most) {
         p.grid = nb;
         p.smem = ((size_t)bound + 15) & ~(size_t)15;
         return p;
@@ -592,12 +627,13 @@ ResPlan res_plan(const DeviceGraph &g, int kind, cudaStream_t s) {
     return p;
 }
 
-size_t res_scratch_bytes(const ResPlan &p) { return 256 + (size_t)p.grid * 2 * sizeof(double2); }
+size_t res_scratch_bytes(unsigned grid) { return 256 + (size_t)grid * 2 * sizeof(double2); }
 
 template <int KIND, bool W, bool STREAM>
 static bool res_go(const ResPlan &p, const ResArgs &a, cudaStream_t s) {
+    // the attribute belongs to the kernel, not to this launch: always the limit
     PRG_CUDA(cudaFuncSetAttribute(res_kernel<KIND, W, STREAM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)p.smem));
+                                  (int)kResSmem));
     PRG_CUDA(cudaMemsetAsync(a.bar, 0, 4, s));
     void *args[] = {(void *)&a};
     const cudaError_t e = cudaLaunchCooperativeKernel((const void *)res_kernel<KIND, W, STREAM>, dim3(p.grid),

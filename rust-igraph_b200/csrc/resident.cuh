@@ -9,6 +9,8 @@
 namespace prg {
 
 constexpr uint32_t kResL1Hot = 8192;
+constexpr uint64_t kResMaxArcs = 10u << 20;  // see resident.cu
+constexpr unsigned kResBlocks = 160;         // most blocks of a launch
 
 enum ResKind : int {
     RES_POWER = 0,  // damped FP64 power iteration (uniform or personalised teleport)
@@ -35,6 +37,12 @@ struct ResArgs {
     uint32_t *bar;        // arrival counter, zero at launch
     Ctl *ctl;             // out: iters, diff, done, status; RES_EIG: dsum = (x.Ax, x.x)
     uint64_t total;       // arcs + alpha n
+    // a plan made without the rows' lengths: the longest row on the device and
+    // the shared memory given; where a block's share may exceed it, every block
+    // returns with Ctl::status = 1 (null: the plan is known to fit).  With
+    // `longest`, a nonzero status at launch makes the kernel return at once.
+    const uint32_t *longest;
+    uint32_t smem;
     uint32_t n, alpha, max_iter;
     uint32_t l1hot;       // sources at or above this id are gathered without L1 allocation
     double damping, thr, shift;
@@ -43,8 +51,11 @@ struct ResArgs {
 // Launch shape for graph g, or grid = 0 where it does not apply (reads the
 // rows' split back from the device when the sizes alone do not decide).
 ResPlan res_plan(const DeviceGraph &g, int kind, cudaStream_t s);
+// The same before the graph is built, for graphs whose indices surely stay in
+// shared memory as long as no row is long (ResArgs::longest checks that).
+ResPlan res_plan_blind(uint32_t n, uint64_t arcs, bool weighted, int kind);
 // Bytes of scratch the launch needs (records and arrival counter).
-size_t res_scratch_bytes(const ResPlan &p);
+size_t res_scratch_bytes(unsigned grid);
 // Iterates until the stop rule holds or max_iter iterations ran; false when
 // the device cannot hold the grid at once (nothing was launched).
 bool launch_resident(int kind, const ResPlan &p, const ResArgs &a, cudaStream_t s);

@@ -252,7 +252,7 @@ ResPlan resident_plan(Workspace &ws, const DeviceGraph &g, int kind, cudaStream_
 }
 
 void resident_scratch(Workspace &ws, const ResPlan &p, ResArgs &a, cudaStream_t s) {
-    const size_t bytes = res_scratch_bytes(p);
+    const size_t bytes = res_scratch_bytes(p.grid);
     if (ws.res_bytes < bytes) {
         wfree(ws.res_buf, s);
         PRG_CUDA(cudaMallocAsync(&ws.res_buf, bytes, s));
