@@ -534,10 +534,7 @@ static bool resident_iterations(const DeviceGraph &g, Workspace &ws, const ResPl
     a.row_ptr = g.row_ptr;
     a.col = g.col;
     a.w64 = g.weighted ? g.w64 : nullptr;
-    a.start = x[0];
     a.x_out = x[0];
-    a.xt[0] = x[1];
-    a.xt[1] = ws.x64[0];
     a.total = g.arcs + (uint64_t)p.alpha * g.n;
     a.n = g.n;
     a.alpha = p.alpha;

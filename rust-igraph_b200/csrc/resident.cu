@@ -27,16 +27,21 @@
 // RES_POWER is the reference's update in its rounding order (pagerank.rs:107-140,
 // pagerank_weighted.rs:129-159, personalized_pagerank.rs:149-182) with its
 // stop rule.  RES_EIG (eigenvector.rs:286-372, 375-538, 600-720 without
-// negative weights) normalises late: block barriers carry max |y|, and the
-// next step divides the row sums and the block's own y by it, so that one
-// barrier per iteration suffices; the change |x' - x| travels with the next
-// record, one product later.
+// negative weights) stops at a change below 1e-14 (1e-12 with weights), which
+// lies under the rounding of such vectors: in plain FP64 the iterates end in a
+// cycle of last-bit flips and most graphs run to the cap of 5000.  So the sums,
+// the maximum and the division carry their rounding errors along (pairs of
+// doubles) and each component is rounded once per iteration; the flips then die
+// out and the rule holds after the 60-150 iterations the spectrum asks for
+// (power law, 50 k vertices, 0.8 M arcs: 37 ms to the cap, 1.3 ms now).  It takes
+// two barriers, one for max |y| and one for the change.
 //
 // The barrier's wait is bounded (about 1.5 s); after that the block sets
 // Ctl::status and returns.
 #include "resident.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 #include "prims.cuh"
 
@@ -80,20 +85,68 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
     return v;
 }
 
+// A running sum: plain FP64, or (DD) the unevaluated sum h + l of two doubles,
+// in which an addition's rounding error is kept (Dekker's and Knuth's exact
+// transformations).
+__device__ __forceinline__ double two_sum(double a, double b, double &e) {
+    const double s = __dadd_rn(a, b), t = __dsub_rn(s, a);
+    e = __dadd_rn(__dsub_rn(a, __dsub_rn(s, t)), __dsub_rn(b, t));
+    return s;
+}
+template <bool DD>
+struct Acc {
+    double h = 0.0, l = 0.0;
+    __device__ __forceinline__ void add(double vh, double vl) {
+        if constexpr (DD) {
+            double e;
+            h = two_sum(h, vh, e);
+            l += e + vl;
+        } else {
+            h += vh;
+        }
+    }
+    __device__ __forceinline__ void add(const Acc &o) { add(o.h, o.l); }
+    // |l| <= ulp(h) / 2; where h is infinite or NaN, l (NaN there) is dropped
+    __device__ __forceinline__ void normalise() {
+        const double s = __dadd_rn(h, l);
+        if (isfinite(s)) {
+            l = __dadd_rn(__dsub_rn(h, s), l);
+            h = s;
+        } else {
+            l = 0.0;
+        }
+    }
+    __device__ __forceinline__ Acc up(int o) const {
+        Acc r;
+        r.h = __shfl_up_sync(0xffffffffu, h, o);
+        if constexpr (DD) r.l = __shfl_up_sync(0xffffffffu, l, o);
+        return r;
+    }
+};
+
 // Inclusive scan of the lanes' open tails: a lane stops adding where a lane of
 // the range it already covers holds a row end (E: the lanes that do).
-__device__ __forceinline__ double open_scan(double tv, uint32_t E) {
+template <bool DD>
+__device__ __forceinline__ Acc<DD> open_scan(Acc<DD> tv, uint32_t E) {
     const uint32_t lane = threadIdx.x & 31;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const double ov = __shfl_up_sync(0xffffffffu, tv, o);
+        const Acc<DD> ov = tv.up(o);
         if (lane >= (uint32_t)o) {
             const uint32_t upto = lane == 31u ? 0xffffffffu : ((1u << (lane + 1)) - 1u);
             const uint32_t rng = upto & ~((1u << (lane - o + 1)) - 1u);
-            if ((E & rng) == 0u) tv += ov;
+            if ((E & rng) == 0u) tv.add(ov);
         }
     }
     return tv;
+}
+
+// (h, l) becomes the larger of itself and (oh, ol), both normalised.
+__device__ __forceinline__ void dd_max(double &h, double &l, double oh, double ol) {
+    if (oh > h || (oh == h && ol > l)) {
+        h = oh;
+        l = ol;
+    }
 }
 
 // First row r in [0, n] with row_ptr[r] + alpha r >= target (one warp, 32
@@ -135,9 +188,9 @@ struct ResShare {
 
 __host__ __device__ inline size_t res_bytes(uint32_t rows, uint32_t chunks, int kind, bool w, bool stream) {
     const size_t r2 = (rows + 1) & ~1u;
-    return r2 * 8 * (stream ? 1 : kind == RES_EIG ? 3 : 2) + (stream ? 0 : (size_t)chunks * (w ? 96 : 32)) +
+    return r2 * 8 * ((kind == RES_EIG ? 2 : 1) + (stream ? 0 : 1)) + (stream ? 0 : (size_t)chunks * (w ? 96 : 32)) +
            (size_t)((chunks + 3) >> 2) * 4 + (size_t)chunks * 2 + (size_t)rows * 2 +
-           (size_t)((chunks + kResNT - 1) / kResNT) * kResWarps * 12 + 16;
+           (size_t)((chunks + kResNT - 1) / kResNT) * kResWarps * (kind == RES_EIG ? 20 : 12) + 16;
 }
 
 // Bound on a block's shared bytes: its arcs + alpha rows exceed the equal share
@@ -145,7 +198,7 @@ __host__ __device__ inline size_t res_bytes(uint32_t rows, uint32_t chunks, int 
 __host__ __device__ inline double res_bound(uint64_t total, unsigned nb, uint32_t alpha, uint32_t longest, bool w,
                                             int kind) {
     const double share = (double)(total / nb + 2) + longest + alpha;
-    const double per_arc = 4.43 + (w ? 8.0 : 0.0), per_row = (kind == RES_EIG ? 26.0 : 18.0) / alpha;
+    const double per_arc = 4.46 + (w ? 8.0 : 0.0), per_row = (kind == RES_EIG ? 26.0 : 18.0) / alpha;
     return share * (per_arc > per_row ? per_arc : per_row) + 16.0 * per_arc + 1024.0;
 }
 
@@ -195,7 +248,8 @@ __global__ void __launch_bounds__(kResNT, 1) res_kernel(const ResArgs a) {
     __shared__ uint32_t s_cut[2];
     __shared__ uint32_t s_scan[33];
     // per tile: the open sum after its last row end, the rank of its first one
-    __shared__ double s_ttail[kResTiles];
+    constexpr bool DD = KIND == RES_EIG;
+    __shared__ double s_ttail[2][kResTiles];
     __shared__ uint32_t s_tfirst[kResTiles];
     __shared__ double s_red[2][kResWarps];
     __shared__ double s_g[2];
@@ -224,18 +278,19 @@ __global__ void __launch_bounds__(kResNT, 1) res_kernel(const ResArgs a) {
     const double *w64 = W ? a.w64 + (size_t)sh.chunk0 * 8 : nullptr;
 
     // shared layout; col and weights as planes of 16 bytes per chunk
-    double *S = reinterpret_cast<double *>(s_raw);  // row sums by rank
+    double *S = reinterpret_cast<double *>(s_raw);  // row sums by rank, with DD their low parts
+    double *L = S + (size_t)rows2;
     const uint32_t ntiles = (nchunk + kResNT - 1) / kResNT;
     // per tile and warp: the open sum after its last row end, and the rank of
     // its first row end (kResOpen: none)
-    double *s_tail = S + (size_t)rows2;
-    uint32_t *s_first = reinterpret_cast<uint32_t *>(s_tail + ntiles * kResWarps);
+    double *s_tail = S + (size_t)rows2 * (DD ? 2 : 1);
+    double *s_taill = s_tail + ntiles * kResWarps;
+    uint32_t *s_first = reinterpret_cast<uint32_t *>(s_tail + ntiles * kResWarps * (DD ? 2 : 1));
     double *vec = reinterpret_cast<double *>(s_first + ntiles * kResWarps);
     // the block's part of the iterate (in memory when streaming: each thread
-    // reads back what it wrote), and for RES_EIG of the newest product
+    // reads back what it wrote)
     double *xs = STREAM ? a.x_out + R0 : vec;
-    double *ys = vec + rows2;
-    double *w_s = vec + (size_t)rows2 * (STREAM ? 0 : KIND == RES_EIG ? 2 : 1);
+    double *w_s = vec + (STREAM ? 0 : (size_t)rows2);
     uint32_t *c_s = reinterpret_cast<uint32_t *>(w_s + (W && !STREAM ? (size_t)nchunk * 8 : 0));
     uint32_t *m_s = c_s + (STREAM ? 0 : (size_t)nchunk * 8);  // row-end bits, one byte per chunk
     uint16_t *b_s = reinterpret_cast<uint16_t *>(m_s + ((nchunk + 3) >> 2));  // row ends before each chunk
@@ -286,17 +341,25 @@ __global__ void __launch_bounds__(kResNT, 1) res_kernel(const ResArgs a) {
         run += tot;
     }
 
-    // Adds (v0, v1) over the grid: block tree, record, barrier, then every
-    // block adds the records in the same order.  v0 is a maximum for RES_EIG.
+    // Sums (v0, v1) over the grid, or with MAX takes the largest normalised pair:
+    // block tree, record, barrier, then every block reduces the records in the
+    // same order.
     uint32_t phase = 0;
-    auto grid_reduce = [&](double &v0, double &v1) -> bool {
-        if (KIND == RES_EIG) {
+    auto grid_reduce = [&](double &v0, double &v1, auto max_tag) -> bool {
+        constexpr bool MAX = decltype(max_tag)::value;
+        auto warp_reduce = [&]() {
+            if constexpr (MAX) {
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v0 = fmax(v0, __shfl_xor_sync(0xffffffffu, v0, o));
-        } else {
-            v0 = warp_sum(v0);
-        }
-        v1 = warp_sum(v1);
+                for (int o = 16; o > 0; o >>= 1) {
+                    const double oh = __shfl_xor_sync(0xffffffffu, v0, o), ol = __shfl_xor_sync(0xffffffffu, v1, o);
+                    dd_max(v0, v1, oh, ol);
+                }
+            } else {
+                v0 = warp_sum(v0);
+                v1 = warp_sum(v1);
+            }
+        };
+        warp_reduce();
         if (lane == 0) {
             s_red[0][warp] = v0;
             s_red[1][warp] = v1;
@@ -305,13 +368,7 @@ __global__ void __launch_bounds__(kResNT, 1) res_kernel(const ResArgs a) {
         if (warp == 0) {
             v0 = s_red[0][lane];
             v1 = s_red[1][lane];
-            if (KIND == RES_EIG) {
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) v0 = fmax(v0, __shfl_xor_sync(0xffffffffu, v0, o));
-            } else {
-                v0 = warp_sum(v0);
-            }
-            v1 = warp_sum(v1);
+            warp_reduce();
             double2 *rec = a.rec + (size_t)(phase & 1u) * nb;
             if (lane == 0) {
                 int ok = 1;
@@ -336,16 +393,14 @@ __global__ void __launch_bounds__(kResNT, 1) res_kernel(const ResArgs a) {
             v1 = q[0].y;
 #pragma unroll
             for (int j = 1; j < kResRecs; j++) {
-                v0 = KIND == RES_EIG ? fmax(v0, q[j].x) : v0 + q[j].x;
-                v1 += q[j].y;
+                if constexpr (MAX) {
+                    dd_max(v0, v1, q[j].x, q[j].y);
+                } else {
+                    v0 += q[j].x;
+                    v1 += q[j].y;
+                }
             }
-            if (KIND == RES_EIG) {
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) v0 = fmax(v0, __shfl_xor_sync(0xffffffffu, v0, o));
-            } else {
-                v0 = warp_sum(v0);
-            }
-            v1 = warp_sum(v1);
+            warp_reduce();
             if (lane == 0) {
                 s_g[0] = v0;
                 s_g[1] = v1;
@@ -357,6 +412,8 @@ __global__ void __launch_bounds__(kResNT, 1) res_kernel(const ResArgs a) {
         phase++;
         return s_ok != 0;
     };
+    const std::false_type sums{};
+    const std::true_type maxima{};
 
     // Row sums S[rank] of the products w x[col].  x is rewritten every
     // iteration by other SMs; the plain loads see the new values because the
@@ -366,7 +423,14 @@ __global__ void __launch_bounds__(kResNT, 1) res_kernel(const ResArgs a) {
         uint32_t tiles = 0;
         for (uint32_t c0 = 0; c0 < nchunk; c0 += kResNT, tiles++) {
             const uint32_t c = c0 + tid;
-            double v[8];
+            double v[8], vl[8];  // products, with DD their rounding errors
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = vl[k] = 0.0;
+            auto times = [&](int k, double w) {
+                const double p = v[k] * w;
+                if constexpr (DD) vl[k] = fma(v[k], w, -p);
+                v[k] = p;
+            };
             uint32_t m = 0, r = 0;
             if (c < nchunk) {
                 uint32_t cc[8];
@@ -388,70 +452,89 @@ __global__ void __launch_bounds__(kResNT, 1) res_kernel(const ResArgs a) {
                         double ww[4];
                         ld_w4(w64 + (size_t)c * 8 + k, ww);
 #pragma unroll
-                        for (int i = 0; i < 4; i++) v[k + i] *= ww[i];
+                        for (int i = 0; i < 4; i++) times(k + i, ww[i]);
                     }
                 } else if (W) {
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
                         const double2 ww = *reinterpret_cast<const double2 *>(w_s + (size_t)(k * nchunk + c) * 2);
-                        v[2 * k] *= ww.x;
-                        v[2 * k + 1] *= ww.y;
+                        times(2 * k, ww.x);
+                        times(2 * k + 1, ww.y);
                     }
                 }
                 if (c * 8 < lo || c * 8 + 8 > hi) {  // arcs of the neighbouring blocks, padding
 #pragma unroll
                     for (int k = 0; k < 8; k++)
-                        if (c * 8 + k < lo || c * 8 + k >= hi) v[k] = 0.0;
+                        if (c * 8 + k < lo || c * 8 + k >= hi) v[k] = vl[k] = 0.0;
                 }
-            } else {
-#pragma unroll
-                for (int k = 0; k < 8; k++) v[k] = 0.0;
             }
             const uint32_t r0 = r;
-            double acc = 0.0, head = 0.0;
+            Acc<DD> acc, head;
 #pragma unroll
             for (int k = 0; k < 8; k++) {
-                acc += v[k];
+                acc.add(v[k], vl[k]);
                 if ((m >> k) & 1u) {
-                    if (r == r0) head = acc;
-                    else S[r] = acc;
+                    if (r == r0) {
+                        head = acc;
+                    } else {
+                        S[r] = acc.h;
+                        if (DD) L[r] = acc.l;
+                    }
                     r++;
-                    acc = 0.0;
+                    acc = Acc<DD>();
                 }
             }
             const uint32_t E = __ballot_sync(0xffffffffu, m != 0u);
-            const double tv = open_scan(acc, E);
-            double cin = __shfl_up_sync(0xffffffffu, tv, 1);
-            if (lane == 0u) cin = 0.0;
+            const Acc<DD> tv = open_scan(acc, E);
+            Acc<DD> cin = tv.up(1);
+            if (lane == 0u) cin = Acc<DD>();
+            const uint32_t at = tiles * kResWarps + warp;
             if (m != 0u) {
-                S[r0] = head + cin;
-                if ((E & lanemask_lt()) == 0u) s_first[tiles * kResWarps + warp] = r0;  // may lack what came before the warp
+                head.add(cin);
+                S[r0] = head.h;
+                if (DD) L[r0] = head.l;
+                if ((E & lanemask_lt()) == 0u) s_first[at] = r0;  // may lack what came before the warp
             }
             if (lane == 31u) {
-                s_tail[tiles * kResWarps + warp] = tv;
-                if (E == 0u) s_first[tiles * kResWarps + warp] = kResOpen;
+                s_tail[at] = tv.h;
+                if (DD) s_taill[at] = tv.l;
+                if (E == 0u) s_first[at] = kResOpen;
             }
         }
+        auto add_to = [&](uint32_t rank, const Acc<DD> &c) {
+            Acc<DD> t;
+            t.h = S[rank];
+            if (DD) t.l = L[rank];
+            t.add(c);
+            S[rank] = t.h;
+            if (DD) L[rank] = t.l;
+        };
         __syncthreads();
         // what a warp's first row holds from the warps before it in its tile
         if (warp < tiles) {
-            const uint32_t first = s_first[warp * kResWarps + lane];
+            const uint32_t at = warp * kResWarps + lane, first = s_first[at];
             const uint32_t F = __ballot_sync(0xffffffffu, first != kResOpen);
-            const double tv = open_scan(s_tail[warp * kResWarps + lane], F);
-            const double cin = __shfl_up_sync(0xffffffffu, tv, 1);
-            if (lane != 0u && first != kResOpen) S[first] += cin;
-            if (lane == 31u) s_ttail[warp] = tv;
+            Acc<DD> tail;
+            tail.h = s_tail[at];
+            if (DD) tail.l = s_taill[at];
+            const Acc<DD> tv = open_scan(tail, F);
+            const Acc<DD> cin = tv.up(1);
+            if (lane != 0u && first != kResOpen) add_to(first, cin);
+            if (lane == 31u) {
+                s_ttail[0][warp] = tv.h;
+                s_ttail[1][warp] = tv.l;
+            }
             const uint32_t tf = __shfl_sync(0xffffffffu, first, F ? __ffs(F) - 1 : 0);
             if (lane == 0u) s_tfirst[warp] = F ? tf : kResOpen;
         }
         __syncthreads();
         if (tiles > 1) {  // and a tile's first row from the tiles before it
-            if (tid < tiles && s_tfirst[tid] != kResOpen) {
+            if (tid > 0 && tid < tiles && s_tfirst[tid] != kResOpen) {
                 int t = (int)tid - 1;
                 while (t > 0 && s_tfirst[t] == kResOpen) t--;
-                double c = 0.0;
-                for (; t >= 0 && t < (int)tid; t++) c += s_ttail[t];
-                if (tid > 0) S[s_tfirst[tid]] += c;
+                Acc<DD> c;
+                for (; t < (int)tid; t++) c.add(s_ttail[0][t], s_ttail[1][t]);
+                add_to(s_tfirst[tid], c);
             }
             __syncthreads();
         }
@@ -472,7 +555,7 @@ __global__ void __launch_bounds__(kResNT, 1) res_kernel(const ResArgs a) {
             if (dv == 0.0) dsum += x;
             a.xt[0][v] = dv == 0.0 ? 0.0 : x / dv;
         }
-        if (!grid_reduce(v0, dsum)) return;
+        if (!grid_reduce(v0, dsum, sums)) return;
         while (it < a.max_iter && !done) {
             const double *src = a.xt[it & 1u];
             double *dst = a.xt[(it & 1u) ^ 1u];
@@ -495,7 +578,7 @@ __global__ void __launch_bounds__(kResNT, 1) res_kernel(const ResArgs a) {
                 if (dv == 0.0) pds += out;
                 dst[v] = dv == 0.0 ? 0.0 : out / dv;
             }
-            if (!grid_reduce(pd, pds)) return;
+            if (!grid_reduce(pd, pds, sums)) return;
             it++;
             last = pd;
             dsum = pds;
@@ -505,45 +588,53 @@ __global__ void __launch_bounds__(kResNT, 1) res_kernel(const ResArgs a) {
             for (uint32_t r = tid; r < rows; r += kResNT) a.x_out[R0 + r] = xs[r];
     } else {
         if (!STREAM)
-            for (uint32_t r = tid; r < rows; r += kResNT) xs[r] = ys[r] = a.start[R0 + r];
-        double mx = 1.0;  // max |y| of the newest product (1: the start is used as it is)
-        double mk = 1.0;  // the scale of the newest iterate: A x = S / mk
-        for (uint32_t k = 0; !done; k++) {
-            // product k + 1 over x_k = y_k / mx, which also gives |x_k - x_{k-1}|
-            row_sums(k == 0 ? a.start : a.xt[k & 1u]);
-            mk = mx;
-            const double *old = k == 0 ? a.start : a.xt[k & 1u];
-            double *dst = a.xt[(k & 1u) ^ 1u];
-            double pm = 0.0, pd = 0.0;
+            for (uint32_t r = tid; r < rows; r += kResNT) xs[r] = a.x_out[R0 + r];
+        // row r of (shift I + A) x as a normalised pair
+        auto product = [&](uint32_t r) {
+            const uint32_t q = rk[r];
+            const double x = xs[r], p = a.shift * x;
+            Acc<DD> y;
+            y.h = p;
+            y.l = fma(a.shift, x, -p);
+            if (q != kResNone) y.add(S[q], L[q]);
+            y.normalise();
+            return y;
+        };
+        while (!done) {
+            row_sums(a.x_out);
+            double mh = 0.0, ml = 0.0;
             for (uint32_t r = tid; r < rows; r += kResNT) {
-                const uint32_t q = rk[r];
-                const double x = (STREAM ? old[R0 + r] : ys[r]) / mx;
-                const double y = a.shift * x + (q == kResNone ? 0.0 : S[q] / mx);
-                if (k > 0) pd += fabs(x - xs[r]);
-                // a streamed start is still gathered by other blocks at k = 0 and equals x
-                if (!STREAM || k > 0) xs[r] = x;
-                if (!STREAM) ys[r] = y;
-                dst[R0 + r] = y;
-                pm = fmax(pm, fabs(y));
+                const Acc<DD> y = product(r);
+                dd_max(mh, ml, y.h, y.l);
             }
-            if (!grid_reduce(pm, pd)) return;
-            mx = pm > 0.0 ? pm : 1.0;  // a zero vector is not scaled
-            it = k;
+            if (!grid_reduce(mh, ml, maxima)) return;  // every block has gathered x
+            double pd = 0.0, unused = 0.0;
+            for (uint32_t r = tid; r < rows; r += kResNT) {
+                const Acc<DD> y = product(r);
+                double x = y.h;
+                if (mh > 0.0) {  // y / max, rounded once; a zero vector is not scaled
+                    const double q = y.h / mh;
+                    x = isfinite(mh) ? q + (fma(-q, mh, y.h) + (y.l - q * ml)) / mh : q;
+                }
+                pd += fabs(x - xs[r]);
+                xs[r] = x;
+                if (!STREAM) a.x_out[R0 + r] = x;
+            }
+            if (!grid_reduce(pd, unused, sums)) return;
+            it++;
             last = pd;
-            done = k > 0 && (last < a.thr || k >= a.max_iter);
+            done = last < a.thr || it >= a.max_iter;
         }
-        // Rayleigh quotient of the last iterate: its product is already there
-        double unused = 0.0, num = 0.0, den = 0.0;
+        // Rayleigh quotient of the last iterate
+        row_sums(a.x_out);
+        double num = 0.0, den = 0.0;
         for (uint32_t r = tid; r < rows; r += kResNT) {
             const uint32_t q = rk[r];
             const double x = xs[r];
-            num += x * (q == kResNone ? 0.0 : S[q] / mk);
+            num += x * (q == kResNone ? 0.0 : isfinite(L[q]) ? S[q] + L[q] : S[q]);
             den += x * x;
-            if (!STREAM) a.x_out[R0 + r] = x;
         }
-        if (!grid_reduce(unused, num)) return;
-        unused = 0.0;
-        if (!grid_reduce(unused, den)) return;
+        if (!grid_reduce(num, den, sums)) return;
         if (blk == 0 && tid == 0) {
             a.ctl->dsum[0] = num;
             a.ctl->dsum[1] = den;

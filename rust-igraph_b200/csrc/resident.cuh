@@ -30,9 +30,9 @@ struct ResArgs {
     const double *w64;    // null: unweighted
     const double *dval;   // RES_POWER
     const double *t64;    // RES_POWER: teleport vector (null: uniform)
-    const double *start;  // start vector (RES_POWER: null = the teleport vector; not an xt[])
-    double *x_out;        // the last iterate; RES_EIG: the start itself
-    double *xt[2];        // gathered vectors, rewritten in turn (RES_EIG: xt[0] is not the start)
+    const double *start;  // RES_POWER: start vector (null = the teleport vector)
+    double *x_out;        // the last iterate; RES_EIG: in, the start vector
+    double *xt[2];        // RES_POWER: gathered vectors, rewritten in turn
     double2 *rec;         // 2 x grid records
     uint32_t *bar;        // arrival counter, zero at launch
     Ctl *ctl;             // out: iters, diff, done, status; RES_EIG: dsum = (x.Ax, x.x)

@@ -409,7 +409,6 @@ SmallStatus small_call(const SmallCall &c, double *out, SmallResult &r, cudaStre
         q.w64 = c.w ? a.w64 : nullptr;
         q.dval = a.dval;
         q.t64 = c.reset ? f64(o_t) : nullptr;
-        q.start = c.kind == RES_EIG ? a.start : nullptr;
         q.x_out = f64(o_x);
         q.xt[0] = f64(o_xt0);
         q.xt[1] = f64(o_xt1);

@@ -128,3 +128,22 @@ def test_eigenvector_matches_the_oracle(cuda_ok, case, weighted):
     (xa, la), (xb, lb) = got
     assert abs(la - lb) <= 1e-10 * abs(lb)
     assert np.abs(xa - xb).max() <= 1e-10
+
+
+@pytest.mark.parametrize("odd", [np.inf, np.nan, 1e308])
+def test_eigenvector_with_weights_beyond_the_finite_range(cuda_ok, odd):
+    # infinite and NaN components appear exactly where plain FP64 sums give them
+    n, f, t, _ = _graph("er_undirected")
+    g = ig.Graph.from_edge_arrays(n, np.minimum(f, t), np.maximum(f, t), False)
+    w = np.ones(len(f))
+    w[::500] = odd
+    got = []
+    for resident in (1, 0):
+        ig.set_tuning("resident", resident)
+        try:
+            got.append(ig.eigenvector_centrality_weighted(g, w, True))
+        finally:
+            ig.reset_tuning()
+    assert np.array_equal(np.isnan(got[0][0]), np.isnan(got[1][0]))
+    ok = ~np.isnan(got[0][0])
+    assert np.abs(got[0][0][ok] - got[1][0][ok]).max(initial=0.0) <= 1e-10
