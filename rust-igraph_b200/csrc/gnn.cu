@@ -51,6 +51,12 @@ constexpr int oW3 = oWm2 + kC * kH;          // [8 x 48] (row 0 used)
 constexpr int oB3 = oW3 + 8 * kZ;            // [8]      (entry 0 used)
 constexpr int kParams = oB3 + 8;             // 3016
 
+// one row of weight-gradient partials per block of the backward passes (the
+// first two blocks per SM, the second up to four)
+constexpr unsigned kTopBlocks = 148 * 2, kBottomBlocks = 148 * 4;
+constexpr int kPartStride = 3072;
+static_assert(kPartStride >= kParams, "partials");
+
 struct Ws {  // BF16 copies of the weight matrices
     __nv_bfloat16 W1[kH * kF], Wm1[kC * kH], W2[kH * kZ], Wm2[kC * kH], W3[8 * kZ];
 };
@@ -297,16 +303,30 @@ __global__ void scale_kernel(const uint32_t *deg, uint32_t n, float *s) {
 }
 
 // ---- loss ------------------------------------------------------------------
-// target x* in internal ids; L = sum_v w_v (y_v - t_v)^2 / n, w_v = n x*_v.
-__global__ void loss_kernel(const float *y, const double *xs, uint32_t n, float *dy, double *part) {
+// target x* in internal ids; L = sum_v w_v (y_v - t_v)^2 / n, w_v = n x*_v; and
+// the gradient through the output layer's aggregated half,
+// dS2 = dy w3[H..] / (1 + |S2|) (slog'(S) = 1 / (1 + |S|)).
+__global__ void loss_kernel(const float *y, const double *xs, uint32_t n, const float *P, const float *S2, float *dy,
+                            float *dS2, double *part) {
     double l = 0.0;
     const double nn = (double)n;
+    float w3[kC];
+#pragma unroll
+    for (int c = 0; c < kC; c++) w3[c] = P[oW3 + kH + c];
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         const double xv = xs[v] > 1e-300 ? xs[v] : 1e-300;
         const double w = nn * xv, tv = log(nn * xv);
         const double e = (double)y[v] - tv;
         l += w * e * e;
-        dy[v] = (float)(2.0 * w * e / nn);
+        const float g = (float)(2.0 * w * e / nn);
+        dy[v] = g;
+        float s[kC];
+        *reinterpret_cast<float4 *>(s) = *reinterpret_cast<const float4 *>(S2 + (size_t)v * kC);
+        *reinterpret_cast<float4 *>(s + 4) = *reinterpret_cast<const float4 *>(S2 + (size_t)v * kC + 4);
+#pragma unroll
+        for (int c = 0; c < kC; c++) s[c] = g * w3[c] / (1.0f + fabsf(s[c]));
+        *reinterpret_cast<float4 *>(dS2 + (size_t)v * kC) = *reinterpret_cast<const float4 *>(s);
+        *reinterpret_cast<float4 *>(dS2 + (size_t)v * kC + 4) = *reinterpret_cast<const float4 *>(s + 4);
     }
     __shared__ double sh[32];
     l = block_sum<double>(l, sh);
@@ -314,139 +334,348 @@ __global__ void loss_kernel(const float *y, const double *xs, uint32_t n, float 
 }
 
 // ---- backward (FP32 CUDA cores) -----------------------------------------------
+// Transposed aggregation, dM[u] += dS[v] over every in-arc u -> v.  16 lanes per
+// row: 8 arcs at a time, two lanes per arc adding four channels each with one
+// 16-byte reduction (one thread per row and one 4-byte atomic per channel took
+// 0.48 ms on 0.5 M vertices and 3 M arcs, this 0.04).  Rows of more than
+// kAggHeavy arcs are skipped: scatter_heavy_kernel spreads them over blocks.
+__device__ __forceinline__ void red_add4(float *p, const float4 &g) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(g.x), "f"(g.y), "f"(g.z),
+                 "f"(g.w)
+                 : "memory");
+}
+
+__global__ void scatter_kernel(uint32_t n, const uint32_t *row_ptr, const uint32_t *col, const float *dS, float *dM) {
+    const uint32_t sub = (threadIdx.x & 15) >> 1, half = threadIdx.x & 1;
+    const uint32_t ngroups = (gridDim.x * blockDim.x) >> 4;
+    for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 4; v < n; v += ngroups) {
+        const uint32_t p0 = row_ptr[v], p1 = row_ptr[v + 1];
+        if (p1 == p0 || p1 - p0 > kAggHeavy) continue;
+        const float4 g = __ldg(reinterpret_cast<const float4 *>(dS + (size_t)v * kC) + half);
+        for (uint32_t p = p0 + sub; p < p1; p += 8) red_add4(dM + (size_t)__ldg(&col[p]) * kC + half * 4, g);
+    }
+}
+
+__global__ void scatter_heavy_kernel(const uint32_t *row_ptr, const uint32_t *col, const float *dS, float *dM,
+                                     const uint32_t *heavy, const uint32_t *nheavy) {
+    const uint32_t cnt = *nheavy, half = threadIdx.x & 1;
+    for (uint32_t i = 0; i < cnt; i++) {
+        const uint32_t v = heavy[i], p0 = row_ptr[v], p1 = row_ptr[v + 1];
+        const float4 g = __ldg(reinterpret_cast<const float4 *>(dS + (size_t)v * kC) + half);
+        for (uint32_t p = p0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 1); p < p1; p += (gridDim.x * blockDim.x) >> 1)
+            red_add4(dM + (size_t)__ldg(&col[p]) * kC + half * 4, g);
+    }
+}
+
+// The two dense backward passes: one warp per vertex, lane k on hidden unit k,
+// kVB vertices per step.  Everything a vertex contributes (its own gradients and
+// its share of the weight gradients) is computed while its rows are on chip:
+// reading per-layer buffers back for separate outer-product and matrix kernels
+// took 2.4 ms on 0.5 M vertices (a thread per vertex walked 128-byte rows).  The
+// rows of the next step arrive by cp.async while a step is computed (without
+// that the passes waited for memory: 306 + 159 us).  What bounds them then is
+// FP32 issue, about 170 instructions per vertex and warp in the first.
+// Weight-gradient sums stay in registers over the warp's vertices, are added over
+// the block's warps in shared memory in warp order, and leave one partial per
+// block for reduce_part_kernel, so everything but the atomic scatters is
+// deterministic.
+constexpr int kVB = 4;
+constexpr int kBwdThreads = 256, kBwdWarps = kBwdThreads / 32;
+
+// 8 consecutive BF16 (16-byte aligned) of shared memory as floats
+__device__ __forceinline__ void ld_bf8s(const unsigned char *p, float (&f)[8]) {
+    const uint4 q = *reinterpret_cast<const uint4 *>(p);
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        f[2 * i] = __uint_as_float(w[i] << 16);
+        f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+    }
+}
+__device__ __forceinline__ void cp16(unsigned char *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+
 __device__ __forceinline__ float bf(const __nv_bfloat16 &x) { return __bfloat162float(x); }
 
-// dy -> dH1 (32) and dA2 (8) through y = [H1 | A2] w3 + b3
-__global__ void bwd_out_kernel(uint32_t n, const float *dy, const float *P, float *dH1, float *dA2) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const float g = dy[v];
-        for (int k = 0; k < kH; k++) dH1[(size_t)v * kH + k] = g * P[oW3 + k];
-        for (int c = 0; c < kC; c++) dA2[(size_t)v * kC + c] = g * P[oW3 + kH + c];
+// acc (one per lane) summed over the block's warps in warp order into out[lane]
+__device__ __forceinline__ void block_lane_sum(float acc, float (*sh)[32], float *out) {
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    __syncthreads();
+    sh[w][l] = acc;
+    __syncthreads();
+    if (w == 0) {
+        float t = sh[0][l];
+        for (int k = 1; k < kBwdWarps; k++) t += sh[k][l];
+        out[l] = t;
     }
 }
 
-// dM[u] += dS[v] over every in-arc u -> v (transposed aggregation), where
-// dS = dA / (1 + |S|) is the gradient through A = slog(S)
-__global__ void scatter_kernel(uint32_t n, const uint32_t *row_ptr, const uint32_t *col, const float *dA,
-                               const float *S, float *dM) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        float g[kC];
-        for (int c = 0; c < kC; c++) g[c] = dA[(size_t)v * kC + c] / (1.0f + fabsf(S[(size_t)v * kC + c]));
-        for (uint32_t p = row_ptr[v]; p < row_ptr[v + 1]; p++) {
-            const uint32_t u = col[p];
-            for (int c = 0; c < kC; c++) atomicAdd(&dM[(size_t)u * kC + c], g[c]);
-        }
-    }
-}
-
-// message layer: G = dM * s; dH += G Wm; then relu mask -> dPre (in place in dH)
-__global__ void bwd_msg_kernel(uint32_t n, const float *dM, const float *s, const float *P, int oWm,
-                               const __nv_bfloat16 *H, float *G, float *dH) {
-    for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x) {
-        float g[kC];
-        for (int c = 0; c < kC; c++) {
-            g[c] = dM[(size_t)u * kC + c] * s[u];
-            G[(size_t)u * kC + c] = g[c];
-        }
-        for (int k = 0; k < kH; k++) {
-            float d = dH[(size_t)u * kH + k];
-            for (int c = 0; c < kC; c++) d += g[c] * P[oWm + c * kH + k];
-            dH[(size_t)u * kH + k] = bf(H[(size_t)u * kH + k]) > 0.0f ? d : 0.0f;
-        }
-    }
-}
-
-// dZ1 = dPre1 W2 -> dH0 (first 32), dA1 (next 8)
-__global__ void bwd_z1_kernel(uint32_t n, const float *dPre1, const float *P, float *dH0, float *dA1) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        float d[kH];
-        for (int j = 0; j < kH; j++) d[j] = dPre1[(size_t)v * kH + j];
-        for (int k = 0; k < kH + kC; k++) {
-            float z = 0.0f;
-            for (int j = 0; j < kH; j++) z += d[j] * P[oW2 + j * kZ + k];
-            if (k < kH) dH0[(size_t)v * kH + k] = z;
-            else dA1[(size_t)v * kC + (k - kH)] = z;
-        }
-    }
-}
-
-// Weight-gradient partials: part[block][o][i] = sum_v A[v][o] * B[v][i], with
-// B = [B0 (I0 cols, BF16) | B1 (I1 cols, BF16)] and optional column sums of A
-// (bias gradients) in part[block][O*I + o].  Fixed vertex ranges per block.
-template <int O, int I0, int I1>
-__global__ void __launch_bounds__(256) outer_kernel(uint32_t n, const float *A, const __nv_bfloat16 *B0, int ld0,
-                                                    const __nv_bfloat16 *B1, int ld1, float *part, int stride) {
-    constexpr int I = I0 + I1, OI = O * I, TV = 64;
-    __shared__ float sA[TV][O];
-    __shared__ float sB[TV][I];
-    constexpr int PER = (OI + O + 255) / 256;
-    float acc[PER];
+// Output layer, second message layer and second hidden layer:
+//   dPre1 = relu'(H1) (dy w3 + (s dM1) Wm2);  dZ1 = dPre1 W2 = [dH0 | dA1];
+//   dS1 = dA1 / (1 + |S1|); partial gradients of w3, b3, Wm2, W2, b2.
+__global__ void __launch_bounds__(kBwdThreads, 2) bwd_top_kernel(
+    uint32_t n, const float *dy, const float *dM1, const float *s, const float *P, const __nv_bfloat16 *H1,
+    const __nv_bfloat16 *A2, const __nv_bfloat16 *H0, const __nv_bfloat16 *A1, const float *S1, float *dH0, float *dS1,
+    float *part) {
+    __shared__ float sW2[kH][kH + kC];                         // W2[j][k], k < 40 (the rest meets zero padding)
+    __shared__ __align__(16) float sD[kBwdWarps][kH][kVB];     // dPre1 of the warp's vertices
+    __shared__ float sRed[kBwdWarps][32], sLast[32];
+    // the rows of kVB vertices: per vertex H1 64 | H0 64 | dM1 32 | S1 32 | A1 16 | A2 16, then dy and s
+    constexpr int kRow = 224, kStage = kVB * kRow + 32;
+    __shared__ __align__(16) unsigned char sIn[kBwdWarps][2][kStage];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < kH * (kH + kC); i += kBwdThreads)
+        sW2[i / (kH + kC)][i % (kH + kC)] = P[oW2 + (i / (kH + kC)) * kZ + i % (kH + kC)];
+    float wm[kC];
 #pragma unroll
-    for (int k = 0; k < PER; k++) acc[k] = 0.0f;
-    const uint64_t per_blk = ((uint64_t)n + gridDim.x - 1) / gridDim.x;
-    const uint64_t lo = per_blk * blockIdx.x, hi = std::min<uint64_t>(lo + per_blk, n);
-    for (uint64_t v0 = lo; v0 < hi; v0 += TV) {
-        const int cnt = (int)std::min<uint64_t>(TV, hi - v0);
-        __syncthreads();
-        for (int i = threadIdx.x; i < TV * O; i += blockDim.x) {
-            const int r = i / O, c = i % O;
-            sA[r][c] = r < cnt ? A[(v0 + r) * O + c] : 0.0f;
-        }
-        for (int i = threadIdx.x; i < TV * I; i += blockDim.x) {
-            const int r = i / I, c = i % I;
-            float b = 0.0f;
-            if (r < cnt) b = c < I0 ? bf(B0[(v0 + r) * ld0 + c]) : bf(B1[(v0 + r) * ld1 + (c - I0)]);
-            sB[r][c] = b;
-        }
-        __syncthreads();
+    for (int c = 0; c < kC; c++) wm[c] = P[oWm2 + c * kH + lane];
+    const float w3 = P[oW3 + lane];
+    __syncthreads();
+    float aW2[kH + kC], aWm[kC], aW3h = 0.0f, aW3a = 0.0f, aB2 = 0.0f, aB3 = 0.0f;
 #pragma unroll
-        for (int k = 0; k < PER; k++) {
-            const int idx = threadIdx.x + k * 256;
-            if (idx < OI) {
-                const int o = idx / I, i = idx % I;
-                float a = acc[k];
-                for (int r = 0; r < cnt; r++) a += sA[r][o] * sB[r][i];
-                acc[k] = a;
-            } else if (idx < OI + O) {
-                const int o = idx - OI;
-                float a = acc[k];
-                for (int r = 0; r < cnt; r++) a += sA[r][o];
-                acc[k] = a;
+    for (int i = 0; i < kH + kC; i++) aW2[i] = 0.0f;
+#pragma unroll
+    for (int c = 0; c < kC; c++) aWm[c] = 0.0f;
+    const uint32_t stride = gridDim.x * kBwdWarps * kVB;
+    auto fetch = [&](uint32_t v0, int st) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int q = lane + 32 * i, b = q / 14, part_ = q % 14;
+            const uint32_t v = v0 + b;
+            if (q < 14 * kVB) {
+                if (v >= n) continue;
+                const void *src;
+                if (part_ < 4) src = H1 + (size_t)v * kH + part_ * 8;
+                else if (part_ < 8) src = H0 + (size_t)v * kH + (part_ - 4) * 8;
+                else if (part_ < 10) src = dM1 + (size_t)v * kC + (part_ - 8) * 4;
+                else if (part_ < 12) src = S1 + (size_t)v * kC + (part_ - 10) * 4;
+                else src = (part_ == 12 ? A1 : A2) + (size_t)v * 16;
+                cp16(&sIn[w][st][b * kRow + part_ * 16], src);
+            } else if (q < 14 * kVB + 2 && v0 < n) {
+                // (the buffers are padded to 256 bytes, so four values can be read at any v0 < n)
+                cp16(&sIn[w][st][kVB * kRow + (q - 14 * kVB) * 16], (q == 14 * kVB ? dy : s) + v0);
             }
         }
+        cp_commit();
+    };
+    uint32_t v0 = (blockIdx.x * kBwdWarps + w) * kVB;
+    fetch(v0, 0);
+    for (int st = 0; v0 < n; v0 += stride, st ^= 1) {
+        __syncwarp();  // the other stage is no longer read
+        fetch(v0 + stride, st ^ 1);
+        cp_wait1();
+        __syncwarp();
+        const unsigned char *in = sIn[w][st];
+        const float4 dy4 = *reinterpret_cast<const float4 *>(in + kVB * kRow);
+        const float4 s4 = *reinterpret_cast<const float4 *>(in + kVB * kRow + 16);
+        const float dyv[kVB] = {dy4.x, dy4.y, dy4.z, dy4.w}, sv[kVB] = {s4.x, s4.y, s4.z, s4.w};
+        float d[kVB];
+#pragma unroll
+        for (int b = 0; b < kVB; b++) {
+            d[b] = 0.0f;
+            if (v0 + b >= n) continue;  // warp-uniform
+            const unsigned char *row = in + b * kRow;
+            const float g = dyv[b], sc = sv[b], h = bf(reinterpret_cast<const __nv_bfloat16 *>(row)[lane]);
+            const float4 m0 = *reinterpret_cast<const float4 *>(row + 128);
+            const float4 m1 = *reinterpret_cast<const float4 *>(row + 144);
+            const float gm[kC] = {m0.x * sc, m0.y * sc, m0.z * sc, m0.w * sc, m1.x * sc, m1.y * sc, m1.z * sc, m1.w * sc};
+            float t = g * w3;
+#pragma unroll
+            for (int c = 0; c < kC; c++) {
+                t += gm[c] * wm[c];
+                aWm[c] += gm[c] * h;
+            }
+            d[b] = h > 0.0f ? t : 0.0f;
+            aB2 += d[b];
+            aW3h += g * h;
+            if (lane < kC) aW3a += g * bf(reinterpret_cast<const __nv_bfloat16 *>(row + 208)[lane]);
+            if (lane == 0) aB3 += g;
+        }
+        __syncwarp();
+        *reinterpret_cast<float4 *>(&sD[w][lane][0]) = make_float4(d[0], d[1], d[2], d[3]);
+        __syncwarp();
+        // dW2[lane][i] += dPre1[lane] Z1[i]
+#pragma unroll
+        for (int b = 0; b < kVB; b++) {
+            const uint32_t v = v0 + b;
+            if (v >= n) continue;
+#pragma unroll
+            for (int q = 0; q < kH / 8 + 1; q++) {
+                float z[8];
+                ld_bf8s(in + b * kRow + (q < kH / 8 ? 64 + q * 16 : 192), z);
+#pragma unroll
+                for (int i = 0; i < 8; i++) aW2[q * 8 + i] += d[b] * z[i];
+            }
+        }
+        // dZ1: hidden unit `lane`, and channel lane & 7 from a quarter of the units
+        float z[kVB] = {0.0f, 0.0f, 0.0f, 0.0f}, zc[kVB] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int j = 0; j < kH; j++) {
+            const float4 q = *reinterpret_cast<const float4 *>(&sD[w][j][0]);
+            const float wj = sW2[j][lane];
+            z[0] += q.x * wj;
+            z[1] += q.y * wj;
+            z[2] += q.z * wj;
+            z[3] += q.w * wj;
+        }
+#pragma unroll
+        for (int i = 0; i < kH / 4; i++) {
+            const int j = (lane >> 3) * (kH / 4) + i;
+            const float4 q = *reinterpret_cast<const float4 *>(&sD[w][j][0]);
+            const float wj = sW2[j][kH + (lane & 7)];
+            zc[0] += q.x * wj;
+            zc[1] += q.y * wj;
+            zc[2] += q.z * wj;
+            zc[3] += q.w * wj;
+        }
+#pragma unroll
+        for (int b = 0; b < kVB; b++) {
+            zc[b] += __shfl_xor_sync(0xffffffffu, zc[b], 8);
+            zc[b] += __shfl_xor_sync(0xffffffffu, zc[b], 16);
+            const uint32_t v = v0 + b;
+            if (v >= n) continue;
+            dH0[(size_t)v * kH + lane] = z[b];
+            if (lane < kC) dS1[(size_t)v * kC + lane] =
+                              zc[b] / (1.0f + fabsf(reinterpret_cast<const float *>(in + b * kRow + 160)[lane]));
+        }
+    }
+    float *out = part + (size_t)blockIdx.x * kPartStride;
+#pragma unroll
+    for (int i = 0; i < kH + kC; i++) {
+        // W2 is [lane][i]: transposed through the block sum
+        const int wi = threadIdx.x >> 5;
+        __syncthreads();
+        sRed[wi][lane] = aW2[i];
+        __syncthreads();
+        if (wi == 0) {
+            float t = sRed[0][lane];
+            for (int k = 1; k < kBwdWarps; k++) t += sRed[k][lane];
+            out[oW2 + lane * kZ + i] = t;
+        }
     }
 #pragma unroll
-    for (int k = 0; k < PER; k++) {
-        const int idx = threadIdx.x + k * 256;
-        if (idx < OI + O) part[(size_t)blockIdx.x * stride + idx] = acc[k];
-    }
+    for (int c = 0; c < kC; c++) block_lane_sum(aWm[c], sRed, out + oWm2 + c * kH);
+    block_lane_sum(aB2, sRed, out + oB2);
+    block_lane_sum(aW3h, sRed, out + oW3);
+    const float b3 = __shfl_sync(0xffffffffu, aB3, 0);
+    block_lane_sum(lane < kC ? aW3a : lane == kC ? b3 : 0.0f, sRed, sLast);
+    __syncthreads();
+    if (threadIdx.x < kC) out[oW3 + kH + threadIdx.x] = sLast[threadIdx.x];
+    if (threadIdx.x == kC) out[oB3] = sLast[kC];
 }
 
-// grad[off + i] = sum over blocks of part[b][i]  (fixed order)
-__global__ void reduce_part_kernel(const float *part, unsigned nb, int stride, int count, float *grad, int off) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (unsigned b = 0; b < nb; b++) s += part[(size_t)b * stride + i];
-        grad[off + i] = (float)s;
+// First message layer and first hidden layer:
+//   dPre0 = relu'(H0) (dH0 + (s dM0) Wm1); partial gradients of Wm1, W1, b1.
+__global__ void __launch_bounds__(kBwdThreads) bwd_bottom_kernel(uint32_t n, const float *dM0, const float *s,
+                                                                 const float *P, const __nv_bfloat16 *H0,
+                                                                 const __nv_bfloat16 *X0, const float *dH0,
+                                                                 float *part) {
+    __shared__ float sRed[kBwdWarps][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float wm[kC], aWm[kC], aW1[8], aB1 = 0.0f;
+#pragma unroll
+    for (int c = 0; c < kC; c++) {
+        wm[c] = P[oWm1 + c * kH + lane];
+        aWm[c] = aW1[c] = 0.0f;
     }
-}
-
-// dy-weighted outer products for the output layer (O = 1)
-__global__ void __launch_bounds__(256) outer_out_kernel(uint32_t n, const float *dy, const __nv_bfloat16 *H1,
-                                                        const __nv_bfloat16 *A2, float *part, int stride) {
-    // threads 0..47: w3 row-0 entries; thread 48: b3
-    float acc = 0.0f;
-    const uint64_t per_blk = ((uint64_t)n + gridDim.x - 1) / gridDim.x;
-    const uint64_t lo = per_blk * blockIdx.x, hi = std::min<uint64_t>(lo + per_blk, n);
-    const int k = threadIdx.x;
-    if (k <= kZ) {
-        for (uint64_t v = lo; v < hi; v++) {
-            float z = 1.0f;
-            if (k < kH) z = bf(H1[v * kH + k]);
-            else if (k < kZ) z = bf(A2[v * 16 + (k - kH)]);
-            acc += dy[v] * z;
+    // per vertex dH0 128 | H0 64 | dM0 32 | X0 16 (features 6 .. 15 are zero), then s
+    constexpr int kRow = 240, kStage = kVB * kRow + 16;
+    __shared__ __align__(16) unsigned char sIn[kBwdWarps][2][kStage];
+    const uint32_t stride = gridDim.x * kBwdWarps * kVB;
+    auto fetch = [&](uint32_t v0, int st) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int q = lane + 32 * i, b = q / 15, part_ = q % 15;
+            const uint32_t v = v0 + b;
+            if (q < 15 * kVB) {
+                if (v >= n) continue;
+                const void *src;
+                if (part_ < 8) src = dH0 + (size_t)v * kH + part_ * 4;
+                else if (part_ < 12) src = H0 + (size_t)v * kH + (part_ - 8) * 8;
+                else if (part_ < 14) src = dM0 + (size_t)v * kC + (part_ - 12) * 4;
+                else src = X0 + (size_t)v * kF;
+                cp16(&sIn[w][st][b * kRow + part_ * 16], src);
+            } else if (q == 15 * kVB && v0 < n) {
+                cp16(&sIn[w][st][kVB * kRow], s + v0);
+            }
         }
-        part[(size_t)blockIdx.x * stride + k] = acc;
+        cp_commit();
+    };
+    uint32_t v0 = (blockIdx.x * kBwdWarps + w) * kVB;
+    fetch(v0, 0);
+    for (int st = 0; v0 < n; v0 += stride, st ^= 1) {
+        __syncwarp();
+        fetch(v0 + stride, st ^ 1);
+        cp_wait1();
+        __syncwarp();
+        const unsigned char *in = sIn[w][st];
+        const float4 s4 = *reinterpret_cast<const float4 *>(in + kVB * kRow);
+        const float sv[kVB] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+        for (int b = 0; b < kVB; b++) {
+            if (v0 + b >= n) continue;
+            const unsigned char *row = in + b * kRow;
+            const float sc = sv[b], h = bf(reinterpret_cast<const __nv_bfloat16 *>(row + 128)[lane]);
+            const float4 m0 = *reinterpret_cast<const float4 *>(row + 192);
+            const float4 m1 = *reinterpret_cast<const float4 *>(row + 208);
+            const float gm[kC] = {m0.x * sc, m0.y * sc, m0.z * sc, m0.w * sc, m1.x * sc, m1.y * sc, m1.z * sc, m1.w * sc};
+            float t = reinterpret_cast<const float *>(row)[lane];
+#pragma unroll
+            for (int c = 0; c < kC; c++) {
+                t += gm[c] * wm[c];
+                aWm[c] += gm[c] * h;
+            }
+            const float d = h > 0.0f ? t : 0.0f;
+            aB1 += d;
+            float x[8];
+            ld_bf8s(row + 224, x);
+#pragma unroll
+            for (int i = 0; i < 8; i++) aW1[i] += d * x[i];
+        }
+    }
+    float *out = part + (size_t)blockIdx.x * kPartStride;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        __syncthreads();
+        sRed[w][lane] = aW1[i];
+        __syncthreads();
+        if (w == 0) {
+            float t = sRed[0][lane];
+            for (int k = 1; k < kBwdWarps; k++) t += sRed[k][lane];
+            out[oW1 + lane * kF + i] = t;
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < kC; c++) block_lane_sum(aWm[c], sRed, out + oWm1 + c * kH);
+    block_lane_sum(aB1, sRed, out + oB1);
+}
+
+// grad[i] = sum over blocks of part[b][i] in FP64: 32 parameters x 8 slices of
+// the blocks per thread block, the slices added in order.
+__global__ void __launch_bounds__(256) reduce_part_kernel(const float *part, unsigned nb_bottom, unsigned nb_top,
+                                                          float *grad) {
+    __shared__ double sh[8][32];
+    const int l = threadIdx.x & 31, q = threadIdx.x >> 5, i = blockIdx.x * 32 + l;
+    // slots no backward pass writes: W1's columns past the features it sees,
+    // W2's zero padding, W3's unused rows and b3's unused entries
+    bool used = i < kParams;
+    if (i < oB1) used = i % kF < 8;
+    else if (i >= oW2 && i < oB2) used = (i - oW2) % kZ < kH + kC;
+    else if (i >= oW3 && i < oB3) used = i < oW3 + kH + kC;
+    else if (i >= oB3) used = i == oB3;
+    const unsigned nb = i < oW2 ? nb_bottom : nb_top;
+    double s = 0.0;
+    if (used)
+        for (unsigned b = q; b < nb; b += 8) s += part[(size_t)b * kPartStride + i];
+    sh[q][l] = s;
+    __syncthreads();
+    if (q == 0 && i < kParams) {
+        for (int k = 1; k < 8; k++) s += sh[k][l];
+        grad[i] = (float)s;
     }
 }
 
@@ -679,8 +908,6 @@ void Net::alloc(cudaStream_t s) {
     PRG_CUDA(cudaMallocAsync((void **)&m, kParams * 4, s));
     PRG_CUDA(cudaMallocAsync((void **)&v, kParams * 4, s));
     PRG_CUDA(cudaMallocAsync((void **)&w, sizeof(Ws), s));
-    // loss_grad writes only the used rows of W3 / entries of B3, so the
-    // gradient's other slots must start (and stay) zero
     PRG_CUDA(cudaMemsetAsync(G, 0, kParams * 4, s));
     PRG_CUDA(cudaMemsetAsync(m, 0, kParams * 4, s));
     PRG_CUDA(cudaMemsetAsync(v, 0, kParams * 4, s));
@@ -710,24 +937,22 @@ void Net::free(cudaStream_t s) {
 }
 
 // scratch layout per vertex (bytes): X0 32, H0 64, M0 32, A1 32, H1 64, M1 32,
-// A2 32, y 4, s 4, dy 4, dH1 128, dA2 32, dM1 32, G1 32, dH0 128, dA1 32,
-// dM0 32, G0 32, S1 32, S2 32  -> 832 bytes per vertex, plus partials.
-constexpr size_t kPerVertex = 832;
-constexpr unsigned kRedBlocks = 512;
-constexpr int kPartStride = 2048;
+// A2 32, y 4, s 4, dy 4, dS2 32, dM1 32, dH0 128, dS1 32, dM0 32, S1 32, S2 32
+// -> 620 bytes per vertex, plus the heavy-row list and partials.
+constexpr size_t kPerVertex = 620;
 
 void Net::ensure(uint32_t n, cudaStream_t s) {
     if (buf && buf_n >= n) return;
     if (buf) cudaFreeAsync(buf, s);
     buf_n = n;
-    const size_t bytes = (size_t)n * kPerVertex + (size_t)kRedBlocks * kPartStride * 4 + 64 * 1024 +
+    const size_t bytes = (size_t)n * kPerVertex + (size_t)kBottomBlocks * kPartStride * 4 + 64 * 1024 +
                          (size_t)n * 4 + 8192;
     PRG_CUDA(cudaMallocAsync((void **)&buf, bytes, s));
 }
 
 struct Views {
     __nv_bfloat16 *X0, *H0, *A1, *H1, *A2;
-    float *M0, *M1, *y, *s, *dy, *dH1, *dA2, *dM1, *G1, *dH0, *dA1, *dM0, *G0, *S1, *S2, *part, *fpart;
+    float *M0, *M1, *y, *s, *dy, *dS2, *dM1, *dH0, *dS1, *dM0, *S1, *S2, *part, *fpart;
     double *dpart;
     uint32_t *heavy, *nheavy;
 };
@@ -750,18 +975,15 @@ static Views views(unsigned char *b, uint32_t n) {
     V.y = (float *)take((size_t)n * 4);
     V.s = (float *)take((size_t)n * 4);
     V.dy = (float *)take((size_t)n * 4);
-    V.dH1 = (float *)take((size_t)n * 128);
-    V.dA2 = (float *)take((size_t)n * 32);
+    V.dS2 = (float *)take((size_t)n * 32);
     V.dM1 = (float *)take((size_t)n * 32);
-    V.G1 = (float *)take((size_t)n * 32);
     V.dH0 = (float *)take((size_t)n * 128);
-    V.dA1 = (float *)take((size_t)n * 32);
+    V.dS1 = (float *)take((size_t)n * 32);
     V.dM0 = (float *)take((size_t)n * 32);
-    V.G0 = (float *)take((size_t)n * 32);
     V.S1 = (float *)take((size_t)n * 32);
     V.S2 = (float *)take((size_t)n * 32);
     V.heavy = (uint32_t *)take((size_t)n * 4);
-    V.part = (float *)take((size_t)kRedBlocks * kPartStride * 4);
+    V.part = (float *)take((size_t)kBottomBlocks * kPartStride * 4);
     V.fpart = (float *)take(4096 * 4);
     V.dpart = (double *)take(4096 * 8);
     V.nheavy = (uint32_t *)take(256);
@@ -824,36 +1046,26 @@ void Net::predict(const DeviceGraph &g, double *x_internal, cudaStream_t s) {
 }
 
 double Net::loss_grad(const DeviceGraph &g, const double *target_internal, cudaStream_t s) {
-    forward(g, s);
+    forward(g, s);  // leaves the heavy rows' list for the scatters
     Views V = views(buf, g.n);
     const uint32_t n = g.n;
-    const unsigned gn = grid_n(n);
     const unsigned gb = 296;
-    loss_kernel<<<gb, 256, 0, s>>>(V.y, target_internal, n, V.dy, V.dpart);
-    // output layer
-    const unsigned nb = std::min<unsigned>(kRedBlocks, std::max<uint32_t>(1, (n + 1023) / 1024));
-    outer_out_kernel<<<nb, 256, 0, s>>>(n, V.dy, V.H1, V.A2, V.part, kPartStride);
-    reduce_part_kernel<<<1, 64, 0, s>>>(V.part, nb, kPartStride, kZ, G, oW3);
-    reduce_part_kernel<<<1, 64, 0, s>>>(V.part + kZ, nb, kPartStride, 1, G, oB3);
-    bwd_out_kernel<<<gn, 256, 0, s>>>(n, V.dy, P, V.dH1, V.dA2);
-    // second aggregation (transposed) and message layer
-    PRG_CUDA(cudaMemsetAsync(V.dM1, 0, (size_t)n * 32, s));
-    scatter_kernel<<<gn, 256, 0, s>>>(n, g.row_ptr, g.col, V.dA2, V.S2, V.dM1);
-    bwd_msg_kernel<<<gn, 256, 0, s>>>(n, V.dM1, V.s, P, oWm2, V.H1, V.G1, V.dH1);
-    outer_kernel<kC, kH, 0><<<nb, 256, 0, s>>>(n, V.G1, V.H1, kH, nullptr, 0, V.part, kPartStride);
-    reduce_part_kernel<<<4, 256, 0, s>>>(V.part, nb, kPartStride, kC * kH, G, oWm2);
-    // layer 2 (dH1 now holds dPre1): dW2 over [H0 | A1 (16 incl. zero pad)] = 48
-    // columns, i.e. W2's row layout, followed by b2 = column sums of dPre1
-    outer_kernel<kH, kH, 16><<<nb, 256, 0, s>>>(n, V.dH1, V.H0, kH, V.A1, 16, V.part, kPartStride);
-    reduce_part_kernel<<<8, 256, 0, s>>>(V.part, nb, kPartStride, kH * kZ + kH, G, oW2);
-    bwd_z1_kernel<<<gn, 256, 0, s>>>(n, V.dH1, P, V.dH0, V.dA1);
-    PRG_CUDA(cudaMemsetAsync(V.dM0, 0, (size_t)n * 32, s));
-    scatter_kernel<<<gn, 256, 0, s>>>(n, g.row_ptr, g.col, V.dA1, V.S1, V.dM0);
-    bwd_msg_kernel<<<gn, 256, 0, s>>>(n, V.dM0, V.s, P, oWm1, V.H0, V.G0, V.dH0);
-    outer_kernel<kC, kH, 0><<<nb, 256, 0, s>>>(n, V.G0, V.H0, kH, nullptr, 0, V.part, kPartStride);
-    reduce_part_kernel<<<4, 256, 0, s>>>(V.part, nb, kPartStride, kC * kH, G, oWm1);
-    outer_kernel<kH, kF, 0><<<nb, 256, 0, s>>>(n, V.dH0, V.X0, kF, nullptr, 0, V.part, kPartStride);
-    reduce_part_kernel<<<4, 256, 0, s>>>(V.part, nb, kPartStride, kH * kF + kH, G, oW1);
+    loss_kernel<<<gb, 256, 0, s>>>(V.y, target_internal, n, P, V.S2, V.dy, V.dS2, V.dpart);
+    const uint64_t steps = ((uint64_t)n + kBwdWarps * kVB - 1) / (kBwdWarps * kVB);
+    const unsigned nbt = (unsigned)std::min<uint64_t>(kTopBlocks, steps);
+    const unsigned nbb = (unsigned)std::min<uint64_t>(kBottomBlocks, steps);
+    auto transposed = [&](const float *dS, float *dM) {
+        PRG_CUDA(cudaMemsetAsync(dM, 0, (size_t)n * 32, s));
+        scatter_kernel<<<148 * 8, 256, 0, s>>>(n, g.row_ptr, g.col, dS, dM);
+        scatter_heavy_kernel<<<148 * 2, 256, 0, s>>>(g.row_ptr, g.col, dS, dM, V.heavy, V.nheavy);
+        PRG_CUDA(cudaGetLastError());
+    };
+    transposed(V.dS2, V.dM1);
+    bwd_top_kernel<<<nbt, kBwdThreads, 0, s>>>(n, V.dy, V.dM1, V.s, P, V.H1, V.A2, V.H0, V.A1, V.S1, V.dH0, V.dS1,
+                                              V.part);
+    transposed(V.dS1, V.dM0);
+    bwd_bottom_kernel<<<nbb, kBwdThreads, 0, s>>>(n, V.dM0, V.s, P, V.H0, V.X0, V.dH0, V.part);
+    reduce_part_kernel<<<(kParams + 31) / 32, 256, 0, s>>>(V.part, nbb, nbt, G);
     PRG_CUDA(cudaGetLastError());
     std::vector<double> lp(gb);
     PRG_CUDA(cudaMemcpyAsync(lp.data(), V.dpart, gb * 8, cudaMemcpyDeviceToHost, s));
