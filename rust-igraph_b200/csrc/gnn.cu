@@ -182,8 +182,43 @@ constexpr uint32_t kAggHeavy = 2048;
 
 __device__ __forceinline__ float slog(float z) { return copysignf(log1pf(fabsf(z)), z); }
 
-__global__ void aggregate_kernel(uint32_t n, const uint32_t *row_ptr, const uint32_t *col, const float *M,
-                                 __nv_bfloat16 *out, float *out_f, uint32_t *heavy, uint32_t *nheavy) {
+// One source's 8-channel message (32-byte aligned) in one load: two 16-byte
+// loads would look the same sector up twice in L1.
+__device__ __forceinline__ void ld_msg(const float *p, float (&q)[kC]) {
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(q[0]), "=f"(q[1]), "=f"(q[2]), "=f"(q[3]), "=f"(q[4]), "=f"(q[5]), "=f"(q[6]), "=f"(q[7])
+        : "l"(p));
+}
+
+// acc += the messages of arcs p, p + STRIDE, ... below p1, added one by one in
+// that order, with kAggAhead of them in flight
+constexpr int kAggAhead = 4;
+template <uint32_t STRIDE>
+__device__ __forceinline__ void add_messages(float (&acc)[kC], uint32_t p, uint32_t p1, const uint32_t *col,
+                                             const float *M) {
+    for (; p < p1; p += STRIDE * kAggAhead) {
+        uint32_t u[kAggAhead];
+        float q[kAggAhead][kC];
+#pragma unroll
+        for (int i = 0; i < kAggAhead; i++)
+            if (p + i * STRIDE < p1) u[i] = __ldg(&col[p + i * STRIDE]);
+#pragma unroll
+        for (int i = 0; i < kAggAhead; i++)
+            if (p + i * STRIDE < p1) ld_msg(M + (size_t)u[i] * kC, q[i]);
+#pragma unroll
+        for (int i = 0; i < kAggAhead; i++)
+            if (p + i * STRIDE < p1) {
+#pragma unroll
+                for (int c = 0; c < kC; c++) acc[c] += q[i][c];
+            }
+    }
+}
+
+// out: slog of the sums in BF16, 16 columns of which the last 8 are zero;
+// out_f (null: not wanted): the sums themselves.
+__global__ void __launch_bounds__(256) aggregate_kernel(uint32_t n, const uint32_t *row_ptr, const uint32_t *col,
+                                                        const float *M, __nv_bfloat16 *out, float *out_f,
+                                                        uint32_t *heavy, uint32_t *nheavy) {
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t sub = threadIdx.x & 7;
     const uint32_t group = gid >> 3, ngroups = (gridDim.x * blockDim.x) >> 3;
@@ -200,13 +235,7 @@ __global__ void aggregate_kernel(uint32_t n, const uint32_t *row_ptr, const uint
                 if (sub == 0) heavy[atomicAdd(nheavy, 1u)] = v;
                 skip = true;
             } else {
-                for (uint32_t p = p0 + sub; p < p1; p += 8) {
-                    const uint32_t u = __ldg(&col[p]);
-                    const float4 q0 = __ldg(reinterpret_cast<const float4 *>(M + (size_t)u * kC));
-                    const float4 q1 = __ldg(reinterpret_cast<const float4 *>(M + (size_t)u * kC) + 1);
-                    acc[0] += q0.x; acc[1] += q0.y; acc[2] += q0.z; acc[3] += q0.w;
-                    acc[4] += q1.x; acc[5] += q1.y; acc[6] += q1.z; acc[7] += q1.w;
-                }
+                add_messages<8>(acc, p0 + sub, p1, col, M);
             }
         }
 #pragma unroll
@@ -215,19 +244,23 @@ __global__ void aggregate_kernel(uint32_t n, const uint32_t *row_ptr, const uint
             acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 2);
             acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 1);
         }
-        if (!skip && sub == 0) {
-            uint4 *dst = reinterpret_cast<uint4 *>(out + (size_t)v * 16);
-            dst[0] = make_uint4(pack_bf16(slog(acc[0]), slog(acc[1])), pack_bf16(slog(acc[2]), slog(acc[3])),
-                                pack_bf16(slog(acc[4]), slog(acc[5])), pack_bf16(slog(acc[6]), slog(acc[7])));
-            dst[1] = make_uint4(0u, 0u, 0u, 0u);
-            for (int c = 0; c < kC; c++) out_f[(size_t)v * kC + c] = acc[c];
+        // lane `sub` finishes channel `sub`
+        float mine = acc[0];
+#pragma unroll
+        for (int c = 1; c < kC; c++) mine = sub == (uint32_t)c ? acc[c] : mine;
+        const float z = slog(mine), zn = __shfl_xor_sync(0xffffffffu, z, 1);
+        if (!skip) {
+            uint32_t *dst = reinterpret_cast<uint32_t *>(out + (size_t)v * 16);
+            if ((sub & 1u) == 0u) dst[sub >> 1] = pack_bf16(z, zn);
+            else dst[4 + (sub >> 1)] = 0u;
+            if (out_f) out_f[(size_t)v * kC + sub] = mine;
         }
     }
 }
 
-__global__ void aggregate_heavy_kernel(const uint32_t *row_ptr, const uint32_t *col, const float *M,
-                                       __nv_bfloat16 *out, float *out_f, const uint32_t *heavy,
-                                       const uint32_t *nheavy) {
+__global__ void __launch_bounds__(256) aggregate_heavy_kernel(const uint32_t *row_ptr, const uint32_t *col,
+                                                              const float *M, __nv_bfloat16 *out, float *out_f,
+                                                              const uint32_t *heavy, const uint32_t *nheavy) {
     __shared__ float sh[kC][32];
     const uint32_t cnt = *nheavy;
     for (uint32_t i = blockIdx.x; i < cnt; i += gridDim.x) {
@@ -236,13 +269,7 @@ __global__ void aggregate_heavy_kernel(const uint32_t *row_ptr, const uint32_t *
         float acc[kC];
 #pragma unroll
         for (int c = 0; c < kC; c++) acc[c] = 0.0f;
-        for (uint32_t p = p0 + threadIdx.x; p < p1; p += blockDim.x) {
-            const uint32_t u = __ldg(&col[p]);
-            const float4 q0 = __ldg(reinterpret_cast<const float4 *>(M + (size_t)u * kC));
-            const float4 q1 = __ldg(reinterpret_cast<const float4 *>(M + (size_t)u * kC) + 1);
-            acc[0] += q0.x; acc[1] += q0.y; acc[2] += q0.z; acc[3] += q0.w;
-            acc[4] += q1.x; acc[5] += q1.y; acc[6] += q1.z; acc[7] += q1.w;
-        }
+        add_messages<256>(acc, p0 + threadIdx.x, p1, col, M);
         const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
 #pragma unroll
         for (int c = 0; c < kC; c++) acc[c] = warp_sum(acc[c]);
@@ -255,7 +282,7 @@ __global__ void aggregate_heavy_kernel(const uint32_t *row_ptr, const uint32_t *
             for (int k = 0; k < (int)(blockDim.x >> 5); k++) tot += sh[threadIdx.x][k];
             out[(size_t)v * 16 + threadIdx.x] = __float2bfloat16_rn(slog(tot));
             out[(size_t)v * 16 + 8 + threadIdx.x] = __float2bfloat16_rn(0.0f);
-            out_f[(size_t)v * kC + threadIdx.x] = tot;
+            if (out_f) out_f[(size_t)v * kC + threadIdx.x] = tot;
         }
     }
 }
@@ -710,18 +737,16 @@ __global__ void to_bf16_kernel(const float *P, Ws *w) {
 // rounding points and the mma sequence are those of rowwise_kernel, so the
 // prediction is that of the training forward pass.
 
-__device__ __forceinline__ float feat(uint32_t r, int c, uint32_t n, float ln, const uint32_t *row_ptr,
-                                      const uint32_t *deg) {
-    if (r >= n || c > 5) return 0.0f;
-    const float li = log1pf((float)(row_ptr[r + 1] - row_ptr[r]));
-    const float lo = log1pf((float)deg[r]);
+// Feature c of a vertex from li = log1p(in-degree), lo = log1p(out-degree).
+__device__ __forceinline__ float feat(int c, float li, float lo, float ln, bool dangling) {
     switch (c) {
         case 0: return li * 0.125f;
         case 1: return lo * 0.125f;
-        case 2: return deg[r] == 0 ? 1.0f : 0.0f;
+        case 2: return dangling ? 1.0f : 0.0f;
         case 3: return 1.0f;
         case 4: return (li - lo) * 0.125f;
-        default: return ln;
+        case 5: return ln;
+        default: return 0.0f;
     }
 }
 
@@ -796,11 +821,19 @@ __global__ void __launch_bounds__(128) fused_kernel(uint32_t n, const uint32_t *
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t tile = warp; tile < ntiles; tile += nwarps) {
         const uint32_t r0 = tile * 16 + g, r1 = r0 + 8;
+        // the quad's four logarithms, one per lane: in- and out-degree of both rows
+        const uint32_t rl = t < 2 ? r0 : r1;
+        uint32_t dg = 0;
+        if (rl < n) dg = (t & 1) ? deg[rl] : row_ptr[rl + 1] - row_ptr[rl];
+        const float lg = log1pf((float)dg);
+        const int q0 = lane & ~3;
+        const float li0 = __shfl_sync(0xffffffffu, lg, q0), lo0 = __shfl_sync(0xffffffffu, lg, q0 + 1);
+        const float li1 = __shfl_sync(0xffffffffu, lg, q0 + 2), lo1 = __shfl_sync(0xffffffffu, lg, q0 + 3);
+        const bool z0 = __shfl_sync(0xffffffffu, dg, q0 + 1) == 0u, z1 = __shfl_sync(0xffffffffu, dg, q0 + 3) == 0u;
         uint32_t ax[1][4];
-        ax[0][0] = pack_bf16(feat(r0, 2 * t, n, ln, row_ptr, deg), feat(r0, 2 * t + 1, n, ln, row_ptr, deg));
-        ax[0][1] = pack_bf16(feat(r1, 2 * t, n, ln, row_ptr, deg), feat(r1, 2 * t + 1, n, ln, row_ptr, deg));
-        ax[0][2] = pack_bf16(feat(r0, 2 * t + 8, n, ln, row_ptr, deg), feat(r0, 2 * t + 9, n, ln, row_ptr, deg));
-        ax[0][3] = pack_bf16(feat(r1, 2 * t + 8, n, ln, row_ptr, deg), feat(r1, 2 * t + 9, n, ln, row_ptr, deg));
+        ax[0][0] = r0 < n ? pack_bf16(feat(2 * t, li0, lo0, ln, z0), feat(2 * t + 1, li0, lo0, ln, z0)) : 0u;
+        ax[0][1] = r1 < n ? pack_bf16(feat(2 * t, li1, lo1, ln, z1), feat(2 * t + 1, li1, lo1, ln, z1)) : 0u;
+        ax[0][2] = ax[0][3] = 0u;  // features 8 .. 15
         float acc[4][4];
         layer<4, 1>(acc, ax, sW1, kF, g, t);
         uint32_t ah[3][4];
@@ -1030,10 +1063,9 @@ void Net::predict(const DeviceGraph &g, double *x_internal, cudaStream_t s) {
     for (int layer = 0; layer < 2; layer++) {
         const float *M = layer ? V.M1 : V.M0;
         __nv_bfloat16 *A = layer ? V.A2 : V.A1;
-        float *S = layer ? V.S2 : V.S1;
         PRG_CUDA(cudaMemsetAsync(V.nheavy, 0, 4, s));
-        aggregate_kernel<<<148 * 16, 256, 0, s>>>(n, g.row_ptr, g.col, M, A, S, V.heavy, V.nheavy);
-        aggregate_heavy_kernel<<<148 * 4, 256, 0, s>>>(g.row_ptr, g.col, M, A, S, V.heavy, V.nheavy);
+        aggregate_kernel<<<148 * 16, 256, 0, s>>>(n, g.row_ptr, g.col, M, A, nullptr, V.heavy, V.nheavy);
+        aggregate_heavy_kernel<<<148 * 4, 256, 0, s>>>(g.row_ptr, g.col, M, A, nullptr, V.heavy, V.nheavy);
         PRG_CUDA(cudaGetLastError());
         if (layer == 0) fused<1>(n, g, V.A1, nullptr, W, P, V.s, V.M1, s);
     }
