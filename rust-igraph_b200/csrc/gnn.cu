@@ -214,14 +214,51 @@ __device__ __forceinline__ void add_messages(float (&acc)[kC], uint32_t p, uint3
     }
 }
 
+// Rows of more than kAggHeavy arcs, listed once per forward pass.
+__global__ void heavy_rows_kernel(uint32_t n, const uint32_t *row_ptr, uint32_t *heavy, uint32_t *nheavy) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+        if (row_ptr[v + 1] - row_ptr[v] > kAggHeavy) heavy[atomicAdd(nheavy, 1u)] = v;
+}
+
 // out: slog of the sums in BF16, 16 columns of which the last 8 are zero;
 // out_f (null: not wanted): the sums themselves.
-__global__ void __launch_bounds__(256) aggregate_kernel(uint32_t n, const uint32_t *row_ptr, const uint32_t *col,
-                                                        const float *M, __nv_bfloat16 *out, float *out_f,
-                                                        uint32_t *heavy, uint32_t *nheavy) {
-    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t sub = threadIdx.x & 7;
-    const uint32_t group = gid >> 3, ngroups = (gridDim.x * blockDim.x) >> 3;
+// The first kAggHeavyBlocks blocks take the heavy rows, one at a time, the others
+// the light rows, 8 lanes per row: the longest hub's chain of loads (0.2 ms on
+// R-MAT s22) runs beside the light rows instead of after them in a launch of its
+// own.
+constexpr unsigned kAggHeavyBlocks = 148 * 2, kAggLightBlocks = 148 * 16;
+__global__ void __launch_bounds__(256, 4) aggregate_kernel(uint32_t n, const uint32_t *row_ptr, const uint32_t *col,
+                                                           const float *M, __nv_bfloat16 *out, float *out_f,
+                                                           const uint32_t *heavy, const uint32_t *nheavy) {
+    __shared__ float sh[kC][32];
+    if (blockIdx.x < kAggHeavyBlocks) {
+        const uint32_t cnt = *nheavy;
+        for (uint32_t i = blockIdx.x; i < cnt; i += kAggHeavyBlocks) {
+            const uint32_t v = heavy[i];
+            const uint32_t p0 = row_ptr[v], p1 = row_ptr[v + 1];
+            float acc[kC];
+#pragma unroll
+            for (int c = 0; c < kC; c++) acc[c] = 0.0f;
+            add_messages<256>(acc, p0 + threadIdx.x, p1, col, M);
+            const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+#pragma unroll
+            for (int c = 0; c < kC; c++) acc[c] = warp_sum(acc[c]);
+            __syncthreads();
+            if (l == 0)
+                for (int c = 0; c < kC; c++) sh[c][w] = acc[c];
+            __syncthreads();
+            if (threadIdx.x < kC) {
+                float tot = 0.0f;
+                for (int k = 0; k < (int)(blockDim.x >> 5); k++) tot += sh[threadIdx.x][k];
+                out[(size_t)v * 16 + threadIdx.x] = __float2bfloat16_rn(slog(tot));
+                out[(size_t)v * 16 + 8 + threadIdx.x] = __float2bfloat16_rn(0.0f);
+                if (out_f) out_f[(size_t)v * kC + threadIdx.x] = tot;
+            }
+        }
+        return;
+    }
+    const uint32_t gid = (blockIdx.x - kAggHeavyBlocks) * blockDim.x + threadIdx.x, sub = threadIdx.x & 7;
+    const uint32_t group = gid >> 3, ngroups = ((gridDim.x - kAggHeavyBlocks) * blockDim.x) >> 3;
     const uint32_t rounds = (n + ngroups - 1) / ngroups;
     for (uint32_t rd = 0; rd < rounds; rd++) {
         const uint32_t v = rd * ngroups + group;
@@ -230,13 +267,9 @@ __global__ void __launch_bounds__(256) aggregate_kernel(uint32_t n, const uint32
         for (int c = 0; c < kC; c++) acc[c] = 0.0f;
         bool skip = v >= n;
         if (!skip) {
-            const uint32_t p0 = row_ptr[v], p1 = row_ptr[v + 1];
-            if (p1 - p0 > kAggHeavy) {
-                if (sub == 0) heavy[atomicAdd(nheavy, 1u)] = v;
-                skip = true;
-            } else {
-                add_messages<8>(acc, p0 + sub, p1, col, M);
-            }
+            const uint32_t p0 = __ldg(&row_ptr[v]), p1 = __ldg(&row_ptr[v + 1]);
+            if (p1 - p0 > kAggHeavy) skip = true;
+            else add_messages<8>(acc, p0 + sub, p1, col, M);
         }
 #pragma unroll
         for (int c = 0; c < kC; c++) {
@@ -254,35 +287,6 @@ __global__ void __launch_bounds__(256) aggregate_kernel(uint32_t n, const uint32
             if ((sub & 1u) == 0u) dst[sub >> 1] = pack_bf16(z, zn);
             else dst[4 + (sub >> 1)] = 0u;
             if (out_f) out_f[(size_t)v * kC + sub] = mine;
-        }
-    }
-}
-
-__global__ void __launch_bounds__(256) aggregate_heavy_kernel(const uint32_t *row_ptr, const uint32_t *col,
-                                                              const float *M, __nv_bfloat16 *out, float *out_f,
-                                                              const uint32_t *heavy, const uint32_t *nheavy) {
-    __shared__ float sh[kC][32];
-    const uint32_t cnt = *nheavy;
-    for (uint32_t i = blockIdx.x; i < cnt; i += gridDim.x) {
-        const uint32_t v = heavy[i];
-        const uint32_t p0 = row_ptr[v], p1 = row_ptr[v + 1];
-        float acc[kC];
-#pragma unroll
-        for (int c = 0; c < kC; c++) acc[c] = 0.0f;
-        add_messages<256>(acc, p0 + threadIdx.x, p1, col, M);
-        const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-#pragma unroll
-        for (int c = 0; c < kC; c++) acc[c] = warp_sum(acc[c]);
-        __syncthreads();
-        if (l == 0)
-            for (int c = 0; c < kC; c++) sh[c][w] = acc[c];
-        __syncthreads();
-        if (threadIdx.x < kC) {
-            float tot = 0.0f;
-            for (int k = 0; k < (int)(blockDim.x >> 5); k++) tot += sh[threadIdx.x][k];
-            out[(size_t)v * 16 + threadIdx.x] = __float2bfloat16_rn(slog(tot));
-            out[(size_t)v * 16 + 8 + threadIdx.x] = __float2bfloat16_rn(0.0f);
-            if (out_f) out_f[(size_t)v * kC + threadIdx.x] = tot;
         }
     }
 }
@@ -737,17 +741,12 @@ __global__ void to_bf16_kernel(const float *P, Ws *w) {
 // rounding points and the mma sequence are those of rowwise_kernel, so the
 // prediction is that of the training forward pass.
 
-// Feature c of a vertex from li = log1p(in-degree), lo = log1p(out-degree).
-__device__ __forceinline__ float feat(int c, float li, float lo, float ln, bool dangling) {
-    switch (c) {
-        case 0: return li * 0.125f;
-        case 1: return lo * 0.125f;
-        case 2: return dangling ? 1.0f : 0.0f;
-        case 3: return 1.0f;
-        case 4: return (li - lo) * 0.125f;
-        case 5: return ln;
-        default: return 0.0f;
-    }
+// Features 2t, 2t + 1 of a vertex in BF16 (features_kernel's, zero from 6 on),
+// from li = log1p(in-degree), lo = log1p(out-degree).
+__device__ __forceinline__ uint32_t feat_pair(int t, float li, float lo, float ln, bool dangling) {
+    const uint32_t f01 = pack_bf16(li * 0.125f, lo * 0.125f), f45 = pack_bf16((li - lo) * 0.125f, ln);
+    const uint32_t f23 = dangling ? 0x3F803F80u : 0x3F800000u;  // (dangling ? 1 : 0, 1)
+    return t == 0 ? f01 : t == 1 ? f23 : t == 2 ? f45 : 0u;
 }
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -757,36 +756,52 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// acc[j] += A(k-tiles) x W^T for n-tiles j < NT; W row-major [N x K] in smem
+// B fragments of W [8 NT x K] (row-major, k-tiles from kt0): two registers per
+// n-tile and k-tile, loaded once per thread (a warp's weight tiles read from
+// shared memory in every row tile kept the L1 data pipe 81 % busy with 2- and
+// 4-way bank conflicts: 95 / 156 / 156 us per stage on R-MAT s22).
 template <int NT, int KT>
-__device__ __forceinline__ void layer(float (&acc)[NT][4], const uint32_t (&a)[KT][4], const __nv_bfloat16 *sW,
-                                      int K, int g, int t) {
+struct BFrag {
+    uint32_t b[KT][NT][2];
+    __device__ __forceinline__ void load(const __nv_bfloat16 *W, int K, int g, int t) {
+#pragma unroll
+        for (int kt = 0; kt < KT; kt++) {
+#pragma unroll
+            for (int j = 0; j < NT; j++) {
+                const __nv_bfloat16 *w = W + (j * 8 + g) * K + kt * 16 + 2 * t;
+                b[kt][j][0] = __ldg(reinterpret_cast<const uint32_t *>(w));
+                b[kt][j][1] = __ldg(reinterpret_cast<const uint32_t *>(w + 8));
+            }
+        }
+    }
+};
+
+// acc[j] = A(k-tiles) x W^T for n-tiles j < NT
+template <int NT, int KT>
+__device__ __forceinline__ void layer(float (&acc)[NT][4], const uint32_t (&a)[KT][4], const BFrag<NT, KT> &w) {
 #pragma unroll
     for (int j = 0; j < NT; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
 #pragma unroll
     for (int kt = 0; kt < KT; kt++) {
 #pragma unroll
-        for (int j = 0; j < NT; j++) {
-            const int col = j * 8 + g;
-            const uint32_t b0 = *reinterpret_cast<const uint32_t *>(sW + col * K + kt * 16 + 2 * t);
-            const uint32_t b1 = *reinterpret_cast<const uint32_t *>(sW + col * K + kt * 16 + 2 * t + 8);
-            mma_bf16(acc[j], a[kt], b0, b1);
-        }
+        for (int j = 0; j < NT; j++) mma_bf16(acc[j], a[kt], w.b[kt][j][0], w.b[kt][j][1]);
     }
 }
 
-// relu(acc + bias) -> BF16 A fragments of the next layer (32 columns = 2 k-tiles)
-__device__ __forceinline__ void to_afrag(const float (&acc)[4][4], const float *bias, int t, uint32_t (&a)[2][4]) {
+// relu(acc + bias) -> BF16 A fragments of the next layer (32 columns = 2
+// k-tiles); bias: the lane's columns 2t, 2t+1 of each n-tile
+template <int KT>
+__device__ __forceinline__ void to_afrag(const float (&acc)[4][4], const float2 (&bias)[4], uint32_t (&a)[KT][4]) {
 #pragma unroll
     for (int kt = 0; kt < 2; kt++) {
         float v[2][4];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const int j = 2 * kt + h, c0 = j * 8 + 2 * t;
-            v[h][0] = fmaxf(acc[j][0] + bias[c0], 0.0f);
-            v[h][1] = fmaxf(acc[j][1] + bias[c0 + 1], 0.0f);
-            v[h][2] = fmaxf(acc[j][2] + bias[c0], 0.0f);
-            v[h][3] = fmaxf(acc[j][3] + bias[c0 + 1], 0.0f);
+            const int j = 2 * kt + h;
+            v[h][0] = fmaxf(acc[j][0] + bias[j].x, 0.0f);
+            v[h][1] = fmaxf(acc[j][1] + bias[j].y, 0.0f);
+            v[h][2] = fmaxf(acc[j][2] + bias[j].x, 0.0f);
+            v[h][3] = fmaxf(acc[j][3] + bias[j].y, 0.0f);
         }
         a[kt][0] = pack_bf16(v[0][0], v[0][1]);
         a[kt][1] = pack_bf16(v[0][2], v[0][3]);
@@ -795,103 +810,120 @@ __device__ __forceinline__ void to_afrag(const float (&acc)[4][4], const float *
     }
 }
 
-__device__ __forceinline__ uint32_t ld_pair(const __nv_bfloat16 *A, uint32_t r, uint32_t n, int k) {
-    return r < n ? *reinterpret_cast<const uint32_t *>(A + (size_t)r * 16 + k) : 0u;
-}
+// What a tile of 16 rows reads, loaded one tile ahead.
+template <int STAGE>
+struct TileIn {
+    uint32_t dg = 0;              // this lane's of the quad's four degrees
+    uint32_t a1[2] = {0u, 0u}, a2[2] = {0u, 0u};
+    float sc[2] = {0.0f, 0.0f};
+    __device__ __forceinline__ void load(uint32_t tile, uint32_t n, int g, int t, const uint32_t *row_ptr,
+                                         const uint32_t *deg, const __nv_bfloat16 *A1, const __nv_bfloat16 *A2,
+                                         const float *scale) {
+        const uint32_t r0 = tile * 16 + g, r1 = r0 + 8, rl = t < 2 ? r0 : r1;
+        dg = 0;
+        if (rl < n) dg = (t & 1) ? __ldg(deg + rl) : __ldg(row_ptr + rl + 1) - __ldg(row_ptr + rl);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint32_t r = h ? r1 : r0;
+            a1[h] = a2[h] = 0u;
+            sc[h] = 0.0f;
+            if (r >= n) continue;
+            if (STAGE >= 1) a1[h] = __ldg(reinterpret_cast<const uint32_t *>(A1 + (size_t)r * 16 + 2 * t));
+            if (STAGE >= 2) a2[h] = __ldg(reinterpret_cast<const uint32_t *>(A2 + (size_t)r * 16 + 2 * t));
+            if (STAGE <= 1) sc[h] = __ldg(scale + r);
+        }
+    }
+};
 
 // STAGE 0: write M0 = s * (H0 Wm1^T); 1: write M1; 2: write y
+// Each warp keeps the inputs of the next tiles in flight; more than one in the
+// later stages costs the registers of a resident block (four blocks with three
+// tiles ahead: 143 / 149 us, five with two spill: 159 / 223 us).
+constexpr int fused_ahead(int stage) { return stage == 0 ? 3 : 1; }
+constexpr unsigned fused_per_sm(int stage) { return stage == 0 ? 7 : 5; }
 template <int STAGE>
-__global__ void __launch_bounds__(128) fused_kernel(uint32_t n, const uint32_t *row_ptr, const uint32_t *deg,
-                                                    const __nv_bfloat16 *A1, const __nv_bfloat16 *A2, const Ws *Wg,
-                                                    const float *P, const float *scale, float *out) {
-    __shared__ __align__(16) __nv_bfloat16 sW1[kH * kF], sWm[kC * kH], sW2[kH * kZ], sW3[8 * kZ];
-    __shared__ float sb1[kH], sb2[kH];
-    for (int i = threadIdx.x; i < kH * kF; i += blockDim.x) sW1[i] = Wg->W1[i];
-    for (int i = threadIdx.x; i < kC * kH; i += blockDim.x) sWm[i] = STAGE == 0 ? Wg->Wm1[i] : Wg->Wm2[i];
-    for (int i = threadIdx.x; i < kH * kZ; i += blockDim.x) sW2[i] = Wg->W2[i];
-    for (int i = threadIdx.x; i < 8 * kZ; i += blockDim.x) sW3[i] = Wg->W3[i];
-    for (int i = threadIdx.x; i < kH; i += blockDim.x) {
-        sb1[i] = P[oB1 + i];
-        sb2[i] = P[oB2 + i];
-    }
-    __syncthreads();
+__global__ void __launch_bounds__(128, fused_per_sm(STAGE)) fused_kernel(uint32_t n, const uint32_t *row_ptr, const uint32_t *deg,
+                                                       const __nv_bfloat16 *A1, const __nv_bfloat16 *A2, const Ws *Wg,
+                                                       const float *P, const float *scale, float *out) {
     const float ln = logf((float)n) * 0.0625f;
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    BFrag<4, 1> w1;
+    w1.load(Wg->W1, kF, g, t);
+    BFrag<4, 3> w2;
+    BFrag<1, 2> wm;
+    BFrag<1, 3> w3;
+    float2 b1[4], b2[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        b1[j] = make_float2(P[oB1 + j * 8 + 2 * t], P[oB1 + j * 8 + 2 * t + 1]);
+        b2[j] = make_float2(P[oB2 + j * 8 + 2 * t], P[oB2 + j * 8 + 2 * t + 1]);
+    }
+    if (STAGE >= 1) w2.load(Wg->W2, kZ, g, t);
+    if (STAGE <= 1) wm.load(STAGE == 0 ? Wg->Wm1 : Wg->Wm2, kH, g, t);
+    if (STAGE == 2) w3.load(Wg->W3, kZ, g, t);
+    const float b3 = P[oB3];
     const uint32_t ntiles = (n + 15) / 16;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t tile = warp; tile < ntiles; tile += nwarps) {
+    constexpr int kFusedAhead = fused_ahead(STAGE);
+    TileIn<STAGE> ring[kFusedAhead];
+#pragma unroll
+    for (int i = 0; i < kFusedAhead; i++)
+        if ((uint64_t)warp + (uint64_t)i * nwarps < ntiles)
+            ring[i].load(warp + i * nwarps, n, g, t, row_ptr, deg, A1, A2, scale);
+    auto work = [&](uint32_t tile, TileIn<STAGE> &slot) {
+        const TileIn<STAGE> in = slot;
+        if ((uint64_t)tile + (uint64_t)kFusedAhead * nwarps < ntiles)
+            slot.load(tile + kFusedAhead * nwarps, n, g, t, row_ptr, deg, A1, A2, scale);
         const uint32_t r0 = tile * 16 + g, r1 = r0 + 8;
         // the quad's four logarithms, one per lane: in- and out-degree of both rows
-        const uint32_t rl = t < 2 ? r0 : r1;
-        uint32_t dg = 0;
-        if (rl < n) dg = (t & 1) ? deg[rl] : row_ptr[rl + 1] - row_ptr[rl];
-        const float lg = log1pf((float)dg);
+        const float lg = log1pf((float)in.dg);
         const int q0 = lane & ~3;
         const float li0 = __shfl_sync(0xffffffffu, lg, q0), lo0 = __shfl_sync(0xffffffffu, lg, q0 + 1);
         const float li1 = __shfl_sync(0xffffffffu, lg, q0 + 2), lo1 = __shfl_sync(0xffffffffu, lg, q0 + 3);
-        const bool z0 = __shfl_sync(0xffffffffu, dg, q0 + 1) == 0u, z1 = __shfl_sync(0xffffffffu, dg, q0 + 3) == 0u;
+        const bool z0 = __shfl_sync(0xffffffffu, in.dg, q0 + 1) == 0u, z1 = __shfl_sync(0xffffffffu, in.dg, q0 + 3) == 0u;
         uint32_t ax[1][4];
-        ax[0][0] = r0 < n ? pack_bf16(feat(2 * t, li0, lo0, ln, z0), feat(2 * t + 1, li0, lo0, ln, z0)) : 0u;
-        ax[0][1] = r1 < n ? pack_bf16(feat(2 * t, li1, lo1, ln, z1), feat(2 * t + 1, li1, lo1, ln, z1)) : 0u;
+        ax[0][0] = r0 < n ? feat_pair(t, li0, lo0, ln, z0) : 0u;
+        ax[0][1] = r1 < n ? feat_pair(t, li1, lo1, ln, z1) : 0u;
         ax[0][2] = ax[0][3] = 0u;  // features 8 .. 15
         float acc[4][4];
-        layer<4, 1>(acc, ax, sW1, kF, g, t);
+        layer<4, 1>(acc, ax, w1);
         uint32_t ah[3][4];
-        {
-            uint32_t h0[2][4];
-            to_afrag(acc, sb1, t, h0);
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                ah[0][q] = h0[0][q];
-                ah[1][q] = h0[1][q];
-            }
-        }
+        to_afrag(acc, b1, ah);
         if constexpr (STAGE >= 1) {
-            // k-tile 2 of [H0 | A1]
-            ah[2][0] = ld_pair(A1, r0, n, 2 * t);
-            ah[2][1] = ld_pair(A1, r1, n, 2 * t);
-            ah[2][2] = ld_pair(A1, r0, n, 2 * t + 8);
-            ah[2][3] = ld_pair(A1, r1, n, 2 * t + 8);
-            layer<4, 3>(acc, ah, sW2, kZ, g, t);
-            uint32_t h1[2][4];
-            to_afrag(acc, sb2, t, h1);
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                ah[0][q] = h1[0][q];
-                ah[1][q] = h1[1][q];
-            }
+            // k-tile 2 of [H0 | A1] (its columns 8 .. 15 are zero)
+            ah[2][0] = in.a1[0];
+            ah[2][1] = in.a1[1];
+            ah[2][2] = ah[2][3] = 0u;
+            layer<4, 3>(acc, ah, w2);
+            to_afrag(acc, b2, ah);
         }
         if constexpr (STAGE <= 1) {
+            const uint32_t a2[2][4] = {{ah[0][0], ah[0][1], ah[0][2], ah[0][3]}, {ah[1][0], ah[1][1], ah[1][2], ah[1][3]}};
             float m[1][4];
-            uint32_t a2[2][4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                a2[0][q] = ah[0][q];
-                a2[1][q] = ah[1][q];
-            }
-            layer<1, 2>(m, a2, sWm, kH, g, t);
-            const int c0 = 2 * t;
-            if (r0 < n) {
-                const float sc = scale[r0];
-                out[(size_t)r0 * kC + c0] = m[0][0] * sc;
-                out[(size_t)r0 * kC + c0 + 1] = m[0][1] * sc;
-            }
-            if (r1 < n) {
-                const float sc = scale[r1];
-                out[(size_t)r1 * kC + c0] = m[0][2] * sc;
-                out[(size_t)r1 * kC + c0 + 1] = m[0][3] * sc;
-            }
+            layer<1, 2>(m, a2, wm);
+            if (r0 < n)
+                *reinterpret_cast<float2 *>(out + (size_t)r0 * kC + 2 * t) =
+                    make_float2(m[0][0] * in.sc[0], m[0][1] * in.sc[0]);
+            if (r1 < n)
+                *reinterpret_cast<float2 *>(out + (size_t)r1 * kC + 2 * t) =
+                    make_float2(m[0][2] * in.sc[1], m[0][3] * in.sc[1]);
         } else {
-            ah[2][0] = ld_pair(A2, r0, n, 2 * t);
-            ah[2][1] = ld_pair(A2, r1, n, 2 * t);
-            ah[2][2] = ld_pair(A2, r0, n, 2 * t + 8);
-            ah[2][3] = ld_pair(A2, r1, n, 2 * t + 8);
+            ah[2][0] = in.a2[0];
+            ah[2][1] = in.a2[1];
+            ah[2][2] = ah[2][3] = 0u;
             float yv[1][4];
-            layer<1, 3>(yv, ah, sW3, kZ, g, t);
+            layer<1, 3>(yv, ah, w3);
             if (t == 0) {
-                if (r0 < n) out[r0] = yv[0][0] + P[oB3];
-                if (r1 < n) out[r1] = yv[0][2] + P[oB3];
+                if (r0 < n) out[r0] = yv[0][0] + b3;
+                if (r1 < n) out[r1] = yv[0][2] + b3;
             }
+        }
+    };
+    for (uint32_t tile = warp; tile < ntiles;) {
+#pragma unroll
+        for (int i = 0; i < kFusedAhead; i++) {
+            if (tile < ntiles) work(tile, ring[i]);
+            tile += nwarps;
         }
     }
 }
@@ -900,7 +932,7 @@ template <int STAGE>
 static void fused(uint32_t n, const DeviceGraph &g, const __nv_bfloat16 *A1, const __nv_bfloat16 *A2, const Ws *W,
                   const float *P, const float *scale, float *out, cudaStream_t s) {
     const uint32_t tiles = (n + 15) / 16;
-    const unsigned grid = (unsigned)std::max<uint32_t>(1, std::min<uint32_t>((tiles + 3) / 4, 148u * 16u));
+    const unsigned grid = (unsigned)std::max<uint32_t>(1, std::min<uint32_t>((tiles + 3) / 4, 148u * fused_per_sm(STAGE)));
     fused_kernel<STAGE><<<grid, 128, 0, s>>>(n, g.row_ptr, g.deg, A1, A2, W, P, scale, out);
     PRG_CUDA(cudaGetLastError());
 }
@@ -1033,6 +1065,8 @@ void Net::forward(const DeviceGraph &g, cudaStream_t s) {
     const unsigned gn = grid_n(n);
     features_kernel<<<gn, 256, 0, s>>>(n, g.row_ptr, g.deg, V.X0);
     scale_kernel<<<gn, 256, 0, s>>>(g.deg, n, V.s);
+    PRG_CUDA(cudaMemsetAsync(V.nheavy, 0, 4, s));
+    heavy_rows_kernel<<<gn, 256, 0, s>>>(n, g.row_ptr, V.heavy, V.nheavy);
     PRG_CUDA(cudaGetLastError());
     rowwise<kF, 0, kH, EPI_RELU_BF16>(n, V.X0, nullptr, W->W1, P + oB1, nullptr, V.H0, nullptr, s);
     rowwise<kH, 0, kC, EPI_SCALE_F32>(n, V.H0, nullptr, W->Wm1, nullptr, V.s, nullptr, V.M0, s);
@@ -1040,9 +1074,8 @@ void Net::forward(const DeviceGraph &g, cudaStream_t s) {
         const float *M = layer ? V.M1 : V.M0;
         __nv_bfloat16 *A = layer ? V.A2 : V.A1;
         float *S = layer ? V.S2 : V.S1;
-        PRG_CUDA(cudaMemsetAsync(V.nheavy, 0, 4, s));
-        aggregate_kernel<<<148 * 16, 256, 0, s>>>(n, g.row_ptr, g.col, M, A, S, V.heavy, V.nheavy);
-        aggregate_heavy_kernel<<<148 * 4, 256, 0, s>>>(g.row_ptr, g.col, M, A, S, V.heavy, V.nheavy);
+        aggregate_kernel<<<kAggHeavyBlocks + kAggLightBlocks, 256, 0, s>>>(n, g.row_ptr, g.col, M, A, S, V.heavy,
+                                                                           V.nheavy);
         PRG_CUDA(cudaGetLastError());
         if (layer == 0) {
             rowwise<kH, 16, kH, EPI_RELU_BF16>(n, V.H0, V.A1, W->W2, P + oB2, nullptr, V.H1, nullptr, s);
@@ -1059,13 +1092,14 @@ void Net::predict(const DeviceGraph &g, double *x_internal, cudaStream_t s) {
     const Ws *W = (const Ws *)w;
     const uint32_t n = g.n;
     scale_kernel<<<grid_n(n), 256, 0, s>>>(g.deg, n, V.s);
+    PRG_CUDA(cudaMemsetAsync(V.nheavy, 0, 4, s));
+    heavy_rows_kernel<<<grid_n(n), 256, 0, s>>>(n, g.row_ptr, V.heavy, V.nheavy);
     fused<0>(n, g, nullptr, nullptr, W, P, V.s, V.M0, s);
     for (int layer = 0; layer < 2; layer++) {
         const float *M = layer ? V.M1 : V.M0;
         __nv_bfloat16 *A = layer ? V.A2 : V.A1;
-        PRG_CUDA(cudaMemsetAsync(V.nheavy, 0, 4, s));
-        aggregate_kernel<<<148 * 16, 256, 0, s>>>(n, g.row_ptr, g.col, M, A, nullptr, V.heavy, V.nheavy);
-        aggregate_heavy_kernel<<<148 * 4, 256, 0, s>>>(g.row_ptr, g.col, M, A, nullptr, V.heavy, V.nheavy);
+        aggregate_kernel<<<kAggHeavyBlocks + kAggLightBlocks, 256, 0, s>>>(n, g.row_ptr, g.col, M, A, nullptr,
+                                                                           V.heavy, V.nheavy);
         PRG_CUDA(cudaGetLastError());
         if (layer == 0) fused<1>(n, g, V.A1, nullptr, W, P, V.s, V.M1, s);
     }
