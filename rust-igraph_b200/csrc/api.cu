@@ -371,7 +371,7 @@ int32_t check_weights(const double *w, uint64_t m) {
 bool small_dropin(prg::SmallCall &c, double *out, int32_t *rc, double *eigenvalue = nullptr) {
     const prg::Tuning &t = prg::tuning();
     const bool seg = c.kind == prg::RES_EIG ? t.seg_eig64 != 0 : t.seg_plain64 != 0;
-    if (!t.resident || !(c.w || seg) || c.m > 0xFFFFFFFFull || check_sizes(c.n, c.m, c.directed) != PRG_OK) return false;
+    if (!t.resident || !seg || c.m > 0xFFFFFFFFull || check_sizes(c.n, c.m, c.directed) != PRG_OK) return false;
     if (!ensure_pool_config()) return false;
     cudaStream_t s = prg::stream_acquire();
     prg::SmallResult r;

@@ -72,7 +72,7 @@ void workspace_free(Workspace &ws, cudaStream_t s) {
 // The tile-segmented passes' index, when this graph uses one.
 static void seg_ensure(Workspace &ws, const DeviceGraph &g, cudaStream_t s) {
     const bool any = g.seg_kry32 != 0 || g.seg_res64 != 0 || g.seg_plain64 != 0 || g.seg_eig64 != 0;
-    if (!g.weighted && any && g.arcs > 0 && ws.seg.mask == nullptr) seg_build(g, ws.seg, s);
+    if (any && g.arcs > 0 && ws.seg.mask == nullptr) seg_build(g, ws.seg, s);
 }
 
 void workspace_ensure(Workspace &ws, const DeviceGraph &g, cudaStream_t s, bool need_seg) {
@@ -91,10 +91,10 @@ void workspace_ensure(Workspace &ws, const DeviceGraph &g, cudaStream_t s, bool 
     ws.nrb = g.nrb;
     ws.nhub = g.nhub;
     unsigned gmax = kPrepParts;
-    const bool seg = !g.weighted && g.seg_kry32 != 0 && g.arcs > 0;
-    const bool seg_res = !g.weighted && g.seg_res64 != 0 && g.arcs > 0;
-    const bool seg_plain = !g.weighted && g.seg_plain64 != 0 && g.arcs > 0;
-    const bool seg_eig = !g.weighted && g.seg_eig64 != 0 && g.arcs > 0;
+    const bool seg = g.seg_kry32 != 0 && g.arcs > 0;
+    const bool seg_res = g.seg_res64 != 0 && g.arcs > 0;
+    const bool seg_plain = g.seg_plain64 != 0 && g.arcs > 0;
+    const bool seg_eig = g.seg_eig64 != 0 && g.arcs > 0;
     for (int m = 0; m < kModes; m++) {
         const bool fp32 = m == MODE_CORR32 || m == MODE_KRY32;
         // (a hot prefix holds whole quads, so fewer than 4 vertices have none)
@@ -242,7 +242,7 @@ void to_f32(const double *a, float *b, uint32_t n, cudaStream_t s) {
 }
 
 ResPlan resident_plan(Workspace &ws, const DeviceGraph &g, int kind, cudaStream_t s) {
-    const bool on = g.resident != 0 && (g.weighted || (kind == RES_EIG ? g.seg_eig64 : g.seg_plain64) != 0);
+    const bool on = g.resident != 0 && (kind == RES_EIG ? g.seg_eig64 : g.seg_plain64) != 0;
     if (!on) return ResPlan{};
     if (!ws.res_planned[kind]) {
         ws.res_plan[kind] = res_plan(g, kind, s);
