@@ -10,11 +10,11 @@
 // individually: a converged column keeps its last iterate and is no longer
 // written.
 //
-// Layout: columns are processed in tiles of W = 32*VEC.  A tile's iterate X
-// and scaled iterate XT = X / outdeg live vertex-major (row v = W floats), so
-// the gather of one source vertex is one coalesced 128*VEC-byte load of a
-// warp: lane l owns columns [l*VEC, l*VEC+VEC).  One warp handles one
-// destination row at a time.  Reset vectors are sparse: a per-vertex seed
+// Layout: columns are processed in tiles of W = LPR*VEC, 32*vec wide but for
+// the last one.  A tile's iterate X and scaled iterate XT = X / outdeg live
+// vertex-major (row v = W floats), so the gather of one source vertex is one
+// coalesced 4*W-byte load of LPR lanes: lane l owns columns [l*VEC, l*VEC+VEC).
+// A group of LPR lanes handles one destination row at a time.  Reset vectors are sparse: a per-vertex seed
 // list (vertex-sorted CSR of (column, weight) entries).
 //
 // Undirected graphs can take Chebyshev semi-iteration in place of the plain
@@ -194,16 +194,24 @@ __device__ __forceinline__ void stv(float *p, const Vec<VEC> &x) {
 }
 
 // Reduces per-lane (diff, dsum) of the block's warps into bpart[block][col].
-template <int VEC>
+template <int VEC, int LPR>
 __device__ __forceinline__ void block_columns(const TileArgs &a, const double (&pd)[VEC], const double (&pds)[VEC],
                                               double *sh) {
-    constexpr int W = 32 * VEC;
+    constexpr int W = LPR * VEC;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < VEC; j++) {
-        sh[(warp * W + lane * VEC + j) * 2] = pd[j];
-        sh[(warp * W + lane * VEC + j) * 2 + 1] = pds[j];
+        double x = pd[j], y = pds[j];
+#pragma unroll
+        for (int o = LPR; o < 32; o *= 2) {  // over the warp's rows
+            x += __shfl_xor_sync(0xffffffffu, x, o);
+            y += __shfl_xor_sync(0xffffffffu, y, o);
+        }
+        if (lane < LPR) {
+            sh[(warp * W + lane * VEC + j) * 2] = x;
+            sh[(warp * W + lane * VEC + j) * 2 + 1] = y;
+        }
     }
     __syncthreads();
     for (int c = threadIdx.x; c < W; c += blockDim.x) {
@@ -219,9 +227,8 @@ __device__ __forceinline__ void block_columns(const TileArgs &a, const double (&
 
 // Column totals over blocks (fixed order) -> column state.  Block b handles
 // columns b, b + gridDim.x, ...  `init`: only record the dangling mass.
-template <int VEC>
+template <int W>
 __device__ __forceinline__ void reduce_columns(const TileArgs &a, int parity_new, bool init, double *sh) {
-    constexpr int W = 32 * VEC;
     for (uint32_t c = blockIdx.x; c < a.tile_w; c += gridDim.x) {
         double x = 0.0, y = 0.0;
         for (uint32_t b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
@@ -304,14 +311,14 @@ __device__ __forceinline__ void reduce_columns(const TileArgs &a, int parity_new
     }
 }
 
-template <int VEC>
+template <int VEC, int LPR>
 __global__ void __launch_bounds__(kBThreads) ppr_tile_kernel(const TileArgs a) {
-    constexpr int W = 32 * VEC;
+    constexpr int W = LPR * VEC;
     __shared__ double sh[kBWarps * W * 2];
     __shared__ int s_any;
-    const int lane = threadIdx.x & 31;
-    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+    const int lane = threadIdx.x % LPR;
+    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) / LPR;
+    const uint32_t nw = (gridDim.x * blockDim.x) / LPR;
     const float d = (float)a.damping;
 
     // dangling mass of the start vectors (the resets)
@@ -325,9 +332,9 @@ __global__ void __launch_bounds__(kBThreads) ppr_tile_kernel(const TileArgs a) {
 #pragma unroll
             for (int j = 0; j < VEC; j++) pds[j] += (double)x.v[j];
         }
-        block_columns<VEC>(a, pd, pds, sh);
+        block_columns<VEC, LPR>(a, pd, pds, sh);
         if (!grid_sync(a)) return;
-        reduce_columns<VEC>(a, 0, true, sh);
+        reduce_columns<W>(a, 0, true, sh);
         if (!grid_sync(a)) return;
     }
 
@@ -370,15 +377,36 @@ __global__ void __launch_bounds__(kBThreads) ppr_tile_kernel(const TileArgs a) {
             float acc[VEC], cmp[VEC];
 #pragma unroll
             for (int j = 0; j < VEC; j++) acc[j] = cmp[j] = 0.0f;
-            for (uint32_t base = p0; base < p1; base += 32) {
-                const uint32_t cnt = min(32u, p1 - base);
-                const uint32_t mine = lane < cnt ? __ldg(&a.col[base + lane]) : 0u;
-                uint32_t k = 0;
-                for (; k + 4 <= cnt; k += 4) {
-                    const uint32_t u0 = __shfl_sync(0xffffffffu, mine, k);
-                    const uint32_t u1 = __shfl_sync(0xffffffffu, mine, k + 1);
-                    const uint32_t u2 = __shfl_sync(0xffffffffu, mine, k + 2);
-                    const uint32_t u3 = __shfl_sync(0xffffffffu, mine, k + 3);
+            if constexpr (LPR == 32) {
+                for (uint32_t base = p0; base < p1; base += 32) {
+                    const uint32_t cnt = min(32u, p1 - base);
+                    const uint32_t mine = lane < cnt ? __ldg(&a.col[base + lane]) : 0u;
+                    uint32_t k = 0;
+                    for (; k + 4 <= cnt; k += 4) {
+                        const uint32_t u0 = __shfl_sync(0xffffffffu, mine, k);
+                        const uint32_t u1 = __shfl_sync(0xffffffffu, mine, k + 1);
+                        const uint32_t u2 = __shfl_sync(0xffffffffu, mine, k + 2);
+                        const uint32_t u3 = __shfl_sync(0xffffffffu, mine, k + 3);
+                        const Vec<VEC> g0 = ldv_cg<VEC>(XT + (size_t)u0 * W + lane * VEC);
+                        const Vec<VEC> g1 = ldv_cg<VEC>(XT + (size_t)u1 * W + lane * VEC);
+                        const Vec<VEC> g2 = ldv_cg<VEC>(XT + (size_t)u2 * W + lane * VEC);
+                        const Vec<VEC> g3 = ldv_cg<VEC>(XT + (size_t)u3 * W + lane * VEC);
+    #pragma unroll
+                        for (int j = 0; j < VEC; j++) kahan_add(acc[j], cmp[j], (g0.v[j] + g1.v[j]) + (g2.v[j] + g3.v[j]));
+                    }
+                    for (; k < cnt; k++) {
+                        const uint32_t u = __shfl_sync(0xffffffffu, mine, k);
+                        const Vec<VEC> g = ldv_cg<VEC>(XT + (size_t)u * W + lane * VEC);
+    #pragma unroll
+                        for (int j = 0; j < VEC; j++) kahan_add(acc[j], cmp[j], g.v[j]);
+                    }
+                }
+            } else {
+                // the row's lanes read each index together (one L1 access)
+                uint32_t p = p0;
+                for (; p + 4 <= p1; p += 4) {
+                    const uint32_t u0 = __ldg(&a.col[p]), u1 = __ldg(&a.col[p + 1]);
+                    const uint32_t u2 = __ldg(&a.col[p + 2]), u3 = __ldg(&a.col[p + 3]);
                     const Vec<VEC> g0 = ldv_cg<VEC>(XT + (size_t)u0 * W + lane * VEC);
                     const Vec<VEC> g1 = ldv_cg<VEC>(XT + (size_t)u1 * W + lane * VEC);
                     const Vec<VEC> g2 = ldv_cg<VEC>(XT + (size_t)u2 * W + lane * VEC);
@@ -386,9 +414,8 @@ __global__ void __launch_bounds__(kBThreads) ppr_tile_kernel(const TileArgs a) {
 #pragma unroll
                     for (int j = 0; j < VEC; j++) kahan_add(acc[j], cmp[j], (g0.v[j] + g1.v[j]) + (g2.v[j] + g3.v[j]));
                 }
-                for (; k < cnt; k++) {
-                    const uint32_t u = __shfl_sync(0xffffffffu, mine, k);
-                    const Vec<VEC> g = ldv_cg<VEC>(XT + (size_t)u * W + lane * VEC);
+                for (; p < p1; p++) {
+                    const Vec<VEC> g = ldv_cg<VEC>(XT + (size_t)__ldg(&a.col[p]) * W + lane * VEC);
 #pragma unroll
                     for (int j = 0; j < VEC; j++) kahan_add(acc[j], cmp[j], g.v[j]);
                 }
@@ -426,9 +453,9 @@ __global__ void __launch_bounds__(kBThreads) ppr_tile_kernel(const TileArgs a) {
             stv<VEC>(a.X[xn_] + (size_t)v * W + lane * VEC, xn);
             stv<VEC>(a.XT[nxt] + (size_t)v * W + lane * VEC, xtn);
         }
-        block_columns<VEC>(a, pd, pds, sh);
+        block_columns<VEC, LPR>(a, pd, pds, sh);
         if (!grid_sync(a)) return;
-        reduce_columns<VEC>(a, xn_, false, sh);
+        reduce_columns<W>(a, xn_, false, sh);
         if (!grid_sync(a)) return;
     }
 }
@@ -473,18 +500,35 @@ __global__ void tile_writeback(const float *X0, const float *X1, const float *X2
     }
 }
 
-template <int VEC>
-static void run_tile(const TileArgs &a, int grid, cudaStream_t s) {
-    void *args[] = {(void *)&a};
-    PRG_CUDA(cudaLaunchCooperativeKernel((const void *)ppr_tile_kernel<VEC>, dim3(grid), dim3(kBThreads), args, 0, s));
+// The kernel for tiles of `width` columns.
+struct TileShape {
+    const void *kernel;
+    uint32_t width;
+};
+template <int VEC, int LPR>
+static TileShape tile_kernel() {
+    return {(const void *)ppr_tile_kernel<VEC, LPR>, VEC * LPR};
+}
+// The narrowest tile of at least `columns` columns, at most 32 vec wide: the
+// pass is bound by the bytes it gathers, so a ragged last tile should not move
+// columns it does not have.  n = 1 M, 20 M arcs, 50 iterations: 8 columns
+// 7.2 ms, 16 12.2, 32 21.3 (32 lanes of one column each: 33), 64 40.0; all of
+// them took 40 in a 64-wide tile, and 200 columns went from 160 to 130 ms.  The
+// 64-wide tile keeps a warp to a row: half-warps of float4 need 78 registers
+// (48) and measured 55 ms, loads of eight arcs ahead 45-72, a cp.async ring 44.
+static TileShape tile_shape(uint32_t vec, uint32_t columns) {
+    if (columns <= 8) return tile_kernel<2, 4>();
+    if (columns <= 16) return tile_kernel<2, 8>();
+    if (columns <= 32 || vec == 1) return tile_kernel<2, 16>();
+    if (columns <= 64 || vec == 2) return tile_kernel<2, 32>();
+    return tile_kernel<4, 32>();
 }
 
-template <int VEC>
-static int tile_grid() {
+static int tile_grid(const TileShape &t) {
     int dev = 0, sms = 0, occ = 0;
     PRG_CUDA(cudaGetDevice(&dev));
     PRG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    PRG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ppr_tile_kernel<VEC>, kBThreads, 0));
+    PRG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, t.kernel, kBThreads, 0));
     return sms * std::max(occ, 1);
 }
 
@@ -494,7 +538,6 @@ int ppr_batch(const DeviceGraph &g, uint32_t K, const uint64_t *seed_offsets, co
     st = BatchStats{};
     const uint32_t n = g.n;
     if (vec != 1 && vec != 2 && vec != 4) vec = 1;
-    const uint32_t W = 32 * vec;
     // the persistent launch keeps every block resident: lane-per-row gathers
     // need the graph's ids < n and the column tiles below
     // seed entries (vertex, column, weight), weight 1/len like
@@ -538,6 +581,9 @@ int ppr_batch(const DeviceGraph &g, uint32_t K, const uint64_t *seed_offsets, co
     PRG_CUDA(cudaMemcpyAsync(sptr, hptr.data(), ((size_t)n + 1) * 4, cudaMemcpyHostToDevice, s));
     uint32_t *kk = ev;
 
+    // full tiles, and the ragged last one in the narrowest tile that holds it
+    const TileShape full = tile_shape(vec, K), last = tile_shape(vec, K % full.width ? K % full.width : full.width);
+    const uint32_t W = full.width;
     // tile buffers (Chebyshev steps need a third iterate)
     const bool cheb = !g.directed && tuning().batch_cheb != 0;
     float *X[3] = {nullptr, nullptr, nullptr}, *XT[2];
@@ -548,7 +594,7 @@ int ppr_batch(const DeviceGraph &g, uint32_t K, const uint64_t *seed_offsets, co
     if (cheb) {
         A((void **)&X[2], (size_t)n * W * 4);
     }
-    const int grid = vec == 4 ? tile_grid<4>() : vec == 2 ? tile_grid<2>() : tile_grid<1>();
+    const int grid_full = tile_grid(full), grid_last = tile_grid(last), grid = std::max(grid_full, grid_last);
     ColState *cs = nullptr;
     double *bpart = nullptr;
     uint32_t *bar = nullptr;
@@ -563,8 +609,9 @@ int ppr_batch(const DeviceGraph &g, uint32_t K, const uint64_t *seed_offsets, co
     PRG_CUDA(cudaEventRecord(e0, s));
     int rc = 0;
     std::vector<ColState> hcs(W);
-    for (uint32_t tb = 0; tb < K && rc == 0; tb += W) {
-        const uint32_t tw = std::min(W, K - tb);
+    for (uint32_t tb = 0; tb < K && rc == 0; tb += full.width) {
+        const TileShape &shape = tb + full.width < K ? full : last;
+        const uint32_t W = shape.width, tw = std::min(W, K - tb);
         PRG_CUDA(cudaMemsetAsync(X[0], 0, (size_t)n * W * 4, s));
         seed_fill<<<std::max<uint32_t>(1, (uint32_t)std::min<uint64_t>((S + 255) / 256, 4096)), 256, 0, s>>>(
             kk, ecs, ews, (uint32_t)S, tb, W, X[0]);
@@ -602,9 +649,9 @@ int ppr_batch(const DeviceGraph &g, uint32_t K, const uint64_t *seed_offsets, co
         a.damping = damping;
         a.tol = tol;
         a.bar_extra = tuning().batch_barrier_extra;
-        if (vec == 4) run_tile<4>(a, grid, s);
-        else if (vec == 2) run_tile<2>(a, grid, s);
-        else run_tile<1>(a, grid, s);
+        void *args[] = {(void *)&a};
+        PRG_CUDA(cudaLaunchCooperativeKernel(shape.kernel, dim3(&shape == &full ? grid_full : grid_last),
+                                             dim3(kBThreads), args, 0, s));
         tile_writeback<<<148 * 8, 256, 0, s>>>(X[0], X[1], X[2], cs, n, W, tw, tb, K, g.perm, d_out);
         PRG_CUDA(cudaGetLastError());
         int32_t hs = 0;
