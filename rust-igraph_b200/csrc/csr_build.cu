@@ -130,114 +130,145 @@ void exclusive_scan_u32(const uint32_t *in, uint32_t *out, uint64_t n, cudaStrea
 
 // ------------------------------------------------------------------ radix sort
 
+constexpr int kRsThreads = 512;
 constexpr int kRsItems = 8;
-constexpr int kRsTile = kThreads * kRsItems;  // 2048 keys
-constexpr int kRsWarps = kThreads / 32;
+constexpr int kRsTile = kRsThreads * kRsItems;  // 4096 pairs
+constexpr int kRsWarps = kRsThreads / 32;
 
 __global__ void __launch_bounds__(kThreads) rs_upsweep(const uint32_t *keys, uint64_t N, uint64_t chunk, int shift,
-                                                       uint32_t *counts, uint32_t G) {
-    __shared__ uint32_t h[kRsWarps][256];
-    for (int i = threadIdx.x; i < kRsWarps * 256; i += kThreads) (&h[0][0])[i] = 0;
+                                                       int bits, uint32_t *counts, uint32_t G) {
+    __shared__ uint32_t h[kThreads / 32][256];
+    for (int i = threadIdx.x; i < kThreads * 8; i += kThreads) (&h[0][0])[i] = 0;
     __syncthreads();
+    const uint32_t mask = (1u << bits) - 1u;
     uint64_t begin = (uint64_t)blockIdx.x * chunk;
     uint64_t end = begin + chunk < N ? begin + chunk : N;
     int w = threadIdx.x >> 5;
     for (uint64_t i = begin + threadIdx.x; i < end; i += kThreads) {
-        uint32_t d = (keys[i] >> shift) & 255u;
+        uint32_t d = (keys[i] >> shift) & mask;
         atomicAdd(&h[w][d], 1u);
     }
     __syncthreads();
     uint32_t t = threadIdx.x;
     uint32_t s = 0;
 #pragma unroll
-    for (int k = 0; k < kRsWarps; k++) s += h[k][t];
-    counts[(uint64_t)t * G + blockIdx.x] = s;
+    for (int k = 0; k < kThreads / 32; k++) s += h[k][t];
+    if (t <= mask) counts[(uint64_t)t * G + blockIdx.x] = s;
 }
 
 // Stable scatter: each chunk is processed tile by tile; within a tile keys
-// are ranked per warp with __match_any_sync in position order, then ordered
-// by digit in shared memory and written out in digit runs (coalesced).
-__global__ void __launch_bounds__(kThreads) rs_downsweep(const uint32_t *kin, const uint32_t *vin, uint32_t *kout,
-                                                         uint32_t *vout, uint64_t N, uint64_t chunk, int shift,
-                                                         const uint32_t *offsets, uint32_t G) {
-    __shared__ uint32_t s_wh[kRsWarps][256];
-    __shared__ uint32_t s_keys[kRsTile];
-    __shared__ uint32_t s_vals[kRsTile];
-    __shared__ uint32_t s_cnt[256];
-    __shared__ uint32_t s_dstart[256];
-    __shared__ uint32_t s_off[256];
-    __shared__ uint32_t s_scan[33];
-
+// are ranked per warp in position order, then ordered by digit in shared
+// memory and written out in digit runs (coalesced).  Bound by the instructions
+// and shared-memory accesses of the ranking, not by memory (67 M pairs: 1.07 GB,
+// 0.16 ms at the copy rate).  So the lanes with equal digits are found by
+// ballots over the digit's bits, for all of a lane's keys before the first
+// count is read (match.any: 0.49 ms against 0.39), key and value move through
+// shared memory as one word, a digit's place in the tile is folded into the
+// warps' counts, and two blocks of 64 registers a thread, which spill nothing,
+// share an SM (three of 40: 0.45; 16 keys per lane 0.55).  67 M pairs, R-MAT
+// scale 22 heads, passes of 8, 7 and 7 bits: 0.58 + 0.51 + 0.51 ms (8 bits each,
+// tiles of 2048, match.any) before, 0.49 + 0.36 + 0.36 now.
+template <int BITS>
+struct RsShared {
+    uint2 pairs[kRsTile];
+    uint32_t at[kRsWarps][1 << BITS];  // a warp's count of each digit, then the place of its first in the tile
+    uint32_t base[1 << BITS];          // of the digit's run in the output, less its start in the tile
+    uint32_t scan[33];
+};
+template <int BITS>
+__global__ void __launch_bounds__(kRsThreads, 2) rs_downsweep(const uint32_t *kin, const uint32_t *vin,
+                                                              uint32_t *kout, uint32_t *vout, uint64_t N,
+                                                              uint64_t chunk, int shift, int bits,
+                                                              const uint32_t *offsets, uint32_t G) {
+    extern __shared__ __align__(16) unsigned char s_rs[];
+    RsShared<BITS> &sh = *reinterpret_cast<RsShared<BITS> *>(s_rs);
+    constexpr int kDigits = 1 << BITS;
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const uint32_t mask = (1u << bits) - 1u;
     uint64_t begin = (uint64_t)blockIdx.x * chunk;
     uint64_t end = begin + chunk < N ? begin + chunk : N;
-    s_off[tid] = offsets[(uint64_t)tid * G + blockIdx.x];
+    uint32_t off = (uint32_t)tid <= mask ? offsets[(uint64_t)tid * G + blockIdx.x] : 0u;
     const uint32_t ltmask = lanemask_lt();
+    const uint32_t first = w * (32 * kRsItems) + lane;  // this lane's first key of a tile
 
     for (uint64_t tb = begin; tb < end; tb += kRsTile) {
-        for (int i = tid; i < kRsWarps * 256; i += kThreads) (&s_wh[0][0])[i] = 0;
-        __syncthreads();
-        uint32_t key[kRsItems], val[kRsItems], dig[kRsItems], rank[kRsItems];
+        uint32_t key[kRsItems], val[kRsItems], peers[kRsItems];
+        const uint32_t nvalid = (uint32_t)min((uint64_t)kRsTile, end - tb);
+        const uint32_t *kt = kin + tb + first, *vt = vin + tb + first;
+#pragma unroll
+        for (int i = 0; i < kRsItems; i++) key[i] = first + 32 * i < nvalid ? __ldcs(kt + 32 * i) : 0u;
+#pragma unroll
+        for (int i = 0; i < kRsItems; i++) val[i] = first + 32 * i < nvalid ? __ldcs(vt + 32 * i) : 0u;
+        for (int i = lane; i < kDigits; i += 32) sh.at[w][i] = 0;
 #pragma unroll
         for (int i = 0; i < kRsItems; i++) {
-            uint64_t pos = tb + (uint64_t)w * (32 * kRsItems) + (uint64_t)i * 32 + lane;
-            bool valid = pos < end;
-            key[i] = valid ? kin[pos] : 0u;
-            val[i] = valid ? vin[pos] : 0u;
-            dig[i] = valid ? ((key[i] >> shift) & 255u) : 256u;
+            const uint32_t d = key[i] >> shift;
+            uint32_t p = __ballot_sync(0xffffffffu, first + 32 * i < nvalid);
+#pragma unroll
+            for (int b = 0; b < BITS; b++) {
+                const uint32_t one = (uint32_t)((int32_t)((d & mask) << (31 - b)) >> 31);  // the bit, 32 times
+                p &= ~(__ballot_sync(0xffffffffu, one) ^ one);
+            }
+            peers[i] = p;
         }
+        __syncwarp();
 #pragma unroll
         for (int i = 0; i < kRsItems; i++) {
-            uint32_t d = dig[i];
-            uint32_t peers = __match_any_sync(0xffffffffu, d);
-            uint32_t before = d < 256u ? s_wh[w][d] : 0u;
+            const uint32_t before = sh.at[w][key[i] >> shift & mask], rank = __popc(peers[i] & ltmask);
             __syncwarp();
-            if (d < 256u && (peers & ltmask) == 0u) s_wh[w][d] = before + __popc(peers);
+            if (first + 32 * i < nvalid && rank == 0u) sh.at[w][key[i] >> shift & mask] = before + __popc(peers[i]);
             __syncwarp();
-            rank[i] = before + __popc(peers & ltmask);
+            peers[i] = before + rank;  // the key's place among the warp's keys of its digit
         }
         __syncthreads();
-        {  // per digit: exclusive prefix across warps, tile count
-            uint32_t run = 0;
+        uint32_t cnt = 0, tot;
+        if (tid < kDigits) {
+#pragma unroll
+            for (int k = 0; k < kRsWarps; k++) cnt += sh.at[k][tid];
+        }
+        uint32_t ds = block_excl_scan(cnt, sh.scan, &tot);
+        if (tid < kDigits) {
+            sh.base[tid] = off - ds;
+            off += cnt;
 #pragma unroll
             for (int k = 0; k < kRsWarps; k++) {
-                uint32_t c = s_wh[k][tid];
-                s_wh[k][tid] = run;
-                run += c;
+                const uint32_t c = sh.at[k][tid];
+                sh.at[k][tid] = ds;
+                ds += c;
             }
-            s_cnt[tid] = run;
         }
         __syncthreads();
-        uint32_t tot;
-        uint32_t ds = block_excl_scan(s_cnt[tid], s_scan, &tot);
-        s_dstart[tid] = ds;
+#pragma unroll
+        for (int i = 0; i < kRsItems; i++)
+            if (first + 32 * i < nvalid)
+                sh.pairs[sh.at[w][key[i] >> shift & mask] + peers[i]] = make_uint2(key[i], val[i]);
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < kRsItems; i++) {
-            uint32_t d = dig[i];
-            if (d < 256u) {
-                uint32_t lp = s_dstart[d] + s_wh[w][d] + rank[i];
-                s_keys[lp] = key[i];
-                s_vals[lp] = val[i];
+            const uint32_t j = tid + i * kRsThreads;
+            if (j < nvalid) {
+                const uint2 p = sh.pairs[j];
+                const uint32_t gpos = sh.base[p.x >> shift & mask] + j;
+                kout[gpos] = p.x;
+                vout[gpos] = p.y;
             }
         }
-        __syncthreads();
-        uint32_t nvalid = tot;
-        for (uint32_t j = tid; j < nvalid; j += kThreads) {
-            uint32_t k = s_keys[j];
-            uint32_t d = (k >> shift) & 255u;
-            uint64_t gpos = (uint64_t)s_off[d] + (j - s_dstart[d]);
-            kout[gpos] = k;
-            vout[gpos] = s_vals[j];
-        }
-        __syncthreads();
-        s_off[tid] += s_cnt[tid];
         __syncthreads();
     }
 }
 
-// Stable passes over the 8-bit digits at shifts first_shift, +8, ... below
-// key_bits.  The first pass reads (keys, vals), which stay as they are, and
+template <int BITS>
+static void launch_downsweep(uint64_t G, const uint32_t *keys, const uint32_t *vals, uint32_t *kout, uint32_t *vout,
+                             uint64_t N, uint64_t chunk, int shift, int bits, const uint32_t *counts, cudaStream_t s) {
+    constexpr int smem = (int)sizeof(RsShared<BITS>);
+    PRG_CUDA(cudaFuncSetAttribute(rs_downsweep<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    rs_downsweep<BITS><<<(unsigned)G, kRsThreads, smem, s>>>(keys, vals, kout, vout, N, chunk, shift, bits, counts,
+                                                             (uint32_t)G);
+}
+
+// Stable passes over the key's bits from first_shift up to key_bits, in as few
+// digits of at most 8 bits as it takes, the bits spread evenly (fewer digits:
+// longer runs to write).  The first pass reads (keys, vals), which stay as they are, and
 // writes (k[0], v[0]); later ones go back and forth between k[0], v[0] and
 // k[1], v[1] (k[1], v[1] may be the source itself, which is then lost).  The
 // result is in *keys / *vals, the source when there is nothing to sort.
@@ -253,12 +284,13 @@ static void radix_passes(const uint32_t **keys, const uint32_t **vals, uint32_t 
     uint64_t chunk = chunk_tiles * kRsTile;
     G = (N + chunk - 1) / chunk;
     uint32_t *counts = dalloc<uint32_t>(256 * G + 1, s);  // + the scan's total
-    int to = 0;
-    for (int shift = first_shift; shift < key_bits; shift += 8, to ^= 1) {
-        rs_upsweep<<<(unsigned)G, kThreads, 0, s>>>(*keys, N, chunk, shift, counts, (uint32_t)G);
-        exclusive_scan_u32(counts, counts, 256 * G, s);  // in place: each tile is loaded before it is written
-        rs_downsweep<<<(unsigned)G, kThreads, 0, s>>>(*keys, *vals, k[to], v[to], N, chunk, shift, counts,
-                                                     (uint32_t)G);
+    int to = 0, left = radix_pass_count(N, first_shift, key_bits);
+    for (int shift = first_shift, bits; shift < key_bits; shift += bits, to ^= 1, left--) {
+        bits = (key_bits - shift + left - 1) / left;
+        rs_upsweep<<<(unsigned)G, kThreads, 0, s>>>(*keys, N, chunk, shift, bits, counts, (uint32_t)G);
+        exclusive_scan_u32(counts, counts, G << bits, s);  // in place: each tile is loaded before it is written
+        (bits > 7 ? launch_downsweep<8> : launch_downsweep<7>)(G, *keys, *vals, k[to], v[to], N, chunk, shift, bits,
+                                                               counts, s);
         PRG_CUDA(cudaGetLastError());
         *keys = k[to];
         *vals = v[to];
