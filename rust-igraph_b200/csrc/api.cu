@@ -103,16 +103,6 @@ bool ensure_pool_config() {
     return true;
 }
 
-// Checks that every endpoint is < n (Graph::add_edges rejects others with
-// IgraphError::VertexOutOfRange, graph.rs:756-785).
-__global__ void max_endpoint_kernel(const uint32_t *a, const uint32_t *b, uint64_t m, uint32_t *out) {
-    uint32_t mx = 0;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x)
-        mx = max(mx, max(a[i], b[i]));
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, mx);
-}
-
 // Size checks shared by both ways of creating a handle.
 static int32_t check_sizes(uint32_t n, uint64_t m, int32_t directed) {
     if (m > 0xFFFFFFFFull) return fail(PRG_ERR_INTERNAL, "ecount overflows u32");
@@ -166,21 +156,13 @@ int32_t create_from_device(uint32_t n, uint64_t m, const uint32_t *d_from, const
     const int32_t rc = check_sizes(n, m, directed);
     if (rc != PRG_OK) return rc;
     prg_graph *h = new_handle(n, m, directed, s, relabel);
-    if (m > 0) {
-        uint32_t *d_mx = nullptr, mx = 0;
-        PRG_CUDA(cudaMallocAsync((void **)&d_mx, 4, s));
-        PRG_CUDA(cudaMemsetAsync(d_mx, 0, 4, s));
-        max_endpoint_kernel<<<148 * 8, 256, 0, s>>>(d_from, d_to, m, d_mx);
-        PRG_CUDA(cudaGetLastError());
-        PRG_CUDA(cudaMemcpyAsync(&mx, d_mx, 4, cudaMemcpyDeviceToHost, s));
-        PRG_CUDA(cudaFreeAsync(d_mx, s));
-        PRG_CUDA(cudaStreamSynchronize(s));
-        if (mx >= n) {
-            delete h;
-            return fail(PRG_ERR_VERTEX_OUT_OF_RANGE, range_message(mx, n));
-        }
+    // every endpoint must be < n (Graph::add_edges rejects others with
+    // IgraphError::VertexOutOfRange, graph.rs:756-785)
+    uint32_t mx = 0;
+    if (!prg::build_graph(h->g, d_from, d_to, d_w, s, &mx)) {
+        delete h;
+        return fail(PRG_ERR_VERTEX_OUT_OF_RANGE, range_message(mx, n));
     }
-    prg::build_graph(h->g, d_from, d_to, d_w, s);
     *out = h;
     return PRG_OK;
 }

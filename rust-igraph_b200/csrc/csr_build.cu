@@ -358,12 +358,24 @@ void preload_gather_f64() {
 // nothing: a vertex without in-arcs rarely has a large out-degree (none with
 // out-degree >= 16 among the 2.2 M of R-MAT scale 22).
 
-__global__ void max_u32_kernel(const uint32_t *a, uint32_t n, uint32_t *out) {
+// One atomic per block: an atomic per warp to one word took 50 us at 4 M
+// entries, ten times the read.
+template <int THREADS>
+__device__ __forceinline__ void block_atomic_max(uint32_t mx, uint32_t *out) {
+    __shared__ uint32_t sh[THREADS / 32];
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < THREADS / 32; w++) mx = max(mx, sh[w]);
+        atomicMax(out, mx);
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) max_u32_kernel(const uint32_t *a, uint32_t n, uint32_t *out) {
     uint32_t mx = 0;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) mx = max(mx, a[v]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, mx);
+    block_atomic_max<kThreads>(mx, out);
 }
 
 // noin: 1 for a vertex without in-arcs (null: out-degree alone); it is the
@@ -413,23 +425,43 @@ __global__ void make_arcs(const uint32_t *from, const uint32_t *to, uint64_t m, 
 // generators, and any degree-sorted numbering, put them there); their counts
 // are first gathered in a per-block shared-memory histogram so thousands of
 // updates to one hub do not serialise on a single L2 address.
-constexpr uint32_t kDegBins = 12288;
+constexpr uint32_t kDegBins = 12224;  // 47.75 KB, the rest of 48 for the block maximum
 constexpr int kDegThreads = 1024;
 
+// The same pass finds the largest endpoint.
+constexpr int kDegItems = 4;  // edges of a thread, loaded before any is used
+
 __global__ void __launch_bounds__(kDegThreads) out_degree_kernel(const uint32_t *from, const uint32_t *to, uint64_t m,
-                                                                 bool directed, uint32_t n, uint32_t *deg) {
+                                                                 bool directed, uint32_t n, uint32_t *deg,
+                                                                 uint32_t *max_endpoint) {
     __shared__ uint32_t bins[kDegBins];
     for (uint32_t i = threadIdx.x; i < kDegBins; i += kDegThreads) bins[i] = 0u;
     __syncthreads();
+    uint32_t mx = 0u;
     auto add = [&](uint32_t v) {
-        if (v >= n) return;  // out-of-range ids are reported by the caller's range check
+        if (v >= n) return;  // out-of-range ids are reported through max_endpoint
         if (v < kDegBins) atomicAdd_block(&bins[v], 1u);
         else atomicAdd(&deg[v], 1u);
     };
-    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
-        add(from[e]);
-        if (!directed) add(to[e]);
+    const uint64_t step = (uint64_t)gridDim.x * kDegThreads * kDegItems;
+    for (uint64_t b = (uint64_t)blockIdx.x * kDegThreads * kDegItems + threadIdx.x; b < m; b += step) {
+        uint32_t f[kDegItems], t[kDegItems];
+#pragma unroll
+        for (int j = 0; j < kDegItems; j++) {
+            const uint64_t e = b + (uint64_t)j * kDegThreads;
+            f[j] = e < m ? __ldcs(from + e) : 0u;
+            t[j] = e < m ? __ldcs(to + e) : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < kDegItems; j++) {
+            mx = max(mx, max(f[j], t[j]));
+            if (b + (uint64_t)j * kDegThreads < m) {
+                add(f[j]);
+                if (!directed) add(t[j]);
+            }
+        }
     }
+    block_atomic_max<kDegThreads>(mx, max_endpoint);
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < kDegBins && i < n; i += kDegThreads)
         if (bins[i]) atomicAdd(&deg[i], bins[i]);
@@ -558,17 +590,16 @@ __global__ void finish_degrees(uint32_t n, const uint32_t *deg, double *strength
         inv32[v] = d > 0.0 ? (float)(1.0 / d) : 0.0f;
         cnt += d == 0.0 ? 1u : 0u;
     }
-    cnt = warp_sum(cnt);
-    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(n_dangling, cnt);
+    __shared__ uint32_t sh[32];
+    cnt = block_sum<uint32_t>(cnt, sh);
+    if (threadIdx.x == 0 && cnt) atomicAdd(n_dangling, cnt);
 }
 
-__global__ void max_degree_kernel(const uint32_t *row_ptr, uint32_t n, uint32_t *out) {
+__global__ void __launch_bounds__(kThreads) max_degree_kernel(const uint32_t *row_ptr, uint32_t n, uint32_t *out) {
     uint32_t mx = 0;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
         mx = max(mx, row_ptr[v + 1] - row_ptr[v]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, mx);
+    block_atomic_max<kThreads>(mx, out);
 }
 
 // ------------------------------------------------------------------ row-blocks
@@ -686,13 +717,13 @@ static int bits_for(uint32_t maxkey) {
 // entries, freed here) holds the out-strengths.
 static void finish_graph(DeviceGraph &g, double *&strength, cudaStream_t s) {
     const uint32_t n = g.n;
-    const unsigned gn = grid_for(n, kThreads);
+    const unsigned gr = grid_for(n, kThreads, 148u * 8u);  // one atomic per block
     PRG_CUDA(cudaMallocAsync((void **)&g.dval, std::max<uint64_t>(n, 1) * 8, s));
     PRG_CUDA(cudaMallocAsync((void **)&g.inv32, std::max<uint64_t>(n, 1) * 4, s));
     uint32_t *d_nd = dalloc<uint32_t>(2, s);
     PRG_CUDA(cudaMemsetAsync(d_nd, 0, 8, s));
-    finish_degrees<<<gn, kThreads, 0, s>>>(n, g.deg, strength, g.weighted, g.dval, g.inv32, d_nd);
-    max_degree_kernel<<<gn, kThreads, 0, s>>>(g.row_ptr, n, d_nd + 1);
+    finish_degrees<<<gr, kThreads, 0, s>>>(n, g.deg, strength, g.weighted, g.dval, g.inv32, d_nd);
+    max_degree_kernel<<<gr, kThreads, 0, s>>>(g.row_ptr, n, d_nd + 1);
     PRG_CUDA(cudaGetLastError());
     uint32_t hnd[2];
     PRG_CUDA(cudaMemcpyAsync(hnd, d_nd, 8, cudaMemcpyDeviceToHost, s));
@@ -715,7 +746,7 @@ static bool relabel_vertices(DeviceGraph &g, cudaStream_t s, const uint32_t *in_
     const unsigned gn = grid_for(n, kThreads);
     uint32_t *d_mx = dalloc<uint32_t>(1, s), maxdeg = 0;
     PRG_CUDA(cudaMemsetAsync(d_mx, 0, 4, s));
-    max_u32_kernel<<<gn, kThreads, 0, s>>>(g.deg, n, d_mx);
+    max_u32_kernel<<<std::min(gn, 148u * 8u), kThreads, 0, s>>>(g.deg, n, d_mx);
     PRG_CUDA(cudaMemcpyAsync(&maxdeg, d_mx, 4, cudaMemcpyDeviceToHost, s));
     PRG_CUDA(cudaStreamSynchronize(s));
     dfree(d_mx, s);
@@ -747,7 +778,8 @@ static bool relabel_vertices(DeviceGraph &g, cudaStream_t s, const uint32_t *in_
     return true;
 }
 
-void build_graph(DeviceGraph &g, const uint32_t *d_from, const uint32_t *d_to, const double *d_w, cudaStream_t s) {
+bool build_graph(DeviceGraph &g, const uint32_t *d_from, const uint32_t *d_to, const double *d_w, cudaStream_t s,
+                 uint32_t *max_endpoint) {
     cudaEvent_t e0, e1;
     PRG_CUDA(cudaEventCreate(&e0));
     PRG_CUDA(cudaEventCreate(&e1));
@@ -765,7 +797,22 @@ void build_graph(DeviceGraph &g, const uint32_t *d_from, const uint32_t *d_to, c
     // out-degree (unweighted divisor; also kept for weighted graphs)
     PRG_CUDA(cudaMallocAsync((void **)&g.deg, std::max<uint64_t>(n, 1) * 4, s));
     PRG_CUDA(cudaMemsetAsync(g.deg, 0, std::max<uint64_t>(n, 1) * 4, s));
-    if (m) out_degree_kernel<<<148 * 2, kDegThreads, 0, s>>>(d_from, d_to, m, directed, n, g.deg);
+    *max_endpoint = 0;
+    if (m) {
+        uint32_t *d_mx = dalloc<uint32_t>(1, s);
+        PRG_CUDA(cudaMemsetAsync(d_mx, 0, 4, s));
+        out_degree_kernel<<<148 * 2, kDegThreads, 0, s>>>(d_from, d_to, m, directed, n, g.deg, d_mx);
+        PRG_CUDA(cudaGetLastError());
+        PRG_CUDA(cudaMemcpyAsync(max_endpoint, d_mx, 4, cudaMemcpyDeviceToHost, s));
+        dfree(d_mx, s);
+        PRG_CUDA(cudaStreamSynchronize(s));
+        if (*max_endpoint >= n) {  // nothing below runs on ids out of range
+            dfree(g.deg, s);
+            cudaEventDestroy(e0);
+            cudaEventDestroy(e1);
+            return false;
+        }
+    }
 
     // Arcs in edge order, stably sorted by destination, in caller ids: a
     // directed unweighted edge list is sorted as it is.  Relabelling afterwards
@@ -865,6 +912,7 @@ void build_graph(DeviceGraph &g, const uint32_t *d_from, const uint32_t *d_to, c
     PRG_CUDA(cudaEventElapsedTime(&g.build_ms, e0, e1));
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    return true;
 }
 
 // ------------------------------------------------------------------ streamed build from host edges
@@ -994,9 +1042,7 @@ bool build_graph_host(DeviceGraph &g, const uint32_t *h_from, const uint32_t *h_
         PRG_CUDA(cudaEventRecord(ev[c], cs));
         PRG_CUDA(cudaStreamWaitEvent(s, ev[c], 0));
         const unsigned gl = grid_for(len, kThreads), gla = grid_for(la, kThreads);
-        max_u32_kernel<<<gl, kThreads, 0, s>>>(d_from + b, (uint32_t)len, d_mx);
-        max_u32_kernel<<<gl, kThreads, 0, s>>>(d_to + b, (uint32_t)len, d_mx);
-        out_degree_kernel<<<148 * 2, kDegThreads, 0, s>>>(d_from + b, d_to + b, len, directed, n, g.deg);
+        out_degree_kernel<<<148 * 2, kDegThreads, 0, s>>>(d_from + b, d_to + b, len, directed, n, g.deg, d_mx);
         make_arcs<<<gl, kThreads, 0, s>>>(d_from + b, d_to + b, len, directed, true, ka, va);
         uint32_t *k0 = ka, *v0 = va, *k1 = kb, *v1 = vb;
         radix_sort_pairs(&k0, &v0, &k1, &v1, la, key_bits, s);

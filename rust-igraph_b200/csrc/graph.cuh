@@ -74,8 +74,10 @@ struct DeviceGraph {
 // Builds the in-CSR, degrees and row-blocks from device edge arrays.
 // d_w may be null (unweighted).  All work is on `s`; temporaries use the
 // stream-ordered allocator.
-void build_graph(DeviceGraph &g, const uint32_t *d_from, const uint32_t *d_to, const double *d_w,
-                 cudaStream_t s);
+// Returns false, with nothing built, when an endpoint is >= n (its maximum in
+// *max_endpoint).
+bool build_graph(DeviceGraph &g, const uint32_t *d_from, const uint32_t *d_to, const double *d_w, cudaStream_t s,
+                 uint32_t *max_endpoint);
 // The same graph from HOST edge arrays, streamed: chunks of the edge list are
 // copied on a side stream and sorted on arrival while the next chunk is in
 // flight, then one scan and one scatter finish the CSR (identical to
