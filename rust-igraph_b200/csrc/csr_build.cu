@@ -1000,7 +1000,7 @@ __global__ void place_arcs(const uint32_t *pos, const uint32_t *val, uint64_t ar
 }
 
 bool build_graph_host(DeviceGraph &g, const uint32_t *h_from, const uint32_t *h_to, const double *h_w, cudaStream_t s,
-                      uint32_t *max_endpoint) {
+                      uint32_t *max_endpoint, DeviceEdges *keep) {
     cudaEvent_t e0, e1;
     PRG_CUDA(cudaEventCreate(&e0));
     PRG_CUDA(cudaEventCreate(&e1));
@@ -1129,8 +1129,12 @@ bool build_graph_host(DeviceGraph &g, const uint32_t *h_from, const uint32_t *h_
         row_weight_sums<<<grid_for((uint64_t)n * 32, kThreads), kThreads, 0, s>>>(g.row_ptr, g.w64, nullptr, n,
                                                                                nullptr, strength);
     }
-    dfree(d_from, s);
-    dfree(d_to, s);
+    if (keep) {
+        *keep = DeviceEdges{d_from, d_to};
+    } else {
+        dfree(d_from, s);
+        dfree(d_to, s);
+    }
     dfree(d_w, s);
     dfree(cnt, s);
     dfree(base, s);

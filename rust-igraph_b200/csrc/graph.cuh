@@ -84,8 +84,13 @@ bool build_graph(DeviceGraph &g, const uint32_t *d_from, const uint32_t *d_to, c
 // build_graph's).  Not for directed weighted graphs (their out-strengths
 // need a second sort by source).  Returns false, with nothing built, when
 // an endpoint is >= n (its maximum in *max_endpoint).
+// With `keep`, the uploaded edge list stays on the device and is the caller's
+// to free on s.
+struct DeviceEdges {
+    uint32_t *from = nullptr, *to = nullptr;
+};
 bool build_graph_host(DeviceGraph &g, const uint32_t *h_from, const uint32_t *h_to, const double *h_w, cudaStream_t s,
-                      uint32_t *max_endpoint);
+                      uint32_t *max_endpoint, DeviceEdges *keep = nullptr);
 constexpr uint64_t kStreamChunks = 16;             // chunks of the streamed build
 constexpr uint64_t kStreamChunkMin = 1ull << 22;   // smallest chunk (edges)
 constexpr uint64_t kStreamMinEdges = 1ull << 23;   // smaller edge lists take the one-shot build
