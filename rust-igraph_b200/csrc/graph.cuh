@@ -49,7 +49,7 @@ struct DeviceGraph {
     uint32_t seg_kry32 = 2, seg_hot = 32768;
     // ... and the FP64 residual pass of the refined / Krylov solves, with a
     // hot prefix of seg_hot64 entries
-    uint32_t seg_res64 = 1, seg_hot64 = 8192;
+    uint32_t seg_res64 = 1, seg_hot64 = 12288;
     // ... and the FP64 power step of the drop-ins and the certified loop, and
     // the FP64 Krylov matvec
     uint32_t seg_plain64 = 1;
@@ -111,7 +111,12 @@ struct Tuning {
                                  // (1 with 4-arc lane quads, 0 = row-block kernel)
     uint32_t seg_hot = 32768;    // its shared-memory hot prefix on relabelled graphs (entries)
     uint32_t seg_res64 = 1;      // unweighted graphs: tile-segmented FP64 residual pass (0 = row-block kernel)
-    uint32_t seg_hot64 = 8192;   // its hot prefix (entries)
+    // its hot prefix (entries), 96 KB beside the passes' 64 KB of row sums.  Build
+    // and FP64 solve, ms, at 8 K / 12 K / 16 K entries: R-MAT scale 19 2.38 / 2.34
+    // / 2.27, 21 5.57 / 5.47 / 5.42, 22 11.60 / 11.32 / 11.30, 23 22.9 / 22.4 /
+    // 22.6, refined solve at 24 19.7 / 19.7 / 20.1; 20 K leaves L1 too little
+    // (scale 22 14.3)
+    uint32_t seg_hot64 = 12288;
     uint32_t seg_plain64 = 1;    // unweighted graphs: tile-segmented FP64 power step and Krylov matvec
                                  // (0 = row-block kernels)
     uint32_t seg_eig64 = 1;      // unweighted graphs: tile-segmented eigenvector / HITS product
