@@ -785,12 +785,11 @@ void solve_krylov(const DeviceGraph &g, Workspace &ws, const SolveOpts &o, const
     if (linsys) {
         // pagerank_linsys returns the iterate itself
         PRG_CUDA(cudaMemcpyAsync(d_out, ws.x64[0], (uint64_t)n * 8, cudaMemcpyDeviceToDevice, s));
+    } else if (o.normalise) {
+        launch_normalise(d_out, ws.x64[1], n, ws.ctl, s);
+        st.kernel_launches += 1u;
     } else {
         PRG_CUDA(cudaMemcpyAsync(d_out, ws.x64[1], (uint64_t)n * 8, cudaMemcpyDeviceToDevice, s));
-        if (o.normalise) {
-            launch_normalise(d_out, n, ws.ctl, s);
-            st.kernel_launches += 1u;
-        }
     }
     st.last_diff = ws.h_ctl->diff;
     st.error_bound = st.residual_l1 * o.damping / (1.0 - o.damping);

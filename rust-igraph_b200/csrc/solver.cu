@@ -464,8 +464,7 @@ static void solve_refined(const DeviceGraph &g, Workspace &ws, const SolveOpts &
     }
     if (o.normalise) {
         // result = g / sum(g) (FP64), sum taken by the last residual pass
-        PRG_CUDA(cudaMemcpyAsync(d_out, ws.x64[1], (uint64_t)g.n * 8, cudaMemcpyDeviceToDevice, s));
-        launch_normalise(d_out, g.n, ws.ctl, s);
+        launch_normalise(d_out, ws.x64[1], g.n, ws.ctl, s);
         st.kernel_launches += 1u;
     } else {
         PRG_CUDA(cudaMemcpyAsync(d_out, ws.x64[1], (uint64_t)g.n * 8, cudaMemcpyDeviceToDevice, s));

@@ -167,7 +167,7 @@ float gather_probe(const DeviceGraph &g, int reps, cudaStream_t s);
 void launch_prepare64(const DeviceGraph &g, double *x, const float *e, double *xt, Ctl *ctl, int parity,
                       double4 *part, cudaStream_t s);
 // x <- x / sum (final FP64 normalisation of the refined result).
-void launch_normalise(double *x, uint32_t n, const Ctl *ctl, cudaStream_t s);
+void launch_normalise(double *out, const double *x, uint32_t n, const Ctl *ctl, cudaStream_t s);
 // x <- t (FP64 copy) or uniform 1/n when t is null.
 void launch_fill_start(double *x, const double *t, uint32_t n, cudaStream_t s);
 // Loads the start, prepare and id-gather kernels now (CUDA loads kernels
