@@ -22,8 +22,9 @@
 // A row that began in an earlier tile is finished by a second, small kernel:
 // tile t leaves the sum before its first row end (head) and the open sum
 // after its last (tail); the row's total is the tails of the tiles it spans
-// plus the head, added in tile order in FP64.  The same kernel applies the
-// epilogue to the rows without arcs.  With degree-sorted ids the first 48 K
+// plus the head, added in tile order in FP64.  The rows without arcs take
+// their epilogue in the same kernel, or between the tiles of the first
+// (spreads_arcless).  With degree-sorted ids the first 48 K
 // entries of the gathered vector (about 45 % of the arcs' sources on R-MAT)
 // sit in shared memory of the one 1024-thread block per SM.
 //
@@ -773,6 +774,13 @@ struct Plain64Pass {
 // beside the index (w64 or w32, 64 or 32 bytes per lane).  FP64 power step with
 // its finishing kernel against the row-block kernel: power law of 2 M vertices
 // and 17 M arcs 113 against 177 us, R-MAT scale 20 84 against 201 us.
+constexpr int kArcless = 2;  // rows without arcs a lane loads ahead (four spill)
+
+// Whether the tile kernel takes the rows without arcs of a dense numbering.  The
+// pipelined FP32 kernel does not: holding the next tile, it spills with them
+// (scale 24, tile and finishing kernel: 473 + 15 us against 448 + 26).
+static bool spreads_arcless(const LaunchCfg &c) { return c.seg == 2 && !c.seg_pipe; }
+
 template <class P, bool HOT, int NT, bool PIPE, bool W>
 __global__ void __launch_bounds__(NT, 1) seg8_kernel(const IterArgs a) {
     using V = typename P::V;
@@ -842,6 +850,28 @@ __global__ void __launch_bounds__(NT, 1) seg8_kernel(const IterArgs a) {
 #pragma unroll
             for (int k = 0; k < 8; k++)
                 if (q + k >= a.arcs) v[k] = V(0);
+        }
+    };
+    // The rows without arcs, when they are the range n - nempty .. n-1 (all
+    // passes but the pipelined one, see spreads_arcless): each warp takes a run
+    // of them, the warps of a block in different rounds of their tiles, so that
+    // these streamed rows, which ask for memory bandwidth, run beside the
+    // gathers, which ask for L1TEX.  In the finishing kernel they had the chip
+    // to themselves: FP64 power step of R-MAT scale 22, tile and finishing
+    // kernel, 209 + 25 us then, 209 + 14 now; residual pass of scale 24 959 + 62
+    // against 916 + 28.
+    auto arcless = [&]() {
+        const uint32_t per = (uint32_t)((a.seg_nempty + nwarps - 1) / nwarps + 31u) & ~31u;
+        const uint64_t lo = warp * per, hi = min(lo + per, (uint64_t)a.seg_nempty);
+        const uint64_t e0 = a.n - a.seg_nempty;
+        for (uint64_t i = lo + lane; i < hi; i += 32 * kArcless) {
+            typename P::Pre q[kArcless];
+#pragma unroll
+            for (int k = 0; k < kArcless; k++)
+                if (i + 32 * k < hi) q[k] = pass.load(a, (uint32_t)(e0 + i + 32 * k));
+#pragma unroll
+            for (int k = 0; k < kArcless; k++)
+                if (i + 32 * k < hi) pass.fin(a, (uint32_t)(e0 + i + 32 * k), q[k], V(0));
         }
     };
     // with PIPE the next tile's indices, mask word and record are loaded while
@@ -916,23 +946,37 @@ __global__ void __launch_bounds__(NT, 1) seg8_kernel(const IterArgs a) {
         }
         __syncwarp();
     };
-    if (PIPE) {
-        // two tiles per trip with the buffers' roles swapped, so nothing is
-        // copied between them
-        uint32_t ca[8], cb[8], ma = 0u, mb = 0u;
-        uint4 ea, eb;
-        load_tile(warp, ca, ma, ea);
-        for (uint64_t t = warp; t < a.seg_ntiles; t += 2 * nwarps) {
-            work(t, ca, ma, ea, cb, mb, eb);
-            if (t + nwarps >= a.seg_ntiles) break;
-            work(t + nwarps, cb, mb, eb, ca, ma, ea);
+    auto tiles = [&](uint64_t t, uint64_t end) {
+        if (PIPE) {
+            // two tiles per trip with the buffers' roles swapped, so nothing is
+            // copied between them
+            uint32_t ca[8], cb[8], ma = 0u, mb = 0u;
+            uint4 ea, eb;
+            load_tile(t, ca, ma, ea);
+            for (; t < end; t += 2 * nwarps) {
+                work(t, ca, ma, ea, cb, mb, eb);
+                if (t + nwarps >= end) break;
+                work(t + nwarps, cb, mb, eb, ca, ma, ea);
+            }
+        } else {
+            uint32_t cc[8], mw = 0u, cn[8], mn = 0u;
+            uint4 meta, en;
+            for (; t < end; t += nwarps) {
+                load_tile(t, cc, mw, meta);
+                work(t, cc, mw, meta, cn, mn, en);
+            }
         }
+    };
+    if (PIPE) {
+        tiles(warp, a.seg_ntiles);
     } else {
-        uint32_t cc[8], mw = 0u, cn[8], mn = 0u;
-        uint4 meta, en;
-        for (uint64_t t = warp; t < a.seg_ntiles; t += nwarps) {
-            load_tile(t, cc, mw, meta);
-            work(t, cc, mw, meta, cn, mn, en);
+        // one copy of the tile loop: twice round, the rows without arcs between
+        const uint64_t mid =
+            a.seg_dense ? warp + (threadIdx.x >> 5) * (a.seg_ntiles / nwarps) / (NT / 32) * nwarps : warp;
+#pragma unroll 1
+        for (int half = 0; half < 2; half++) {
+            tiles(half ? mid : warp, half ? a.seg_ntiles : mid);
+            if (half == 0 && a.seg_dense) arcless();
         }
     }
     pass.end(a, 0u, s_red, false);
@@ -944,7 +988,7 @@ __global__ void __launch_bounds__(NT, 1) seg8_kernel(const IterArgs a) {
 // order in FP64: one thread per row for spans of up to kSegLongSpan tiles,
 // one warp (lanes strided over the tiles, then a fixed tree) for longer ones.
 template <class P>
-__global__ void __launch_bounds__(kSegFixNT) seg_finish(const IterArgs a, unsigned rec0) {
+__global__ void __launch_bounds__(kSegFixNT) seg_finish(const IterArgs a, unsigned rec0, bool arcless) {
     using V = typename P::V;
     __shared__ double s_red[96];
     if (P::stopped(a)) return;
@@ -972,6 +1016,10 @@ __global__ void __launch_bounds__(kSegFixNT) seg_finish(const IterArgs a, unsign
     // aligned), their operand loads issued together; with dense ids they are
     // the range n - nempty .. n-1
     if (a.seg_dense) {
+        if (!arcless) {  // the tile kernel has taken them
+            pass.end(a, rec0, s_red, true);
+            return;
+        }
         // four rows per thread and step, nth apart, so that every load and
         // store of a warp covers consecutive rows
         const uint64_t e0 = a.n - a.seg_nempty;
@@ -1070,21 +1118,21 @@ LaunchCfg seg_config(const DeviceGraph &g, uint32_t hot_entries, int variant, in
 void launch_seg(int mode, const IterArgs &a, const LaunchCfg &c, cudaStream_t s) {
     if (mode == MODE_KRES64) {
         seg8_pick<Res64Pass>(c.hot != 0, c.threads, c.seg_pipe, c.seg_w, nullptr)(a, c, s);
-        seg_finish<Res64Pass><<<c.seg_g2, kSegFixNT, 0, s>>>(a, c.seg_g1);
+        seg_finish<Res64Pass><<<c.seg_g2, kSegFixNT, 0, s>>>(a, c.seg_g1, !spreads_arcless(c));
     } else if (mode == MODE_EIG64) {
         seg8_pick<Eig64Pass>(c.hot != 0, c.threads, c.seg_pipe, c.seg_w, nullptr)(a, c, s);
-        seg_finish<Eig64Pass><<<c.seg_g2, kSegFixNT, 0, s>>>(a, c.seg_g1);
+        seg_finish<Eig64Pass><<<c.seg_g2, kSegFixNT, 0, s>>>(a, c.seg_g1, !spreads_arcless(c));
     } else if (mode == MODE_KRY64) {
         seg8_pick<Kry64Pass>(c.hot != 0, c.threads, c.seg_pipe, c.seg_w, nullptr)(a, c, s);
-        seg_finish<Kry64Pass><<<c.seg_g2, kSegFixNT, 0, s>>>(a, c.seg_g1);
+        seg_finish<Kry64Pass><<<c.seg_g2, kSegFixNT, 0, s>>>(a, c.seg_g1, !spreads_arcless(c));
     } else if (mode == MODE_PLAIN64 || mode == MODE_PPR64) {
         seg8_pick<Plain64Pass>(c.hot != 0, c.threads, c.seg_pipe, c.seg_w, nullptr)(a, c, s);
-        seg_finish<Plain64Pass><<<c.seg_g2, kSegFixNT, 0, s>>>(a, c.seg_g1);
+        seg_finish<Plain64Pass><<<c.seg_g2, kSegFixNT, 0, s>>>(a, c.seg_g1, !spreads_arcless(c));
     } else {
         if (c.seg == 2) seg8_pick<Kry32Pass>(c.hot != 0, c.threads, c.seg_pipe, c.seg_w, nullptr)(a, c, s);
         else if (c.hot) kry32_seg_kernel<true><<<c.seg_g1, kSegNT, c.smem, s>>>(a);
         else kry32_seg_kernel<false><<<c.seg_g1, kSegNT, c.smem, s>>>(a);
-        seg_finish<Kry32Pass><<<c.seg_g2, kSegFixNT, 0, s>>>(a, c.seg_g1);
+        seg_finish<Kry32Pass><<<c.seg_g2, kSegFixNT, 0, s>>>(a, c.seg_g1, !spreads_arcless(c));
     }
     PRG_CUDA(cudaGetLastError());
 }
