@@ -322,16 +322,17 @@ int32_t prg_autotune(prg_graph *g, int32_t tune_batch, const char *cache_path, p
  * keeps the most-gathered prefix; defaults 16384 / 2048, 0 = all allocate),
  * "defaults" (any value: every key back to its default),
  * "krylov_floor_pct" (Krylov inner solves aim at this percentage of the
- * certified final threshold, 1-90; default 70), "seg_kry32" (unweighted
- * graphs: the tile-segmented FP32 Krylov matvec, 1 with 4-arc lane quads, 2
- * with 8 consecutive arcs per lane; 0 the row-block kernel),
+ * certified final threshold, 1-90; default 70), "seg_kry32" (the
+ * tile-segmented FP32 Krylov matvec, 1 with 4-arc lane quads, on unweighted
+ * graphs, 2 with 8 consecutive arcs per lane; 0 the row-block kernel),
  * "seg_hot" (its shared-memory hot prefix on relabelled graphs, entries),
- * "seg_res64" (unweighted graphs: 1 the tile-segmented FP64 residual pass
+ * "seg_res64" (1 the tile-segmented FP64 residual pass
  * of the refined and Krylov solves, 0 the row-block kernel), "seg_hot64"
- * (its hot prefix, at most 20480 entries; the FP64 power step shares it),
- * "seg_eig64" (unweighted graphs: 1 the tile-segmented adjacency product of
+ * (its hot prefix, at most 20480 entries, default 12288; the other FP64 passes
+ * share it),
+ * "seg_eig64" (1 the tile-segmented adjacency product of
  * the eigenvector and HITS iterations, the default; 0 the row-block kernel),
- * "seg_plain64" (unweighted graphs: 1 the tile-segmented FP64 power step of
+ * "seg_plain64" (1 the tile-segmented FP64 power step of
  * the drop-ins and the certified FP64 loop, and the FP64 Krylov matvec of
  * the FP64 Krylov and pagerank_linsys solves; 0 the row-block kernel),
  * "resident" (graphs whose arcs fit the SMs' shared memory, unless

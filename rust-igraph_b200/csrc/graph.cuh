@@ -44,7 +44,7 @@ struct DeviceGraph {
     // block size of those passes (256: several blocks per SM; 512 or 1024:
     // one block per SM with a larger prefix)
     uint32_t hot_cache = 0, hot_cache64 = 8192, hot_threads = 1024;
-    // unweighted graphs: the FP32 Krylov matvec as the tile-segmented pass
+    // the FP32 Krylov matvec as the tile-segmented pass
     // (segspmv.cu), with a hot prefix of seg_hot entries on relabelled graphs
     uint32_t seg_kry32 = 2, seg_hot = 32768;
     // ... and the FP64 residual pass of the refined / Krylov solves, with a
@@ -107,19 +107,19 @@ struct Tuning {
     // FP64 passes on relabelled graphs: a 8 K-entry shared-memory hot prefix in
     // one 1024-thread block per SM (measured 7 % faster at R-MAT s24)
     uint32_t hot_cache = 0, hot_cache64 = 8192, hot_threads = 1024;
-    uint32_t seg_kry32 = 2;      // unweighted graphs: tile-segmented FP32 Krylov matvec, 2 with 8 arcs per lane
-                                 // (1 with 4-arc lane quads, 0 = row-block kernel)
+    uint32_t seg_kry32 = 2;      // tile-segmented FP32 Krylov matvec, 2 with 8 arcs per lane (1 with 4-arc
+                                 // lane quads, unweighted graphs; 0 = row-block kernel)
     uint32_t seg_hot = 32768;    // its shared-memory hot prefix on relabelled graphs (entries)
-    uint32_t seg_res64 = 1;      // unweighted graphs: tile-segmented FP64 residual pass (0 = row-block kernel)
+    uint32_t seg_res64 = 1;      // tile-segmented FP64 residual pass (0 = row-block kernel)
     // its hot prefix (entries), 96 KB beside the passes' 64 KB of row sums.  Build
     // and FP64 solve, ms, at 8 K / 12 K / 16 K entries: R-MAT scale 19 2.38 / 2.34
     // / 2.27, 21 5.57 / 5.47 / 5.42, 22 11.60 / 11.32 / 11.30, 23 22.9 / 22.4 /
     // 22.6, refined solve at 24 19.7 / 19.7 / 20.1; 20 K leaves L1 too little
     // (scale 22 14.3)
     uint32_t seg_hot64 = 12288;
-    uint32_t seg_plain64 = 1;    // unweighted graphs: tile-segmented FP64 power step and Krylov matvec
+    uint32_t seg_plain64 = 1;    // tile-segmented FP64 power step and Krylov matvec
                                  // (0 = row-block kernels)
-    uint32_t seg_eig64 = 1;      // unweighted graphs: tile-segmented eigenvector / HITS product
+    uint32_t seg_eig64 = 1;      // tile-segmented eigenvector / HITS product
     uint32_t resident = 1;       // small graphs: block-resident persistent iterations (resident.cu)
     uint32_t seg_prefetch = 1;   // segmented passes: L2 prefetch of each warp's next index tile
     uint32_t seg_threads = 1024;  // segmented passes: tile-kernel block size (1024, 768 or 512)

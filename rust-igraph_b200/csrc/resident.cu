@@ -55,8 +55,8 @@ constexpr uint32_t kResOpen = 0xFFFFFFFFu;   // no row end
 // kernels, with a hot prefix in shared memory, are as fast or faster there
 // (16 M arcs: 77 us an iteration on R-MAT).  us per iteration, resident /
 // launched: 0.1 M arcs 4.7 / 18, 1 M 8.1 / 21, 4 M 23 / 38, 8 M 38 / 56 on
-// uniform random graphs (weighted 4.7 / 13, 8.3 / 20, 26 / 48, 49 / 79);
-// R-MAT 4 M 15 / 28, 8 M 27 / 37 (weighted 17 / 136, 38 / 151).
+// uniform random graphs (weighted 1 M 8.3 / 24, 4 M 26 / 43, 8 M 49 / 63);
+// R-MAT 4 M 15 / 28, 8 M 27 / 37 (weighted 8 M 38 / 43).
 // Hence kResMaxArcs.
 constexpr int kResTiles = 32;                // tiles of 8192 arcs a block can take
 // Shared memory of a block (dynamic): L1 needs the rest for the gathers in

@@ -1,5 +1,5 @@
 // segspmv.cu — the FP32 Krylov matvec y = A p (MODE_KRY32) as a
-// tile-segmented pass over the in-CSR, for unweighted graphs.
+// tile-segmented pass over the in-CSR, and the FP64 passes on the same tiling.
 //
 // The row-block kernel (spmv.cu) walks rows: each warp stages a row-block's
 // products and sums them per row, so every step waits on an index load and
@@ -453,14 +453,16 @@ __device__ __forceinline__ const double *arc_weights(const IterArgs &a, double) 
 __device__ __forceinline__ const float *arc_weights(const IterArgs &a, float) { return a.w32; }
 
 // ------------------------------------------------------------------ pass kinds
-// The 8-arcs-per-lane tile kernel and the finishing kernel are shared by two
+// The 8-arcs-per-lane tile kernel and the finishing kernel are shared by five
 // passes, which differ in value type, gathered vector, prologue, epilogue and
 // records:
 //   Kry32Pass — the FP32 Krylov matvec above (MODE_KRY32);
 //   Res64Pass — the FP64 residual pass r = G(x) - x of the refined and
 //               Krylov solves (MODE_KRES64), with iter_kernel<MODE_KRES64>'s
 //               epilogue and its Ctl bookkeeping done by the last finishing
-//               block.
+//               block;
+//   Kry64Pass, Plain64Pass, Eig64Pass — the FP64 Krylov matvec, the FP64 power
+//               step and the adjacency product (below).
 
 struct Kry32Pass {
     using V = float;

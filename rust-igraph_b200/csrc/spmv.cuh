@@ -149,7 +149,7 @@ LaunchCfg iteration_config(int mode, bool weighted, uint32_t hot_entries, uint32
 void launch_iteration(int mode, bool weighted, const IterArgs &a, const LaunchCfg &c, cudaStream_t s);
 
 // Tile-segmented FP32 Krylov matvec (segspmv.cu): builds the row-end index of
-// g (unweighted graphs), frees it, gives its launch shape (hot prefix of up
+// g, frees it, gives its launch shape (hot prefix of up
 // to hot_entries vertices in shared memory) and launches it (two kernels:
 // the tiles, then the rows that span tiles and the rows without arcs).
 void seg_build(const DeviceGraph &g, SegIndex &x, cudaStream_t s);
