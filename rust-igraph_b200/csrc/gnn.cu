@@ -190,28 +190,58 @@ __device__ __forceinline__ void ld_msg(const float *p, float (&q)[kC]) {
         : "l"(p));
 }
 
-// acc += the messages of arcs p, p + STRIDE, ... below p1, added one by one in
-// that order, with kAggAhead of them in flight
+// The sources of arcs p, p + STRIDE, ... below p1, kAggAhead of them.
 constexpr int kAggAhead = 4;
 template <uint32_t STRIDE>
+__device__ __forceinline__ void ld_sources(const uint32_t *col, uint32_t p, uint32_t p1, uint32_t (&u)[kAggAhead]) {
+#pragma unroll
+    for (int i = 0; i < kAggAhead; i++) u[i] = p + i * STRIDE < p1 ? __ldg(&col[p + i * STRIDE]) : 0u;
+}
+
+// acc += the messages of arcs p, p + STRIDE, ... below p1, added one by one in
+// that order, with kAggAhead of them in flight.  u: the first sources, loaded
+// before; while the last messages are in flight it takes those of the arcs from
+// q on, below q1 (the next row's).
+template <uint32_t STRIDE>
 __device__ __forceinline__ void add_messages(float (&acc)[kC], uint32_t p, uint32_t p1, const uint32_t *col,
-                                             const float *M) {
-    for (; p < p1; p += STRIDE * kAggAhead) {
-        uint32_t u[kAggAhead];
-        float q[kAggAhead][kC];
+                                             const float *M, uint32_t (&u)[kAggAhead], uint32_t q, uint32_t q1) {
+    bool more;
+    do {
+        float m[kAggAhead][kC];
 #pragma unroll
         for (int i = 0; i < kAggAhead; i++)
-            if (p + i * STRIDE < p1) u[i] = __ldg(&col[p + i * STRIDE]);
+            if (p + i * STRIDE < p1) ld_msg(M + (size_t)u[i] * kC, m[i]);
+        const uint32_t at = p;
+        p += STRIDE * kAggAhead;
+        more = p < p1;
+        ld_sources<STRIDE>(col, more ? p : q, more ? p1 : q1, u);
 #pragma unroll
         for (int i = 0; i < kAggAhead; i++)
-            if (p + i * STRIDE < p1) ld_msg(M + (size_t)u[i] * kC, q[i]);
+            if (at + i * STRIDE < p1) {
 #pragma unroll
-        for (int i = 0; i < kAggAhead; i++)
-            if (p + i * STRIDE < p1) {
-#pragma unroll
-                for (int c = 0; c < kC; c++) acc[c] += q[i][c];
+                for (int c = 0; c < kC; c++) acc[c] += m[i][c];
             }
+    } while (more);
+}
+
+// The sums of acc over a row's 8 lanes; lane `sub` gets channel `sub`.  At each
+// step a lane keeps half of its channels and gives the others away: 7 shuffles
+// instead of 3 per channel, each sum added in the same order.
+__device__ __forceinline__ float row_channel(const float (&acc)[kC], uint32_t sub) {
+    float a[4], b[2];
+    const bool up4 = (sub & 4u) != 0u, up2 = (sub & 2u) != 0u, up1 = (sub & 1u) != 0u;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const float got = __shfl_xor_sync(0xffffffffu, up4 ? acc[c] : acc[c + 4], 4);
+        a[c] = (up4 ? acc[c + 4] : acc[c]) + got;
     }
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+        const float got = __shfl_xor_sync(0xffffffffu, up2 ? a[c] : a[c + 2], 2);
+        b[c] = (up2 ? a[c + 2] : a[c]) + got;
+    }
+    const float got = __shfl_xor_sync(0xffffffffu, up1 ? b[0] : b[1], 1);
+    return (up1 ? b[1] : b[0]) + got;
 }
 
 // Rows of more than kAggHeavy arcs, listed once per forward pass.
@@ -239,7 +269,9 @@ __global__ void __launch_bounds__(256, 4) aggregate_kernel(uint32_t n, const uin
             float acc[kC];
 #pragma unroll
             for (int c = 0; c < kC; c++) acc[c] = 0.0f;
-            add_messages<256>(acc, p0 + threadIdx.x, p1, col, M);
+            uint32_t u[kAggAhead];
+            ld_sources<256>(col, p0 + threadIdx.x, p1, u);
+            add_messages<256>(acc, p0 + threadIdx.x, p1, col, M, u, 0u, 0u);
             const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
 #pragma unroll
             for (int c = 0; c < kC; c++) acc[c] = warp_sum(acc[c]);
@@ -260,27 +292,43 @@ __global__ void __launch_bounds__(256, 4) aggregate_kernel(uint32_t n, const uin
     const uint32_t gid = (blockIdx.x - kAggHeavyBlocks) * blockDim.x + threadIdx.x, sub = threadIdx.x & 7;
     const uint32_t group = gid >> 3, ngroups = ((gridDim.x - kAggHeavyBlocks) * blockDim.x) >> 3;
     const uint32_t rounds = (n + ngroups - 1) / ngroups;
+    // A row's arcs as an empty range when another block sums it (or there is no
+    // such row).  Row ends are read two rows ahead and a row's first sources one
+    // ahead, so a row waits for its messages alone, not for the chain of row
+    // end, source and message (0.5 M vertices, 3 M arcs 53 us a layer with the
+    // chain, 45 without; R-MAT s22, where L1's data pipe is the bound, 488 and
+    // 485: a lookup per message, the messages' bytes and the shuffles share it,
+    // 82 % busy with three shuffles per channel, 525 us).
+    auto row = [&](uint64_t v, uint32_t &p0, uint32_t &p1) {
+        p0 = p1 = 0u;
+        if (v < n) {
+            p0 = __ldg(&row_ptr[v]);
+            p1 = __ldg(&row_ptr[v + 1]);
+        }
+    };
+    uint32_t p0, p1, n0, n1, u[kAggAhead];
+    row(group, p0, p1);
+    row((uint64_t)group + ngroups, n0, n1);
+    bool heavy_row = p1 - p0 > kAggHeavy;
+    if (heavy_row) p1 = p0;
+    ld_sources<8>(col, p0 + sub, p1, u);
     for (uint32_t rd = 0; rd < rounds; rd++) {
         const uint32_t v = rd * ngroups + group;
         float acc[kC];
 #pragma unroll
         for (int c = 0; c < kC; c++) acc[c] = 0.0f;
-        bool skip = v >= n;
-        if (!skip) {
-            const uint32_t p0 = __ldg(&row_ptr[v]), p1 = __ldg(&row_ptr[v + 1]);
-            if (p1 - p0 > kAggHeavy) skip = true;
-            else add_messages<8>(acc, p0 + sub, p1, col, M);
-        }
-#pragma unroll
-        for (int c = 0; c < kC; c++) {
-            acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 4);
-            acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 2);
-            acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 1);
-        }
-        // lane `sub` finishes channel `sub`
-        float mine = acc[0];
-#pragma unroll
-        for (int c = 1; c < kC; c++) mine = sub == (uint32_t)c ? acc[c] : mine;
+        uint32_t f0, f1;
+        row(v + 2ull * ngroups, f0, f1);
+        const bool skip = v >= n || heavy_row;
+        const bool next_heavy = n1 - n0 > kAggHeavy;
+        add_messages<8>(acc, p0 + sub, p1, col, M, u, n0 + sub, next_heavy ? 0u : n1);
+        const bool some = p1 > p0;
+        p0 = n0;
+        p1 = next_heavy ? n0 : n1;
+        heavy_row = next_heavy;
+        n0 = f0;
+        n1 = f1;
+        const float mine = __any_sync(0xffffffffu, some) ? row_channel(acc, sub) : 0.0f;
         const float z = slog(mine), zn = __shfl_xor_sync(0xffffffffu, z, 1);
         if (!skip) {
             uint32_t *dst = reinterpret_cast<uint32_t *>(out + (size_t)v * 16);
