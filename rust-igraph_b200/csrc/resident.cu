@@ -59,6 +59,7 @@ constexpr uint32_t kResOpen = 0xFFFFFFFFu;   // no row end
 // R-MAT 4 M 15 / 28, 8 M 27 / 37 (weighted 8 M 38 / 43).
 // Hence kResMaxArcs.
 constexpr int kResTiles = 32;                // tiles of 8192 arcs a block can take
+constexpr uint32_t kResMaxChunks = kResTiles * kResNT;
 // Shared memory of a block (dynamic): L1 needs the rest for the gathers in
 // flight and the hot sources.  R-MAT passes of 8 M arcs took 72-84 us with
 // 190 KB of shared memory and 27 us with 144 KB; a power law's of 4 M arcs 40
@@ -664,6 +665,18 @@ static size_t res_limits(uint64_t arcs, uint32_t n, unsigned &nb) {
     return std::min(kResSmem, (size_t)optin - kResStatic);
 }
 
+// Whether the mean share, streamed, fits a block.
+static bool res_mean_fits(uint32_t n, uint64_t arcs, bool weighted, int kind) {
+    unsigned nb = 0;
+    const size_t most = res_limits(arcs, n, nb);
+    const uint64_t chunks = arcs / 8 / nb;
+    return chunks <= kResMaxChunks && res_bytes(n / nb, (uint32_t)chunks, kind, weighted, true) <= most;
+}
+
+bool res_sizes_fit(uint32_t n, uint64_t arcs, bool weighted, int kind) {
+    return n >= 2 && arcs > 0 && arcs <= kResMaxArcs && res_mean_fits(n, arcs, weighted, kind);
+}
+
 ResPlan res_plan_blind(uint32_t n, uint64_t arcs, bool weighted, int kind) {
     ResPlan p;
     if (n < 2 || arcs == 0 || arcs > kResMaxArcs) return p;
@@ -683,7 +696,6 @@ ResPlan res_plan(const DeviceGraph &g, int kind, cudaStream_t s) {
     if (g.n < 2 || g.arcs == 0 || g.arcs > kResMaxArcs) return p;
     unsigned nb = 0;
     const size_t most = res_limits(g.arcs, g.n, nb);
-    const uint32_t max_chunks = kResTiles * kResNT;
     // small graphs fit whatever their rows look like
     p.alpha = res_alpha(0);
     const uint64_t total = g.arcs + (uint64_t)p.alpha * g.n;
@@ -694,9 +706,7 @@ ResPlan res_plan(const DeviceGraph &g, int kind, cudaStream_t s) {
         return p;
     }
     // otherwise the shares themselves decide, unless even the mean does not fit
-    if (res_bytes(g.n / nb, (uint32_t)(g.arcs / 8 / nb), kind, g.weighted, true) > most ||
-        g.arcs / 8 / nb > max_chunks)
-        return p;
+    if (!res_mean_fits(g.n, g.arcs, g.weighted, kind)) return p;
     uint32_t *d = nullptr, h[3 * kResSplits];
     PRG_CUDA(cudaMallocAsync((void **)&d, sizeof(h), s));
     PRG_CUDA(cudaMemsetAsync(d, 0, sizeof(h), s));
@@ -708,7 +718,7 @@ ResPlan res_plan(const DeviceGraph &g, int kind, cudaStream_t s) {
     for (unsigned k = 0; k < kResSplits; k++) {
         const bool stream = h[3 * k] > most;
         const uint32_t bytes = h[3 * k + (stream ? 1 : 0)];
-        if (bytes > most || h[3 * k + 2] > max_chunks) continue;
+        if (bytes > most || h[3 * k + 2] > kResMaxChunks) continue;
         p.alpha = res_alpha(k);
         p.stream = stream;
         p.grid = nb;

@@ -51,7 +51,9 @@ struct ResArgs {
 // Launch shape for graph g, or grid = 0 where it does not apply (reads the
 // rows' split back from the device when the sizes alone do not decide).
 ResPlan res_plan(const DeviceGraph &g, int kind, cudaStream_t s);
-// The same before the graph is built, for graphs whose indices surely stay in
+// Whether a graph of these sizes can have a plan at all, whatever its rows.
+bool res_sizes_fit(uint32_t n, uint64_t arcs, bool weighted, int kind);
+// The plan before the graph is built, for graphs whose indices surely stay in
 // shared memory as long as no row is long (ResArgs::longest checks that).
 ResPlan res_plan_blind(uint32_t n, uint64_t arcs, bool weighted, int kind);
 // Bytes of scratch the launch needs (records and arrival counter).

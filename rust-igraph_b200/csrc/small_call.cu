@@ -19,7 +19,7 @@
 // and these graphs' vectors fit L2).  Weighted directed graphs run the same
 // phases a second time by source for the out-strengths.
 //
-// Limits: kResMaxArcs.  Where res_plan_blind gives no plan, or the rows turn out
+// Limits: res_sizes_fit.  Where res_plan_blind gives no plan, or the rows turn out
 // too uneven for its shares (Ctl::status), the iteration is planned from the CSR
 // just built, and only if that fails does the caller take the general path.
 #include "small_call.cuh"
@@ -342,7 +342,11 @@ SmallStatus small_call(const SmallCall &c, double *out, SmallResult &r, cudaStre
     const uint64_t arcs = c.directed ? c.m : 2 * c.m;
     const uint32_t n = c.n;
     const bool two = c.w != nullptr && c.directed;
-    if (c.m == 0 || n < 2 || arcs > kResMaxArcs) return SMALL_NOT_HERE;
+    // Before anything is copied: from 2.0-2.4 M vertices on (1.1-1.3 M with
+    // eigenvectors) no share fits a block.  Copying and building first, to be
+    // refused by the plan, made a call on 3 M vertices and 6 M edges 12.7 ms
+    // instead of 8.6.
+    if (!res_sizes_fit(n, arcs, c.w != nullptr, c.kind)) return SMALL_NOT_HERE;
     // without a blind plan the iteration is planned once the rows are known
     const ResPlan p = res_plan_blind(n, arcs, c.w != nullptr, c.kind);
     static int sms = 0;

@@ -1,0 +1,62 @@
+"""Which way a one-call drop-in goes, seen in the kernels it launches and the
+bytes it uploads: a call that the small-graph path cannot serve must cost what
+the general path costs, and give its result to the bit."""
+import json
+
+import numpy as np
+import pytest
+
+import igraph_b200 as ig
+
+pytestmark = pytest.mark.gpu
+
+
+def traced(call, path):
+    """(result, kernel names, bytes copied host to device)"""
+    from torch.profiler import ProfilerActivity, profile
+
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        out = call()
+    p.export_chrome_trace(path)
+    with open(path) as fh:
+        events = json.load(fh)["traceEvents"]
+    names = [e["name"] for e in events if e.get("cat") == "kernel"]
+    up = sum(e["args"]["bytes"] for e in events if e.get("cat") == "gpu_memcpy" and "HtoD" in e["name"])
+    assert names, "the profiler saw no kernels"
+    return out, names, up
+
+
+def both(call, tmp_path):
+    """The call as it goes by default and over the general path alone."""
+    ig.pagerank(ig.Graph.from_edge_arrays(2, np.zeros(1, np.uint32), np.ones(1, np.uint32), True))  # context, kernels
+    got = traced(call, str(tmp_path / "default.json"))
+    try:
+        ig.set_tuning("resident", 0)
+        general = traced(call, str(tmp_path / "general.json"))
+    finally:
+        ig.reset_tuning()
+    return got, general
+
+
+CALLS = {
+    "pagerank": lambda g, w: ig.pagerank(g),
+    "weighted": lambda g, w: ig.pagerank_weighted(g, w),
+    "eigenvector": lambda g, w: ig.eigenvector_centrality(g),
+    "eigenvector_weighted": lambda g, w: ig.eigenvector_centrality_weighted(g, w),
+}
+
+
+@pytest.mark.parametrize("kind,n,m", [("pagerank", 3_000_000, 1_000_000), ("pagerank", 2_450_000, 6_000_000),
+                                      ("weighted", 3_000_000, 1_000_000), ("eigenvector", 1_400_000, 300_000),
+                                      ("eigenvector_weighted", 1_400_000, 300_000)])
+def test_many_vertices_are_refused_before_any_copy(cuda_ok, kind, n, m, tmp_path):
+    rng = np.random.default_rng(n)
+    f, t = rng.integers(0, n, m).astype(np.uint32), rng.integers(0, n, m).astype(np.uint32)
+    directed = not kind.startswith("eigen")
+    if not directed:
+        f, t = np.minimum(f, t), np.maximum(f, t)
+    g, w = ig.Graph.from_edge_arrays(n, f, t, directed), rng.random(m) + 0.5
+    (x, names, up), (ref, _, ref_up) = both(lambda: CALLS[kind](g, w), tmp_path)
+    assert not any("small_build_kernel" in k or "res_kernel" in k for k in names)
+    assert up == ref_up
+    assert np.array_equal(x, ref)
