@@ -60,6 +60,19 @@ constexpr uint32_t kResOpen = 0xFFFFFFFFu;   // no row end
 // Hence kResMaxArcs.
 constexpr int kResTiles = 32;                // tiles of 8192 arcs a block can take
 constexpr uint32_t kResMaxChunks = kResTiles * kResNT;
+// The block with the most arcs sets an iteration's time, 3.3-4.5 us per tile
+// where it gathers from L2, and the launched kernels spread a row over the chip;
+// so a plan that gives one block, by a long row or by the coarse splits below,
+// this many arcs more than the equal share is refused.  us per iteration,
+// resident / launched, one row of 32 K, 48 K, 64 K, 96 K, 128 K arcs among 0.5 M:
+// 20 / 22, 22 / 23, 30 / 23, 44 / 23, 54 / 21, among 5 M: 25 / 44, 46 / 45,
+// 56 / 44, 58 / 45, 81 / 45; R-MAT scale 19 with 47 K above the share 36 / 42,
+// with 50 K 48 / 43, scale 20 with 87 K 60 / 50 (weighted 92 / 56).  The lines
+// cross near 48 K.  Between there and 68 K a solve on a resident graph loses
+// 0.1-0.2 ms, but a drop-in wins more from the build (1.3-1.5 against 0.4-0.6 ms
+// for 40-400 K arcs), and both must iterate in the same kernel to give the same
+// bits.
+constexpr uint64_t kResExcess = 68 << 10;
 // Shared memory of a block (dynamic): L1 needs the rest for the gathers in
 // flight and the hot sources.  R-MAT passes of 8 M arcs took 72-84 us with
 // 190 KB of shared memory and 27 us with 144 KB; a power law's of 4 M arcs 40
@@ -696,7 +709,7 @@ ResPlan res_plan(const DeviceGraph &g, int kind, cudaStream_t s) {
     if (g.n < 2 || g.arcs == 0 || g.arcs > kResMaxArcs) return p;
     unsigned nb = 0;
     const size_t most = res_limits(g.arcs, g.n, nb);
-    // small graphs fit whatever their rows look like
+    // small graphs fit whatever their rows look like (36 K arcs in a block at most)
     p.alpha = res_alpha(0);
     const uint64_t total = g.arcs + (uint64_t)p.alpha * g.n;
     const double bound = res_bound(total, nb, p.alpha, g.max_in_degree, g.weighted, kind);
@@ -715,10 +728,11 @@ ResPlan res_plan(const DeviceGraph &g, int kind, cudaStream_t s) {
     PRG_CUDA(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, s));
     PRG_CUDA(cudaFreeAsync(d, s));
     PRG_CUDA(cudaStreamSynchronize(s));
+    const uint64_t most_chunks = std::min<uint64_t>(kResMaxChunks, (g.arcs / nb + kResExcess) / 8 + 1);
     for (unsigned k = 0; k < kResSplits; k++) {
         const bool stream = h[3 * k] > most;
         const uint32_t bytes = h[3 * k + (stream ? 1 : 0)];
-        if (bytes > most || h[3 * k + 2] > kResMaxChunks) continue;
+        if (bytes > most || h[3 * k + 2] > most_chunks) continue;
         p.alpha = res_alpha(k);
         p.stream = stream;
         p.grid = nb;

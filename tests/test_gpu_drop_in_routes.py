@@ -1,12 +1,14 @@
-"""Which way a one-call drop-in goes, seen in the kernels it launches and the
-bytes it uploads: a call that the small-graph path cannot serve must cost what
-the general path costs, and give its result to the bit."""
+"""Which way a drop-in or a solve goes, seen in the kernels it launches and the
+bytes it uploads: a drop-in that the small-graph path cannot serve must cost
+what the general path costs, and give its result to the bit; a graph whose
+longest row would hold up one block does not iterate in the persistent kernel."""
 import json
 
 import numpy as np
 import pytest
 
 import igraph_b200 as ig
+import oracle as O
 
 pytestmark = pytest.mark.gpu
 
@@ -60,3 +62,30 @@ def test_many_vertices_are_refused_before_any_copy(cuda_ok, kind, n, m, tmp_path
     assert not any("small_build_kernel" in k or "res_kernel" in k for k in names)
     assert up == ref_up
     assert np.array_equal(x, ref)
+
+
+def hub_graph(n, m, longest):
+    """Directed: one in-row of `longest` arcs, the others short."""
+    rng = np.random.default_rng(longest)
+    t = np.concatenate([np.full(longest, n // 3), rng.integers(0, n, m - longest)]).astype(np.uint32)
+    rng.shuffle(t)
+    return rng.integers(0, n, m).astype(np.uint32), t
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("longest,resident", [(30_000, True), (60_000, True), (90_000, False), (200_000, False)])
+def test_long_rows_do_not_hold_up_one_block(cuda_ok, longest, resident, weighted, tmp_path):
+    n, m = 60_000, 600_000  # 4 K arcs to a block
+    f, t = hub_graph(n, m, longest)
+    w = np.random.default_rng(1).random(m) + 0.5 if weighted else None
+    with ig.DeviceGraph.from_host(n, f, t, True, w) as dg:
+        dg.solve()
+        (x, _), names, _ = traced(dg.solve, str(tmp_path / "solve.json"))
+    assert any("res_kernel" in k for k in names) == resident and any("seg8_kernel" in k for k in names) != resident
+    ref = O.pagerank_weighted(n, f, t, True, w) if weighted else O.pagerank(n, f, t, True)
+    assert np.abs(x - ref).max() <= 1e-10  # the stop rule's tolerance
+    lo, hi = np.minimum(f, t), np.maximum(f, t)
+    g = ig.Graph.from_edge_arrays(n, lo, hi, False)
+    call = "eigenvector_weighted" if weighted else "eigenvector"
+    _, names, _ = traced(lambda: CALLS[call](g, w), str(tmp_path / "eigen.json"))
+    assert any("seg8_kernel" in k for k in names) != resident
