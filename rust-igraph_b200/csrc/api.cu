@@ -179,16 +179,35 @@ static int32_t create_reverse(uint32_t n, uint64_t m, const uint32_t *d_from, co
     return rc;
 }
 
+// An edge list the small-graph path uploaded and left for the general one.
+struct Uploaded {
+    prg::SmallEdges e;
+    Uploaded() = default;
+    Uploaded(const Uploaded &) = delete;
+    ~Uploaded() {
+        if (e.block) cudaFree(e.block);
+    }
+};
+
 // With `rev`, also the graph with every edge reversed; the edge list is
 // uploaded once for both (from pageable memory the upload is most of the
-// work: 8.4 M edges 5.7 ms, their reversed graph from the device 0.6 ms).
+// work: 8.4 M edges 5.7 ms, their reversed graph from the device 0.6 ms).  With
+// `up` holding the same list on the device, nothing is uploaded.
 int32_t create_from_host(uint32_t n, uint64_t m, const uint32_t *from, const uint32_t *to, const double *w,
-                         int32_t directed, prg_graph **out, int relabel = -1, prg_graph **rev = nullptr) {
+                         int32_t directed, prg_graph **out, int relabel = -1, prg_graph **rev = nullptr,
+                         Uploaded *up = nullptr) {
     if (!ensure_pool_config()) return fail(PRG_ERR_CUDA, "cuda: no usable device");
     cudaStream_t s = prg::stream_acquire();
     if (m > 0xFFFFFFFFull) {
         prg::stream_release(s);
         return fail(PRG_ERR_INTERNAL, "ecount overflows u32");
+    }
+    if (up && up->e.block) {
+        const int32_t rc = create_from_device(n, m, up->e.from, up->e.to, up->e.w, directed, s, out, relabel);
+        cudaFreeAsync(up->e.block, s);
+        up->e.block = nullptr;
+        if (rc != PRG_OK) prg::stream_release(s);
+        return rc;
     }
     if (m >= prg::kStreamMinEdges && !(w && (directed || rev))) {
         // large edge lists: chunked copies overlapped with the build
@@ -375,8 +394,9 @@ int32_t check_weights(const double *w, uint64_t m) {
 
 // A drop-in on a small graph in two launches (small_call.cu): true when it
 // ran, with the call's status in *rc and the eigenvalue in *eigenvalue; false
-// sends the call to the general path.
-bool small_dropin(prg::SmallCall &c, double *out, int32_t *rc, double *eigenvalue = nullptr) {
+// sends the call to the general path, with the edge list in *up if it is on the
+// device by then.
+bool small_dropin(prg::SmallCall &c, double *out, int32_t *rc, Uploaded *up, double *eigenvalue = nullptr) {
     const prg::Tuning &t = prg::tuning();
     const bool seg = c.kind == prg::RES_EIG ? t.seg_eig64 != 0 : t.seg_plain64 != 0;
     if (!t.resident || !seg || c.m > 0xFFFFFFFFull || check_sizes(c.n, c.m, c.directed) != PRG_OK) return false;
@@ -390,6 +410,7 @@ bool small_dropin(prg::SmallCall &c, double *out, int32_t *rc, double *eigenvalu
         prg::stream_release(s);
         throw;
     }
+    up->e = r.edges;
     prg::stream_release(s);
     if (st == prg::SMALL_NOT_HERE) return false;
     if (st == prg::SMALL_BAD_WEIGHT) {
@@ -406,6 +427,7 @@ bool small_dropin(prg::SmallCall &c, double *out, int32_t *rc, double *eigenvalu
 // here (and before any device error is reported).
 int32_t dropin(uint32_t n, uint64_t m, const uint32_t *from, const uint32_t *to, int32_t directed, const double *w,
                const double *norm_reset, double damping, double *out, int precision = PRG_PRECISION_FP64) {
+    Uploaded up;
     if (precision == PRG_PRECISION_FP64) {
         prg::SmallCall c;
         const prg::SolveOpts d;  // the reference's eps and max_iter
@@ -422,7 +444,7 @@ int32_t dropin(uint32_t n, uint64_t m, const uint32_t *from, const uint32_t *to,
         c.max_iter = d.max_iter;
         int32_t rc = PRG_OK;
         try {
-            if (small_dropin(c, out, &rc)) return rc;
+            if (small_dropin(c, out, &rc, &up)) return rc;
         } catch (...) {
             if (w && (rc = check_weights(w, m)) != PRG_OK) return rc;
             throw;
@@ -431,7 +453,7 @@ int32_t dropin(uint32_t n, uint64_t m, const uint32_t *from, const uint32_t *to,
     if (w)
         if (int32_t bad = check_weights(w, m)) return bad;
     prg_graph *h = nullptr;
-    int32_t rc = create_from_host(n, m, from, to, w, directed, &h);
+    int32_t rc = create_from_host(n, m, from, to, w, directed, &h, -1, nullptr, &up);
     if (rc != PRG_OK) return rc;
     prg::SolveOpts so;
     so.damping = damping;
@@ -498,7 +520,7 @@ int32_t prg_pagerank(uint32_t n, uint64_t m, const uint32_t *from, const uint32_
 // The undirected eigenvector iterations without negative weights
 // (eigenvector.rs:286-372, 375-538) on a small graph.
 static bool small_eigenvector(uint32_t n, uint64_t m, const uint32_t *from, const uint32_t *to, const double *w,
-                              double eps, double *out, double *eigenvalue, int32_t *rc) {
+                              double eps, double *out, double *eigenvalue, int32_t *rc, Uploaded *up) {
     for (uint64_t e = 0; w && e < m; e++)
         if (!std::isfinite(w[e])) return false;
     prg::SmallCall c;
@@ -513,7 +535,7 @@ static bool small_eigenvector(uint32_t n, uint64_t m, const uint32_t *from, cons
     c.shift = 1.0;
     c.max_iter = 5000;
     c.strength_seed = w != nullptr;
-    return small_dropin(c, out, rc, eigenvalue);
+    return small_dropin(c, out, rc, up, eigenvalue);
 }
 
 int32_t prg_eigenvector_centrality(uint32_t n, uint64_t m, const uint32_t *from, const uint32_t *to, int32_t directed,
@@ -530,9 +552,10 @@ int32_t prg_eigenvector_centrality(uint32_t n, uint64_t m, const uint32_t *from,
         return PRG_OK;
     }
     int32_t rc = PRG_OK;
-    if (small_eigenvector(n, m, from, to, nullptr, 1e-14, out, eigenvalue, &rc)) return rc;
+    Uploaded up;
+    if (small_eigenvector(n, m, from, to, nullptr, 1e-14, out, eigenvalue, &rc, &up)) return rc;
     prg_graph *h = nullptr;
-    rc = create_from_host(n, m, from, to, nullptr, 0, &h);
+    rc = create_from_host(n, m, from, to, nullptr, 0, &h, -1, nullptr, &up);
     if (rc != PRG_OK) return rc;
     try {
         cudaStream_t s = h->stream;
@@ -632,9 +655,10 @@ int32_t prg_eigenvector_centrality_weighted(uint32_t n, uint64_t m, const uint32
     o.eps = 1e-12;
     o.negative = any_negative(weights, m);
     int32_t rc = PRG_OK;
-    if (!o.negative && small_eigenvector(n, m, from, to, weights, o.eps, out, eigenvalue, &rc)) return rc;
+    Uploaded up;
+    if (!o.negative && small_eigenvector(n, m, from, to, weights, o.eps, out, eigenvalue, &rc, &up)) return rc;
     prg_graph *h = nullptr;
-    rc = create_from_host(n, m, from, to, weights, 0, &h);
+    rc = create_from_host(n, m, from, to, weights, 0, &h, -1, nullptr, &up);
     if (rc != PRG_OK) return rc;
     try {
         cudaStream_t s = h->stream;
@@ -732,14 +756,15 @@ int32_t prg_hub_and_authority_scores_weighted(uint32_t n, uint64_t m, const uint
         o.negative = neg;
         int32_t rc = PRG_OK;
         double lam = 0.0;
-        if (!neg && small_eigenvector(n, m, from, to, weights, o.eps, hub, &lam, &rc)) {
+        Uploaded up;
+        if (!neg && small_eigenvector(n, m, from, to, weights, o.eps, hub, &lam, &rc, &up)) {
             if (rc != PRG_OK) return rc;
             for (uint32_t i = 0; i < n; i++) authority[i] = hub[i];
             if (eigenvalue) *eigenvalue = lam * lam;
             return PRG_OK;
         }
         prg_graph *h = nullptr;
-        rc = create_from_host(n, m, from, to, weights, 0, &h);
+        rc = create_from_host(n, m, from, to, weights, 0, &h, -1, nullptr, &up);
         if (rc != PRG_OK) return rc;
         try {
             cudaStream_t s = h->stream;

@@ -678,12 +678,23 @@ static size_t res_limits(uint64_t arcs, uint32_t n, unsigned &nb) {
     return std::min(kResSmem, (size_t)optin - kResStatic);
 }
 
+// Most 8-arc chunks of a block's share.
+static uint64_t most_chunks(uint64_t arcs, unsigned nb) {
+    return std::min<uint64_t>(kResMaxChunks, (arcs / nb + kResExcess) / 8 + 1);
+}
+
 // Whether the mean share, streamed, fits a block.
 static bool res_mean_fits(uint32_t n, uint64_t arcs, bool weighted, int kind) {
     unsigned nb = 0;
     const size_t most = res_limits(arcs, n, nb);
     const uint64_t chunks = arcs / 8 / nb;
     return chunks <= kResMaxChunks && res_bytes(n / nb, (uint32_t)chunks, kind, weighted, true) <= most;
+}
+
+uint32_t res_longest_row(uint32_t n, uint64_t arcs) {
+    unsigned nb = 0;
+    res_limits(arcs, n, nb);
+    return 8 * (uint32_t)most_chunks(arcs, nb);
 }
 
 bool res_sizes_fit(uint32_t n, uint64_t arcs, bool weighted, int kind) {
@@ -728,11 +739,11 @@ ResPlan res_plan(const DeviceGraph &g, int kind, cudaStream_t s) {
     PRG_CUDA(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, s));
     PRG_CUDA(cudaFreeAsync(d, s));
     PRG_CUDA(cudaStreamSynchronize(s));
-    const uint64_t most_chunks = std::min<uint64_t>(kResMaxChunks, (g.arcs / nb + kResExcess) / 8 + 1);
+    const uint64_t top = most_chunks(g.arcs, nb);
     for (unsigned k = 0; k < kResSplits; k++) {
         const bool stream = h[3 * k] > most;
         const uint32_t bytes = h[3 * k + (stream ? 1 : 0)];
-        if (bytes > most || h[3 * k + 2] > most_chunks) continue;
+        if (bytes > most || h[3 * k + 2] > top) continue;
         p.alpha = res_alpha(k);
         p.stream = stream;
         p.grid = nb;

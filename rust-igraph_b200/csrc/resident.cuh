@@ -53,6 +53,8 @@ struct ResArgs {
 ResPlan res_plan(const DeviceGraph &g, int kind, cudaStream_t s);
 // Whether a graph of these sizes can have a plan at all, whatever its rows.
 bool res_sizes_fit(uint32_t n, uint64_t arcs, bool weighted, int kind);
+// No plan holds a longer row.
+uint32_t res_longest_row(uint32_t n, uint64_t arcs);
 // The plan before the graph is built, for graphs whose indices surely stay in
 // shared memory as long as no row is long (ResArgs::longest checks that).
 ResPlan res_plan_blind(uint32_t n, uint64_t arcs, bool weighted, int kind);

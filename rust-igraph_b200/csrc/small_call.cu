@@ -19,9 +19,11 @@
 // and these graphs' vectors fit L2).  Weighted directed graphs run the same
 // phases a second time by source for the out-strengths.
 //
-// Limits: res_sizes_fit.  Where res_plan_blind gives no plan, or the rows turn out
-// too uneven for its shares (Ctl::status), the iteration is planned from the CSR
-// just built, and only if that fails does the caller take the general path.
+// Limits: res_sizes_fit, and rows of up to res_longest_row arcs: the first arc
+// past that ends the build.  Where res_plan_blind gives no plan, or the rows turn
+// out too uneven for its shares (Ctl::status), the iteration is planned from the
+// CSR just built, and only if that fails does the caller take the general path,
+// with the edge list as uploaded here.
 #include "small_call.cuh"
 
 #include <algorithm>
@@ -44,6 +46,7 @@ constexpr uint32_t kSmallRange = 1u << 20;           // ids per bitmap of the bl
 __host__ __device__ constexpr uint32_t small_word(uint32_t i) { return i + (i >> 5); }
 constexpr size_t kSmallSmem = small_word(kSmallRange / 32) * 4;  // also 32 warp buffers
 constexpr uint32_t kSmallSpins = 1u << 21;
+constexpr size_t kSmallJoint = 8 << 20;
 static_assert(kSmallSmem >= (size_t)(kSmallNT / 32) * kSmallWarpBuf * 4, "warp buffers");
 
 struct SmallSide {
@@ -58,7 +61,7 @@ struct SmallSide {
 struct SmallArgs {
     const uint32_t *from, *to;
     const double *w;
-    uint32_t n, m;
+    uint32_t n, m, longest;  // longest: of a row
     int directed, check_w, seed;  // seed 0: none, 1: ones, 2: dval / max dval (ones when that is 0)
     SmallSide in, outs;      // outs only for weighted directed graphs
     uint32_t *deg;           // directed, unweighted: out-degrees, zero at launch
@@ -66,7 +69,7 @@ struct SmallArgs {
     double *w64;             // arcs + kColPad
     double *dval, *start;
     // [0] largest endpoint [1] longest in-row [2] barrier [3], [4] listed in- / out-rows [5] ~first refused
-    // weight's edge (0: none) [6..7] max dval bits
+    // weight's edge (0: none) [6..7] max dval bits [8] a row is too long
     uint32_t *word;          // zero at launch
     Ctl *ctl;
 };
@@ -141,21 +144,26 @@ __global__ void __launch_bounds__(kSmallNT, 1) small_build_kernel(const SmallArg
     const bool two = a.w != nullptr && a.directed;
     uint32_t phase = 0;
 
-    // 1: slots
+    // 1: slots.  A row too long for any plan ends the phase: its arcs' atomics on
+    // one word and its sort by one block would be in vain (a row of 5 M arcs held
+    // a call up by 20 ms).  A slot is looked at one step later, when it has arrived.
     {
-        uint32_t mx = 0, bad = 0;
+        uint32_t mx = 0, bad = 0, s0 = 0, s1 = 0;
+        uint32_t *too_long = a.word + 8;
         for (uint32_t e = gtid; e < m; e += gn) {
             const uint32_t u = a.from[e], v = a.to[e];
+            if (*(volatile uint32_t *)too_long) break;
+            if (max(s0, s1) >= a.longest) *(volatile uint32_t *)too_long = 1u;
             mx = max(mx, max(u, v));
             if (a.check_w && !(a.w[e] >= 0.0 && isfinite(a.w[e]))) bad = max(bad, ~e);
             if (u >= n || v >= n) continue;
             if (a.directed) {
-                a.in.slot[e] = atomicAdd(&a.in.cnt[v], 1u);
+                a.in.slot[e] = s0 = atomicAdd(&a.in.cnt[v], 1u);
                 if (two) a.outs.slot[e] = atomicAdd(&a.outs.cnt[u], 1u);
                 else atomicAdd(&a.deg[u], 1u);
             } else {
-                a.in.slot[2 * e] = atomicAdd(&a.in.cnt[u], 1u);
-                a.in.slot[2 * e + 1] = atomicAdd(&a.in.cnt[v], 1u);
+                a.in.slot[2 * e] = s0 = atomicAdd(&a.in.cnt[u], 1u);
+                a.in.slot[2 * e + 1] = s1 = atomicAdd(&a.in.cnt[v], 1u);
             }
         }
         mx = __reduce_max_sync(0xffffffffu, mx);
@@ -163,7 +171,11 @@ __global__ void __launch_bounds__(kSmallNT, 1) small_build_kernel(const SmallArg
         if (bad) atomicMax(a.word + 5, bad);
     }
     if (!small_barrier(a, phase)) return;
-    if (*(volatile uint32_t *)(a.word + 5) != 0u) {  // every block sees the same
+    if (*(volatile uint32_t *)(a.word + 8) != 0u) {  // every block sees the same
+        if (gtid == 0) a.ctl->status = SMALL_LONG_ROW;
+        return;
+    }
+    if (*(volatile uint32_t *)(a.word + 5) != 0u) {
         if (gtid == 0) a.ctl->status = SMALL_BAD_WEIGHT;
         return;
     }
@@ -359,7 +371,7 @@ SmallStatus small_call(const SmallCall &c, double *out, SmallResult &r, cudaStre
     // few arcs need few blocks: a barrier over fewer is shorter
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(sms, (arcs + n) / 2048));
 
-    // one allocation: first what must be zero, then the rest
+    // scratch: first what must be zero, then the rest
     size_t at = 0;
     auto take = [&](size_t bytes) {
         const size_t o = at;
@@ -368,32 +380,38 @@ SmallStatus small_call(const SmallCall &c, double *out, SmallResult &r, cudaStre
     };
     const size_t o_ctl = take(sizeof(Ctl)), o_word = take(64), o_bar = take(4), o_cnt = take(n * 4ull),
                  o_deg = take(c.directed && !c.w ? n * 4ull : 4), o_cnt2 = take(two ? n * 4ull : 4), zeroed = at;
-    const size_t o_from = take(c.m * 4), o_to = take(c.m * 4), o_w = take(c.w ? c.m * 8 : 8),
-                 o_slot = take(arcs * 4), o_ptr = take((n + 1ull) * 4), o_ids = take(arcs * 4), o_bs = take(grid * 4ull),
+    const size_t o_slot = take(arcs * 4), o_ptr = take((n + 1ull) * 4), o_ids = take(arcs * 4), o_bs = take(grid * 4ull),
                  o_long = take(n * 4ull), o_slot2 = take(two ? arcs * 4 : 4), o_ptr2 = take(two ? (n + 1ull) * 4 : 4),
                  o_ids2 = take(two ? arcs * 4 : 4), o_bs2 = take(grid * 4ull), o_long2 = take(two ? n * 4ull : 4),
                  o_col = take((arcs + kColPad) * 4), o_w64 = take(c.w ? (arcs + kColPad) * 8 : 8), o_dval = take(n * 8ull),
                  o_x = take(n * 8ull), o_t = take(c.reset ? n * 8ull : 8), o_xt0 = take(n * 8ull), o_xt1 = take(n * 8ull),
                  o_rec = take(res_scratch_bytes(kResBlocks));
-    unsigned char *b = nullptr;
+    // The edge list may outlive the rest, so it is an allocation of its own where
+    // the rest would be missed (a second allocation takes 3 us).
+    const size_t ids = (c.m * 4 + 255) & ~(size_t)255, edges = 2 * ids + (c.w ? c.m * 8 : 0);
+    const bool joint = at <= kSmallJoint;
+    unsigned char *b = nullptr, *eb = nullptr;
     Ctl *h = static_cast<Ctl *>(pinned_acquire());
     SmallStatus status = SMALL_DONE;
     try {
-        PRG_CUDA(cudaMallocAsync((void **)&b, at, s));
+        PRG_CUDA(cudaMallocAsync((void **)&b, joint ? at + edges : at, s));
+        if (joint) eb = b + at;
+        else PRG_CUDA(cudaMallocAsync((void **)&eb, edges, s));
         PRG_CUDA(cudaMemsetAsync(b, 0, zeroed, s));
-        PRG_CUDA(cudaMemcpyAsync(b + o_from, c.from, c.m * 4, cudaMemcpyHostToDevice, s));
-        PRG_CUDA(cudaMemcpyAsync(b + o_to, c.to, c.m * 4, cudaMemcpyHostToDevice, s));
-        if (c.w) PRG_CUDA(cudaMemcpyAsync(b + o_w, c.w, c.m * 8, cudaMemcpyHostToDevice, s));
+        PRG_CUDA(cudaMemcpyAsync(eb, c.from, c.m * 4, cudaMemcpyHostToDevice, s));
+        PRG_CUDA(cudaMemcpyAsync(eb + ids, c.to, c.m * 4, cudaMemcpyHostToDevice, s));
+        if (c.w) PRG_CUDA(cudaMemcpyAsync(eb + 2 * ids, c.w, c.m * 8, cudaMemcpyHostToDevice, s));
         if (c.reset) PRG_CUDA(cudaMemcpyAsync(b + o_t, c.reset, n * 8ull, cudaMemcpyHostToDevice, s));
         auto u32 = [&](size_t o) { return reinterpret_cast<uint32_t *>(b + o); };
         auto f64 = [&](size_t o) { return reinterpret_cast<double *>(b + o); };
         SmallArgs a;
         std::memset(&a, 0, sizeof(a));
-        a.from = u32(o_from);
-        a.to = u32(o_to);
-        a.w = c.w ? f64(o_w) : nullptr;
+        a.from = reinterpret_cast<uint32_t *>(eb);
+        a.to = reinterpret_cast<uint32_t *>(eb + ids);
+        a.w = c.w ? reinterpret_cast<double *>(eb + 2 * ids) : nullptr;
         a.n = n;
         a.m = (uint32_t)c.m;
+        a.longest = res_longest_row(n, arcs);
         a.directed = c.directed ? 1 : 0;
         a.check_w = c.w && c.check_weights ? 1 : 0;
         a.seed = c.kind == RES_EIG ? (c.strength_seed ? 2 : 1) : 0;
@@ -468,7 +486,7 @@ SmallStatus small_call(const SmallCall &c, double *out, SmallResult &r, cudaStre
         }
         if (status == SMALL_DONE) {
             if (h->status == 7) throw TimeoutError{"small-graph call: a grid barrier timed out"};
-            status = (SmallStatus)h->status;
+            status = h->status == SMALL_LONG_ROW ? SMALL_NOT_HERE : (SmallStatus)h->status;
             r.max_endpoint = h_word[0];
             r.bad_edge = ~h_word[5];
             r.iterations = h->iters;
@@ -481,10 +499,20 @@ SmallStatus small_call(const SmallCall &c, double *out, SmallResult &r, cudaStre
     } catch (...) {
         cudaStreamSynchronize(s);
         if (b) cudaFreeAsync(b, s);
+        if (eb && !joint) cudaFreeAsync(eb, s);
         pinned_release(h);
         throw;
     }
-    cudaFreeAsync(b, s);
+    if (status == SMALL_NOT_HERE) {
+        r.edges.block = joint ? b : eb;
+        r.edges.from = reinterpret_cast<uint32_t *>(eb);
+        r.edges.to = reinterpret_cast<uint32_t *>(eb + ids);
+        r.edges.w = c.w ? reinterpret_cast<double *>(eb + 2 * ids) : nullptr;
+        if (!joint) cudaFreeAsync(b, s);
+    } else {
+        cudaFreeAsync(b, s);
+        if (!joint) cudaFreeAsync(eb, s);
+    }
     pinned_release(h);
     return status;
 }

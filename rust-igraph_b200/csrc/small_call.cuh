@@ -23,9 +23,17 @@ struct SmallCall {
     bool strength_seed = false;     // RES_EIG: start from the row sums over their maximum (else from ones)
 };
 
+// An uploaded edge list (one allocation).
+struct SmallEdges {
+    unsigned char *block = nullptr;  // null: nothing is held
+    const uint32_t *from = nullptr, *to = nullptr;
+    const double *w = nullptr;
+};
+
 struct SmallResult {
     uint32_t iterations = 0, max_endpoint = 0, bad_edge = 0;
     double eigenvalue = 0;
+    SmallEdges edges;  // SMALL_NOT_HERE after the upload: for the general path, the caller's to free
 };
 
 enum SmallStatus : int32_t {
@@ -33,6 +41,7 @@ enum SmallStatus : int32_t {
     SMALL_NOT_HERE = 1,      // take the general path (nothing written to out)
     SMALL_OUT_OF_RANGE = 2,  // an endpoint is >= n: SmallResult::max_endpoint
     SMALL_BAD_WEIGHT = 3,    // check_weights: SmallResult::bad_edge is the first such edge
+    SMALL_LONG_ROW = 4,      // (device) a row no plan holds
 };
 
 // Solves into out (host double[n]).  Sizes, tuning and the rows' lengths

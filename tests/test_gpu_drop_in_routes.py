@@ -89,3 +89,35 @@ def test_long_rows_do_not_hold_up_one_block(cuda_ok, longest, resident, weighted
     call = "eigenvector_weighted" if weighted else "eigenvector"
     _, names, _ = traced(lambda: CALLS[call](g, w), str(tmp_path / "eigen.json"))
     assert any("seg8_kernel" in k for k in names) != resident
+
+
+@pytest.mark.parametrize("kind", CALLS)
+@pytest.mark.parametrize("m,longest", [(100_000, 99_000), (600_000, 90_000), (1_500_000, 700_000), (9_000_000, 400_000)])
+def test_long_rows_upload_once(cuda_ok, kind, m, longest, tmp_path):
+    # rows no plan holds, found in the build (or, with few edges a thread, by the plan)
+    if kind != "pagerank" and m > 5_000_000:
+        pytest.skip("more than 10 M arcs, or a long call")
+    n = 60_000
+    f, t = hub_graph(n, m, longest)
+    directed = not kind.startswith("eigen")
+    if not directed:
+        f, t = np.minimum(f, t), np.maximum(f, t)
+    g, w = ig.Graph.from_edge_arrays(n, f, t, directed), np.random.default_rng(2).random(m) + 0.5
+    (x, names, up), (ref, _, ref_up) = both(lambda: CALLS[kind](g, w), tmp_path)
+    assert any("small_build_kernel" in k for k in names)
+    assert up == ref_up
+    assert np.array_equal(x, ref)
+
+
+def test_long_rows_report_what_is_wrong_with_the_input(cuda_ok):
+    # the build ends early, the errors are the general path's
+    n, m = 60_000, 1_500_000
+    f, t = hub_graph(n, m, 700_000)
+    w = np.ones(m)
+    w[m - 1] = -1.0
+    g = ig.Graph.from_edge_arrays(n, f, t, True)
+    with pytest.raises(ig.InvalidArgument, match=f"weight at edge {m - 1} must be non-negative"):
+        ig.pagerank_weighted(g, w)
+    t[m - 1] = n
+    with pytest.raises(Exception, match=f"vertex id {n} out of range"):
+        ig._check(ig.lib().prg_pagerank(n, m, ig._ptr(f), ig._ptr(t), 1, ig._ptr(np.empty(n))))
