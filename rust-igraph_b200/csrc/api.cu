@@ -48,6 +48,7 @@ void set_last_error(const std::string &msg) { g_err = msg; }
 namespace {
 
 int32_t from_cuda(const prg::CudaError &e) {
+    cudaGetLastError();  // reported here: the caller's next runtime call must not see it again
     if (e.err == cudaErrorMemoryAllocation) return fail(PRG_ERR_OUT_OF_MEMORY, "cuda: out of memory");
     return fail(PRG_ERR_CUDA, std::string("cuda: ") + cudaGetErrorString(e.err) + " (" + e.what + ")");
 }
@@ -150,6 +151,24 @@ static std::string range_message(uint32_t mx, uint32_t n) {
     return "vertex id " + std::to_string(mx) + " out of range (vcount = " + std::to_string(n) + ")";
 }
 
+// Frees a handle; its stream stays.
+static void drop(prg_graph *h) {
+    cudaStream_t s = h->stream;
+    prg::workspace_free(h->ws, s);
+    for (void *p : {(void *)h->g.row_ptr, (void *)h->g.col, (void *)h->g.w64, (void *)h->g.w32, (void *)h->g.deg,
+                    (void *)h->g.dval, (void *)h->g.inv32, (void *)h->g.rb, (void *)h->g.hubs, (void *)h->g.perm,
+                    (void *)h->g.iperm, (void *)h->d_reset, (void *)h->d_out, (void *)h->d_start})
+        if (p) cudaFreeAsync(p, s);
+    delete h;
+}
+
+void destroy(prg_graph *h) {
+    if (!h) return;
+    cudaStream_t s = h->stream;
+    drop(h);
+    prg::stream_release(s);
+}
+
 // Creates a handle from device edge arrays (copies nothing on the host).
 int32_t create_from_device(uint32_t n, uint64_t m, const uint32_t *d_from, const uint32_t *d_to, const double *d_w,
                            int32_t directed, cudaStream_t s, prg_graph **out, int relabel = -1) {
@@ -159,22 +178,32 @@ int32_t create_from_device(uint32_t n, uint64_t m, const uint32_t *d_from, const
     // every endpoint must be < n (Graph::add_edges rejects others with
     // IgraphError::VertexOutOfRange, graph.rs:756-785)
     uint32_t mx = 0;
-    if (!prg::build_graph(h->g, d_from, d_to, d_w, s, &mx)) {
-        delete h;
+    bool ok = false;
+    try {
+        ok = prg::build_graph(h->g, d_from, d_to, d_w, s, &mx);
+    } catch (...) {
+        drop(h);
+        throw;
+    }
+    if (!ok) {
+        drop(h);
         return fail(PRG_ERR_VERTEX_OUT_OF_RANGE, range_message(mx, n));
     }
     *out = h;
     return PRG_OK;
 }
 
-void destroy(prg_graph *h);
-
-// The graph with every edge reversed, from the same device edge arrays, on a
-// stream of its own; complete when it returns.
-static int32_t create_reverse(uint32_t n, uint64_t m, const uint32_t *d_from, const uint32_t *d_to, const double *d_w,
-                              int32_t directed, prg_graph **rev, int relabel) {
+// The same on a stream of its own; complete when it returns.
+static int32_t create_on_own_stream(uint32_t n, uint64_t m, const uint32_t *d_from, const uint32_t *d_to,
+                                    const double *d_w, int32_t directed, prg_graph **out, int relabel = -1) {
     cudaStream_t s = prg::stream_acquire();
-    const int32_t rc = create_from_device(n, m, d_to, d_from, d_w, directed, s, rev, relabel);
+    int32_t rc = PRG_OK;
+    try {
+        rc = create_from_device(n, m, d_from, d_to, d_w, directed, s, out, relabel);
+    } catch (...) {
+        prg::stream_release(s);
+        throw;
+    }
     if (rc != PRG_OK) prg::stream_release(s);
     return rc;
 }
@@ -197,18 +226,16 @@ int32_t create_from_host(uint32_t n, uint64_t m, const uint32_t *from, const uin
                          int32_t directed, prg_graph **out, int relabel = -1, prg_graph **rev = nullptr,
                          Uploaded *up = nullptr) {
     if (!ensure_pool_config()) return fail(PRG_ERR_CUDA, "cuda: no usable device");
-    cudaStream_t s = prg::stream_acquire();
-    if (m > 0xFFFFFFFFull) {
-        prg::stream_release(s);
-        return fail(PRG_ERR_INTERNAL, "ecount overflows u32");
-    }
+    if (m > 0xFFFFFFFFull) return fail(PRG_ERR_INTERNAL, "ecount overflows u32");
     if (up && up->e.block) {
-        const int32_t rc = create_from_device(n, m, up->e.from, up->e.to, up->e.w, directed, s, out, relabel);
-        cudaFreeAsync(up->e.block, s);
-        up->e.block = nullptr;
-        if (rc != PRG_OK) prg::stream_release(s);
+        const int32_t rc = create_on_own_stream(n, m, up->e.from, up->e.to, up->e.w, directed, out, relabel);
+        if (rc == PRG_OK) {
+            cudaFreeAsync(up->e.block, (*out)->stream);
+            up->e.block = nullptr;
+        }
         return rc;
     }
+    cudaStream_t s = prg::stream_acquire();
     if (m >= prg::kStreamMinEdges && !(w && (directed || rev))) {
         // large edge lists: chunked copies overlapped with the build
         int32_t rc = check_sizes(n, m, directed);
@@ -217,17 +244,20 @@ int32_t create_from_host(uint32_t n, uint64_t m, const uint32_t *from, const uin
             uint32_t mx = 0;
             bool ok = false;
             prg::DeviceEdges edges;
+            auto free_edges = [&]() {
+                if (edges.from) cudaFreeAsync(edges.from, s);
+                if (edges.to) cudaFreeAsync(edges.to, s);
+            };
             try {
                 ok = prg::build_graph_host(h->g, from, to, w, s, &mx, rev ? &edges : nullptr);
-                if (ok && rev) {
-                    rc = create_reverse(n, m, edges.from, edges.to, nullptr, directed, rev, relabel);
-                    cudaFreeAsync(edges.from, s);
-                    cudaFreeAsync(edges.to, s);
-                }
+                if (ok && rev)
+                    rc = create_on_own_stream(n, m, edges.to, edges.from, nullptr, directed, rev, relabel);
             } catch (...) {
+                free_edges();
                 destroy(h);
                 throw;
             }
+            free_edges();
             if (rc != PRG_OK) {
                 destroy(h);
                 return rc;
@@ -245,27 +275,41 @@ int32_t create_from_host(uint32_t n, uint64_t m, const uint32_t *from, const uin
     uint32_t *d_f = nullptr, *d_t = nullptr;
     double *d_w = nullptr;
     const uint64_t mm = m ? m : 1;
-    PRG_CUDA(cudaMallocAsync((void **)&d_f, mm * 4, s));
-    PRG_CUDA(cudaMallocAsync((void **)&d_t, mm * 4, s));
-    if (m) {
-        PRG_CUDA(cudaMemcpyAsync(d_f, from, m * 4, cudaMemcpyHostToDevice, s));
-        PRG_CUDA(cudaMemcpyAsync(d_t, to, m * 4, cudaMemcpyHostToDevice, s));
-    }
-    if (w) {
-        PRG_CUDA(cudaMallocAsync((void **)&d_w, mm * 8, s));
-        if (m) PRG_CUDA(cudaMemcpyAsync(d_w, w, m * 8, cudaMemcpyHostToDevice, s));
-    }
-    int32_t rc = create_from_device(n, m, d_f, d_t, w ? d_w : nullptr, directed, s, out, relabel);
-    const bool built = rc == PRG_OK;
-    if (built && rev) rc = create_reverse(n, m, d_f, d_t, w ? d_w : nullptr, directed, rev, relabel);
-    cudaFreeAsync(d_f, s);
-    cudaFreeAsync(d_t, s);
-    if (d_w) cudaFreeAsync(d_w, s);
-    if (rc != PRG_OK) {
-        if (built) destroy(*out);  // and the stream
+    prg_graph *h = nullptr;
+    int32_t rc = PRG_OK;
+    auto free_edges = [&]() {
+        for (void *p : {(void *)d_f, (void *)d_t, (void *)d_w})
+            if (p) cudaFreeAsync(p, s);
+    };
+    auto give_up = [&]() {
+        free_edges();
+        if (h) destroy(h);  // and the stream
         else prg::stream_release(s);
+    };
+    try {
+        PRG_CUDA(cudaMallocAsync((void **)&d_f, mm * 4, s));
+        PRG_CUDA(cudaMallocAsync((void **)&d_t, mm * 4, s));
+        if (m) {
+            PRG_CUDA(cudaMemcpyAsync(d_f, from, m * 4, cudaMemcpyHostToDevice, s));
+            PRG_CUDA(cudaMemcpyAsync(d_t, to, m * 4, cudaMemcpyHostToDevice, s));
+        }
+        if (w) {
+            PRG_CUDA(cudaMallocAsync((void **)&d_w, mm * 8, s));
+            if (m) PRG_CUDA(cudaMemcpyAsync(d_w, w, m * 8, cudaMemcpyHostToDevice, s));
+        }
+        rc = create_from_device(n, m, d_f, d_t, d_w, directed, s, &h, relabel);
+        if (rc == PRG_OK && rev) rc = create_on_own_stream(n, m, d_t, d_f, d_w, directed, rev, relabel);
+    } catch (...) {
+        give_up();
+        throw;
     }
-    return rc;
+    if (rc != PRG_OK) {
+        give_up();
+        return rc;
+    }
+    free_edges();
+    *out = h;
+    return PRG_OK;
 }
 
 // Set-up for a handle returned to the caller: the allocation-free solve's
@@ -280,31 +324,6 @@ static void prepare_handle(prg_graph *&h) {
         h = nullptr;
         throw;
     }
-}
-
-void destroy(prg_graph *h) {
-    if (!h) return;
-    cudaStream_t s = h->stream;
-    prg::workspace_free(h->ws, s);
-    auto f = [&](void *p) {
-        if (p) cudaFreeAsync(p, s);
-    };
-    f(h->g.row_ptr);
-    f(h->g.col);
-    f(h->g.w64);
-    f(h->g.w32);
-    f(h->g.deg);
-    f(h->g.dval);
-    f(h->g.inv32);
-    f(h->g.rb);
-    f(h->g.hubs);
-    f(h->g.perm);
-    f(h->g.iperm);
-    f(h->d_reset);
-    f(h->d_out);
-    f(h->d_start);
-    prg::stream_release(s);
-    delete h;
 }
 
 prg::SolveOpts to_solve_opts(const prg_options *o) {
@@ -1005,10 +1024,8 @@ int32_t prg_graph_create_device(uint32_t n, uint64_t m, const uint32_t *d_from, 
     if (!out) return fail(PRG_ERR_INVALID_ARGUMENT, "null output handle");
     *out = nullptr;
     if (!ensure_pool_config()) return fail(PRG_ERR_CUDA, "cuda: no usable device");
-    cudaStream_t s = prg::stream_acquire();
-    int32_t rc = create_from_device(n, m, d_from, d_to, d_weights, directed, s, out);
-    if (rc != PRG_OK) prg::stream_release(s);
-    else prepare_handle(*out);
+    const int32_t rc = create_on_own_stream(n, m, d_from, d_to, d_weights, directed, out);
+    if (rc == PRG_OK) prepare_handle(*out);
     return rc;
     PRG_GUARD_END
 }

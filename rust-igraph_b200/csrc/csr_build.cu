@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
+#include <exception>
 #include <vector>
 
 #include "graph.cuh"
@@ -36,15 +37,42 @@ static inline unsigned grid_for(uint64_t n, unsigned per_block, unsigned cap = 1
     return (unsigned)g;
 }
 
+// What the build running on this thread holds: an exception (out of device
+// memory) frees it.
+struct Scratch {
+    cudaStream_t s;
+    std::vector<void *> held;
+    Scratch *outer;
+    int unwinding = std::uncaught_exceptions();
+    static thread_local Scratch *top;
+    explicit Scratch(cudaStream_t stream) : s(stream), outer(top) { top = this; }
+    Scratch(const Scratch &) = delete;
+    ~Scratch() {
+        top = outer;
+        if (std::uncaught_exceptions() == unwinding) return;
+        for (void *p : held) cudaFreeAsync(p, s);
+    }
+    // p is freed, or the graph's from here on
+    static void forget(void *p) {
+        if (!top) return;
+        auto &h = top->held;
+        h.erase(std::remove(h.begin(), h.end(), p), h.end());
+    }
+};
+thread_local Scratch *Scratch::top = nullptr;
+
 template <class T>
 static T *dalloc(uint64_t count, cudaStream_t s) {
     void *p = nullptr;
     PRG_CUDA(cudaMallocAsync(&p, std::max<uint64_t>(count, 1) * sizeof(T), s));
+    if (Scratch::top) Scratch::top->held.push_back(p);
     return (T *)p;
 }
 template <class T>
 static void dfree(T *&p, cudaStream_t s) {
-    if (p) cudaFreeAsync(p, s);
+    if (!p) return;
+    Scratch::forget((void *)p);
+    cudaFreeAsync((void *)p, s);
     p = nullptr;
 }
 
@@ -693,7 +721,9 @@ void build_row_blocks(DeviceGraph &g, uint32_t capw, uint32_t shortmax, uint32_t
     g.nrb = hv[0];
     g.nhub = hv[1];
     g.rb = dalloc<uint4>(g.nrb, s);
+    Scratch::forget(g.rb);
     g.hubs = dalloc<Hub>(g.nhub, s);
+    Scratch::forget(g.hubs);
     rb_fill<<<gb, kThreads, 0, s>>>(g.row_ptr, n, shortmax, split, off, hoff, g.rb, g.hubs);
     rb_fix<<<grid_for(g.nrb, kThreads), kThreads, 0, s>>>(g.row_ptr, g.rb, g.nrb, n);
     PRG_CUDA(cudaGetLastError());
@@ -771,6 +801,7 @@ static bool relabel_vertices(DeviceGraph &g, cudaStream_t s, const uint32_t *in_
     relabel_finish<<<gn, kThreads, 0, s>>>(g.perm, g.deg, n, g.iperm, deg_new);
     cudaFreeAsync(g.deg, s);
     g.deg = deg_new;
+    Scratch::forget(g.deg);
     dfree(pk, s);
     dfree(pv, s);
     dfree(pk1, s);
@@ -780,6 +811,7 @@ static bool relabel_vertices(DeviceGraph &g, cudaStream_t s, const uint32_t *in_
 
 bool build_graph(DeviceGraph &g, const uint32_t *d_from, const uint32_t *d_to, const double *d_w, cudaStream_t s,
                  uint32_t *max_endpoint) {
+    Scratch scratch(s);
     cudaEvent_t e0, e1;
     PRG_CUDA(cudaEventCreate(&e0));
     PRG_CUDA(cudaEventCreate(&e1));
@@ -861,6 +893,7 @@ bool build_graph(DeviceGraph &g, const uint32_t *d_from, const uint32_t *d_to, c
     double *strength = nullptr;
     if (!weighted && !relabelled && vs != d_from) {
         g.col = v[vs == v[1]];  // in place
+        Scratch::forget(g.col);
         v[vs == v[1]] = nullptr;
     } else {
         PRG_CUDA(cudaMallocAsync((void **)&g.col, padded * 4, s));
@@ -1001,6 +1034,7 @@ __global__ void place_arcs(const uint32_t *pos, const uint32_t *val, uint64_t ar
 
 bool build_graph_host(DeviceGraph &g, const uint32_t *h_from, const uint32_t *h_to, const double *h_w, cudaStream_t s,
                       uint32_t *max_endpoint, DeviceEdges *keep) {
+    Scratch scratch(s);
     cudaEvent_t e0, e1;
     PRG_CUDA(cudaEventCreate(&e0));
     PRG_CUDA(cudaEventCreate(&e1));
@@ -1027,7 +1061,15 @@ bool build_graph_host(DeviceGraph &g, const uint32_t *h_from, const uint32_t *h_
     uint32_t *ka = dalloc<uint32_t>(chunk_arcs, s), *va = dalloc<uint32_t>(chunk_arcs, s);
     uint32_t *kb = dalloc<uint32_t>(chunk_arcs, s), *vb = dalloc<uint32_t>(chunk_arcs, s);
 
-    cudaStream_t cs = stream_acquire();
+    struct CopyStream {
+        cudaStream_t s = stream_acquire();
+        ~CopyStream() { release(); }
+        void release() {  // waits for the copies
+            if (s) stream_release(s);
+            s = nullptr;
+        }
+    } copies;
+    const cudaStream_t cs = copies.s;
     std::vector<cudaEvent_t> ev(nchunks + 1);
     for (cudaEvent_t &e : ev) PRG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     // the copy stream starts once the allocations above are usable
@@ -1063,7 +1105,7 @@ bool build_graph_host(DeviceGraph &g, const uint32_t *h_from, const uint32_t *h_
     PRG_CUDA(cudaMemcpyAsync(&mx, d_mx, 4, cudaMemcpyDeviceToHost, s));
     PRG_CUDA(cudaStreamSynchronize(s));
     for (cudaEvent_t &e : ev) cudaEventDestroy(e);
-    stream_release(cs);
+    copies.release();
     dfree(ka, s);
     dfree(va, s);
     dfree(kb, s);
@@ -1131,6 +1173,8 @@ bool build_graph_host(DeviceGraph &g, const uint32_t *h_from, const uint32_t *h_
     }
     if (keep) {
         *keep = DeviceEdges{d_from, d_to};
+        Scratch::forget(d_from);
+        Scratch::forget(d_to);
     } else {
         dfree(d_from, s);
         dfree(d_to, s);
