@@ -393,6 +393,12 @@ SmallStatus small_call(const SmallCall &c, double *out, SmallResult &r, cudaStre
     unsigned char *b = nullptr, *eb = nullptr;
     Ctl *h = static_cast<Ctl *>(pinned_acquire());
     SmallStatus status = SMALL_DONE;
+    auto give_up = [&]() {
+        cudaStreamSynchronize(s);
+        if (b) cudaFreeAsync(b, s);
+        if (eb && !joint) cudaFreeAsync(eb, s);
+        pinned_release(h);
+    };
     try {
         PRG_CUDA(cudaMallocAsync((void **)&b, joint ? at + edges : at, s));
         if (joint) eb = b + at;
@@ -496,11 +502,13 @@ SmallStatus small_call(const SmallCall &c, double *out, SmallResult &r, cudaStre
                 PRG_CUDA(cudaStreamSynchronize(s));
             }
         }
+    } catch (const CudaError &e) {
+        give_up();
+        if (e.err != cudaErrorMemoryAllocation) throw;
+        cudaGetLastError();
+        return SMALL_NOT_HERE;  // (the general path's build takes less where ids have few bits)
     } catch (...) {
-        cudaStreamSynchronize(s);
-        if (b) cudaFreeAsync(b, s);
-        if (eb && !joint) cudaFreeAsync(eb, s);
-        pinned_release(h);
+        give_up();
         throw;
     }
     if (status == SMALL_NOT_HERE) {

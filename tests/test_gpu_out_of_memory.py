@@ -74,3 +74,27 @@ def test_hits_gives_back_what_it_allocated(cuda_ok, weighted, m):
             assert np.array_equal(r.hub, ref.hub)
             break
     assert outcomes[-1] and outcomes.count(False) >= 5
+
+
+def test_drop_in_goes_where_there_is_room(cuda_ok):
+    # 8-bit ids: the general build sorts in one pass and takes less memory than the small-graph path
+    n, m = 200, 8_000_000
+    rng = np.random.default_rng(m)
+    f, t = rng.integers(0, n, m).astype(np.uint32), rng.integers(0, n, m).astype(np.uint32)
+    g = ig.Graph.from_edge_arrays(n, f, t, True)
+    ref = ig.pagerank(g)
+    pool = Pool()
+    before = pool.used()
+    outcomes = []
+    for size in range(96 * MB, 320 * MB, 8 * MB):
+        try:
+            ig.set_tuning("resident", 0)
+            general = with_free_memory(pool, size, lambda: ig.pagerank(g))
+        finally:
+            ig.reset_tuning()
+        x = with_free_memory(pool, size, lambda: ig.pagerank(g))
+        outcomes.append((general is not None, x is not None))
+        assert pool.used() - before <= MB
+        assert x is None or np.abs(x - ref).max() <= 1e-10
+    assert (False, False) in outcomes and (True, True) in outcomes
+    assert (True, False) not in outcomes
