@@ -663,19 +663,24 @@ __global__ void __launch_bounds__(kResNT, 1) res_kernel(const ResArgs a) {
 
 // ------------------------------------------------------------------ host side
 
+const DeviceLimits &device_limits() {
+    static const DeviceLimits limits = []() {
+        DeviceLimits d;
+        int dev = 0;
+        PRG_CUDA(cudaGetDevice(&dev));
+        PRG_CUDA(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
+        PRG_CUDA(cudaDeviceGetAttribute(&d.smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+        return d;
+    }();
+    return limits;
+}
+
 // Shared memory a block may take, and the blocks of a launch.
 static size_t res_limits(uint64_t arcs, uint32_t n, unsigned &nb) {
-    static int sms = 0, optin = 0;
-    if (sms == 0) {
-        int dev = 0, o = 0;
-        PRG_CUDA(cudaGetDevice(&dev));
-        PRG_CUDA(cudaDeviceGetAttribute(&o, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        optin = o;
-        PRG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    }
+    const DeviceLimits &d = device_limits();
     nb = (unsigned)std::max<uint64_t>(
-        1, std::min<uint64_t>(std::min<unsigned>(sms, kResBlocks), (arcs + (uint64_t)res_alpha(0) * n) / kResMinShare));
-    return std::min(kResSmem, (size_t)optin - kResStatic);
+        1, std::min<uint64_t>(std::min<unsigned>(d.sms, kResBlocks), (arcs + (uint64_t)res_alpha(0) * n) / kResMinShare));
+    return std::min(kResSmem, (size_t)d.smem_optin - kResStatic);
 }
 
 // Most 8-arc chunks of a block's share.

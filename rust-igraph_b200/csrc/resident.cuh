@@ -17,6 +17,12 @@ enum ResKind : int {
     RES_EIG = 1,    // max-normalised iteration x' = (shift I + A) x / max
 };
 
+// Read once, by whichever thread comes first.
+struct DeviceLimits {
+    int sms = 0, smem_optin = 0;
+};
+const DeviceLimits &device_limits();
+
 struct ResPlan {
     unsigned grid = 0;   // 0: the graph does not fit, use the other kernels
     size_t smem = 0;     // dynamic shared memory per block

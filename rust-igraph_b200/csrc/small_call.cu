@@ -361,15 +361,9 @@ SmallStatus small_call(const SmallCall &c, double *out, SmallResult &r, cudaStre
     if (!res_sizes_fit(n, arcs, c.w != nullptr, c.kind)) return SMALL_NOT_HERE;
     // without a blind plan the iteration is planned once the rows are known
     const ResPlan p = res_plan_blind(n, arcs, c.w != nullptr, c.kind);
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        PRG_CUDA(cudaGetDevice(&dev));
-        PRG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    }
     PRG_CUDA(cudaFuncSetAttribute(small_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem));
     // few arcs need few blocks: a barrier over fewer is shorter
-    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(sms, (arcs + n) / 2048));
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(device_limits().sms, (arcs + n) / 2048));
 
     // scratch: first what must be zero, then the rest
     size_t at = 0;
