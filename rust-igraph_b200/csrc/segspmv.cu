@@ -1117,7 +1117,10 @@ LaunchCfg seg_config(const DeviceGraph &g, uint32_t hot_entries, int variant, in
     else if (res) seg8_pick<Plain64Pass>(c.hot != 0, c.threads, c.seg_pipe, c.seg_w, &k);
     else if (c.seg == 2) seg8_pick<Kry32Pass>(c.hot != 0, c.threads, c.seg_pipe, c.seg_w, &k);
     else k = c.hot ? (const void *)kry32_seg_kernel<true> : (const void *)kry32_seg_kernel<false>;
-    PRG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem));
+    // the attribute belongs to the kernel, which graphs of other sizes launch too: always the limit
+    constexpr int most = (int)((kSegNT / 32) * kSegTile + kSegHotMax) * (int)sizeof(float);
+    static_assert(most == (int)((kSegNT / 32) * kSegTile + kSegHotMax64) * (int)sizeof(double), "both value types");
+    PRG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     c.seg_g1 = (unsigned)sms;
     c.seg_g2 = (unsigned)sms * 4u;
     c.grid = c.seg_g1 + c.seg_g2;  // block records the consumers add

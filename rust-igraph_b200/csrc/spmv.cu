@@ -31,6 +31,7 @@
 #include <algorithm>
 
 #include "prims.cuh"
+#include "resident.cuh"
 #include "spmv.cuh"
 
 namespace prg {
@@ -552,30 +553,25 @@ __global__ void __launch_bounds__(NT, NT != kThreads ? 1 : HOT ? (kIs32<MODE> ? 
 template <int MODE, bool W, bool HOT, int NT>
 static void kernel_config(uint32_t hot_entries, uint32_t blocks_per_sm, uint32_t n, LaunchCfg &c) {
     using A = typename ModeT<MODE>::A;
-    static int sms = 0, smem_optin = 0;
-    if (sms == 0) {
-        int dev = 0;
-        PRG_CUDA(cudaGetDevice(&dev));
-        PRG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        PRG_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    }
+    const DeviceLimits &dev = device_limits();
+    const size_t most = (size_t)dev.smem_optin - 2048;  // leaves the kernel's static shared memory (reduction scratch)
     const size_t bufs = (size_t)(NT / 32) * kWarpBuf * sizeof(A);
     size_t hot = 0;
     if (HOT) {
-        // leave room for the kernel's static shared memory (reduction scratch)
-        const size_t avail = ((size_t)smem_optin - bufs - 2048) / sizeof(A);
+        const size_t avail = (most - bufs) / sizeof(A);
         hot = std::min<size_t>(std::min<size_t>(hot_entries, avail), n) & ~(size_t)3;
     }
     c.smem = bufs + hot * sizeof(A);
     c.hot = (uint32_t)hot;
     c.threads = NT;
+    // the attribute belongs to the kernel, which graphs of other sizes launch too: always the limit
     PRG_CUDA(cudaFuncSetAttribute(iter_kernel<MODE, W, HOT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)c.smem));
+                                  (int)most));
     int occ = 0;
     PRG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, iter_kernel<MODE, W, HOT, NT>, NT, c.smem));
     int per = occ > 0 ? occ : 1;
     if (blocks_per_sm > 0 && (int)blocks_per_sm < per) per = (int)blocks_per_sm;
-    c.grid = (unsigned)(sms * per);
+    c.grid = (unsigned)(dev.sms * per);
 }
 
 template <int MODE, bool W>
