@@ -47,7 +47,7 @@ enum prg_status {
     PRG_ERR_CUDA = 4,                 /* IgraphError::Internal("cuda: ...") */
     PRG_ERR_OUT_OF_MEMORY = 5,        /* IgraphError::Internal("cuda: out of memory") */
     PRG_ERR_DID_NOT_CONVERGE = 6,     /* IgraphError::DidNotConverge (never raised by the drop-ins) */
-    PRG_ERR_TIMEOUT = 7,              /* a bounded device wait expired (batched solver) */
+    PRG_ERR_TIMEOUT = 7,              /* a bounded device wait expired (batched solver, block-resident iterations) */
     PRG_ERR_PARSE = 8,                /* IgraphError::Parse { line, message } */
     PRG_ERR_IO = 9,                   /* IgraphError::Io (the text is not valid UTF-8) */
     PRG_ERR_UNSUPPORTED = 10          /* IgraphError::Unsupported(&'static str) */
@@ -352,7 +352,9 @@ int32_t prg_autotune(prg_graph *g, int32_t tune_batch, const char *cache_path, p
  * "batch_barrier_extra" (failure-detection test hook, 0 or 1: with 1 every
  * grid barrier of the batched solver waits for an arrival that never comes,
  * so its bounded wait (about 1.5 s) expires and the call returns
- * PRG_ERR_TIMEOUT with the context still usable; leave it 0). */
+ * PRG_ERR_TIMEOUT with the context still usable; leave it 0),
+ * "resident_barrier_extra" (the same for the block-resident iterations, 1, and
+ * the small-graph build of the drop-ins, 2; leave it 0). */
 int32_t prg_set_tuning(const char *key, int64_t value);
 
 /* ---- batched personalized PageRank ---------------------------------- */

@@ -1503,6 +1503,9 @@ int32_t prg_set_tuning(const char *key, int64_t value) {
     } else if (k == "batch_cheb") {
         if (value != 0 && value != 1) return fail(PRG_ERR_INVALID_ARGUMENT, "batch_cheb must be 0 or 1");
         t.batch_cheb = (uint32_t)value;
+    } else if (k == "resident_barrier_extra") {
+        if (value > 2) return fail(PRG_ERR_INVALID_ARGUMENT, "resident_barrier_extra must be 0, 1 or 2");
+        t.resident_barrier_extra = (uint32_t)value;
     } else if (k == "batch_barrier_extra") {
         if (value > 1) return fail(PRG_ERR_INVALID_ARGUMENT, "batch_barrier_extra must be 0 or 1");
         t.batch_barrier_extra = (uint32_t)value;

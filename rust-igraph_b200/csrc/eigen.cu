@@ -576,6 +576,15 @@ Result eigenvector_centrality(const DeviceGraph &g, Workspace &ws, double *d_out
     State *d_st = alloc<State>(1, s), *h_st = nullptr;
     static_assert(2 * sizeof(State) <= kSlabBytes, "iteration state slab");
     h_st = static_cast<State *>(pinned_acquire());
+    auto free_all = [&]() {
+        pinned_release(h_st);
+        release(x[0], s);
+        release(x[1], s);
+        release(recs, s);
+        release(part, s);
+        release(pvrec, s);
+        release(d_st, s);
+    };
     try {
         State init;
         std::memset(&init, 0, sizeof(init));
@@ -625,16 +634,10 @@ Result eigenvector_centrality(const DeviceGraph &g, Workspace &ws, double *d_out
         PRG_CUDA(cudaStreamSynchronize(s));
     } catch (...) {
         cudaStreamSynchronize(s);
-        pinned_release(h_st);
+        free_all();
         throw;
     }
-    pinned_release(h_st);
-    release(x[0], s);
-    release(x[1], s);
-    release(recs, s);
-    release(part, s);
-    release(pvrec, s);
-    release(d_st, s);
+    free_all();
     PRG_CUDA(cudaStreamSynchronize(s));
     return r;
 }

@@ -130,6 +130,7 @@ struct Tuning {
     double krylov_rel = 1e-4;
     double krylov_floor = 0.7;         // refined / Krylov inner solves aim at this fraction of the final threshold
     uint32_t batch_barrier_extra = 0;  // test hook: batched grid barriers wait for arrivals that never come
+    uint32_t resident_barrier_extra = 0;  // the same for the barriers of resident.cu (1) and small_call.cu (2)
     uint32_t batch_cheb = 0;           // batched solver on undirected graphs: 1 Chebyshev steps, 0 plain steps
 };
 Tuning &tuning();

@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(kResNT, 1) res_kernel(const ResArgs a) {
                 int ok = 1;
                 __stcg(rec + blk, make_double2(v0, v1));
                 red_release(a.bar, 1u);
-                const uint32_t target = (phase + 1u) * nb;
+                const uint32_t target = (phase + 1u) * nb + a.bar_extra;
                 for (uint32_t spins = 0; ld_acquire(a.bar) < target;) {
                     if (++spins > kResSpins) {
                         a.ctl->status = 7;  // PRG_ERR_TIMEOUT
@@ -777,7 +777,9 @@ static bool res_go(const ResPlan &p, const ResArgs &a, cudaStream_t s) {
     return true;
 }
 
-bool launch_resident(int kind, const ResPlan &p, const ResArgs &a, cudaStream_t s) {
+bool launch_resident(int kind, const ResPlan &p, const ResArgs &args, cudaStream_t s) {
+    ResArgs a = args;
+    a.bar_extra = tuning().resident_barrier_extra == 1u ? 1u : 0u;
     const bool w = a.w64 != nullptr;
     if (kind == RES_EIG) {
         if (p.stream) return w ? res_go<RES_EIG, true, true>(p, a, s) : res_go<RES_EIG, false, true>(p, a, s);

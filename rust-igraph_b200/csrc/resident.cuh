@@ -50,6 +50,7 @@ struct ResArgs {
     const uint32_t *longest;
     uint32_t smem;
     uint32_t n, alpha, max_iter;
+    uint32_t bar_extra;   // test hook: arrivals every barrier waits for beyond the grid's
     uint32_t l1hot;       // sources at or above this id are gathered without L1 allocation
     double damping, thr, shift;
 };

@@ -62,6 +62,7 @@ struct SmallArgs {
     const uint32_t *from, *to;
     const double *w;
     uint32_t n, m, longest;  // longest: of a row
+    uint32_t bar_extra;      // test hook: arrivals a barrier waits for beyond the grid's
     int directed, check_w, seed;  // seed 0: none, 1: ones, 2: dval / max dval (ones when that is 0)
     SmallSide in, outs;      // outs only for weighted directed graphs
     uint32_t *deg;           // directed, unweighted: out-degrees, zero at launch
@@ -85,7 +86,7 @@ __device__ bool small_barrier(const SmallArgs &a, uint32_t &phase) {
         uint32_t seen = 0;
         for (uint32_t spins = 0;;) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.word + 2) : "memory");
-            if (seen >= phase * gridDim.x) break;
+            if (seen >= phase * gridDim.x + a.bar_extra) break;
             if (++spins > kSmallSpins) {
                 a.ctl->status = 7;  // PRG_ERR_TIMEOUT
                 ok = 0;
@@ -412,6 +413,7 @@ SmallStatus small_call(const SmallCall &c, double *out, SmallResult &r, cudaStre
         a.n = n;
         a.m = (uint32_t)c.m;
         a.longest = res_longest_row(n, arcs);
+        a.bar_extra = tuning().resident_barrier_extra == 2u ? 1u : 0u;
         a.directed = c.directed ? 1 : 0;
         a.check_w = c.w && c.check_weights ? 1 : 0;
         a.seed = c.kind == RES_EIG ? (c.strength_seed ? 2 : 1) : 0;
