@@ -91,12 +91,12 @@ def test_long_rows_do_not_hold_up_one_block(cuda_ok, longest, resident, weighted
     assert any("seg8_kernel" in k for k in names) != resident
 
 
-@pytest.mark.parametrize("kind", CALLS)
-@pytest.mark.parametrize("m,longest", [(100_000, 99_000), (600_000, 90_000), (1_500_000, 700_000), (9_000_000, 400_000)])
+LONG = [(100_000, 99_000), (600_000, 90_000), (1_500_000, 700_000)]
+
+
+@pytest.mark.parametrize("kind,m,longest", [(k, *r) for k in CALLS for r in LONG] + [("pagerank", 9_000_000, 400_000)])
 def test_long_rows_upload_once(cuda_ok, kind, m, longest, tmp_path):
     # rows no plan holds, found in the build (or, with few edges a thread, by the plan)
-    if kind != "pagerank" and m > 5_000_000:
-        pytest.skip("more than 10 M arcs, or a long call")
     n = 60_000
     f, t = hub_graph(n, m, longest)
     directed = not kind.startswith("eigen")
