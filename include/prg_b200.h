@@ -335,10 +335,10 @@ int32_t prg_autotune(prg_graph *g, int32_t tune_batch, const char *cache_path, p
  * "seg_plain64" (1 the tile-segmented FP64 power step of
  * the drop-ins and the certified FP64 loop, and the FP64 Krylov matvec of
  * the FP64 Krylov and pagerank_linsys solves; 0 the row-block kernel),
- * "resident" (graphs whose arcs fit the SMs' shared memory, unless
- * "seg_plain64" / "seg_eig64" ask for the row-block kernel: 1 the FP64 power
- * and eigenvector iterations as one persistent launch, the default; 0 one
- * launch sequence per iteration),
+ * "resident" (graphs of up to 10 M arcs whose rows spread evenly enough over
+ * the SMs, unless "seg_plain64" / "seg_eig64" ask for the row-block kernel: 1
+ * the FP64 power and eigenvector iterations as one persistent launch, the
+ * default; 0 one launch sequence per iteration),
  * "seg_prefetch" (segmented passes:
  * 1 each warp prefetches its next tile of column indices into L2, 0 off),
  * "seg_threads" (their tile kernel's block size, one block per SM: 1024, 768
@@ -363,7 +363,7 @@ typedef struct prg_batch_stats {
     uint64_t column_iterations; /* sum over columns of the iterations each ran */
     uint32_t max_iters;         /* iterations of the slowest column */
     uint32_t tiles;             /* column tiles (one persistent launch each) */
-    uint32_t tile_width;        /* columns per tile (32 * vec) */
+    uint32_t tile_width;        /* columns per full tile (32 * vec; the last tile may run in a narrower kernel) */
     uint32_t kernel_launches;
     double ms;                  /* device time (CUDA events) */
     uint32_t chebyshev;         /* 1: Chebyshev steps (undirected graph), 0: plain power steps */

@@ -1183,7 +1183,7 @@ int32_t prg_graph_matvec32(prg_graph *h, int32_t kernel, const float *d_p, const
     if (!h) return fail(PRG_ERR_INVALID_ARGUMENT, "null graph handle");
     if (kernel < 0 || kernel > 2) return fail(PRG_ERR_INVALID_ARGUMENT, "kernel must be 0, 1 or 2");
     if (kernel != 0 && h->g.weighted)
-        return fail(PRG_ERR_UNSUPPORTED, "the tile-segmented matvec serves unweighted graphs");
+        return fail(PRG_ERR_UNSUPPORTED, "kernels 1 and 2 of this probe take unweighted graphs");
     if (!(damping >= 0.0 && damping <= 1.0)) return fail(PRG_ERR_INVALID_ARGUMENT, "damping must be in [0, 1]");
     if (h->g.n == 0 || h->g.arcs == 0) return fail(PRG_ERR_INVALID_ARGUMENT, "the graph has no arcs");
     if (!d_p || !d_pt || !d_y) return fail(PRG_ERR_INVALID_ARGUMENT, "null vector");

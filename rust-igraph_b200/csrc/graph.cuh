@@ -55,8 +55,8 @@ struct DeviceGraph {
     uint32_t seg_plain64 = 1;
     // ... and the adjacency product of the eigenvector and HITS iterations
     uint32_t seg_eig64 = 1;
-    // graphs whose arcs fit the SMs' shared memory: FP64 power and eigenvector
-    // iterations as one persistent launch (resident.cu)
+    // graphs of up to 10 M arcs, no block's share too large: FP64 power and
+    // eigenvector iterations as one persistent launch (resident.cu)
     uint32_t resident = 1;
     uint32_t seg_prefetch = 1;  // segmented passes: prefetch each warp's next index tile into L2
     // their tile kernel: threads of its one block per SM (1024, 768 or 512)

@@ -391,13 +391,13 @@ __global__ void __launch_bounds__(kBThreads) ppr_tile_kernel(const TileArgs a) {
                         const Vec<VEC> g1 = ldv_cg<VEC>(XT + (size_t)u1 * W + lane * VEC);
                         const Vec<VEC> g2 = ldv_cg<VEC>(XT + (size_t)u2 * W + lane * VEC);
                         const Vec<VEC> g3 = ldv_cg<VEC>(XT + (size_t)u3 * W + lane * VEC);
-    #pragma unroll
+#pragma unroll
                         for (int j = 0; j < VEC; j++) kahan_add(acc[j], cmp[j], (g0.v[j] + g1.v[j]) + (g2.v[j] + g3.v[j]));
                     }
                     for (; k < cnt; k++) {
                         const uint32_t u = __shfl_sync(0xffffffffu, mine, k);
                         const Vec<VEC> g = ldv_cg<VEC>(XT + (size_t)u * W + lane * VEC);
-    #pragma unroll
+#pragma unroll
                         for (int j = 0; j < VEC; j++) kahan_add(acc[j], cmp[j], g.v[j]);
                     }
                 }

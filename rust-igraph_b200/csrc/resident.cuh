@@ -1,5 +1,5 @@
 // resident.cuh — launch interface of the block-resident persistent iteration
-// (resident.cu) for graphs whose arcs fit the SMs' shared memory.
+// (resident.cu) for graphs of up to kResMaxArcs arcs.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -14,7 +14,8 @@
 //   * in each lane, a running sum over its 4 arcs that restarts after a row end;
 //   * across the 32 lanes, an inclusive scan of the lanes' open tails (5
 //     shuffles) whose segment breaks come from one ballot of "lane holds a
-//     row end", with no flag shuffles;
+//     row end", with no flag shuffles (the 8-arc kernel takes differences of
+//     one unbroken scan on unweighted graphs, see its cross-lane step);
 //   * the k-th row end of tile t belongs to nz_row[tile_j0[t] + k] (the rows
 //     that have arcs, in order); its sum goes to the warp's shared buffer at
 //     rank k, and the epilogues then run with lane i on rank i, so the loads
@@ -775,7 +776,7 @@ struct Plain64Pass {
 // Weighted graphs (W) multiply each gathered value by its arc's weight, streamed
 // beside the index (w64 or w32, 64 or 32 bytes per lane).  FP64 power step with
 // its finishing kernel against the row-block kernel: power law of 2 M vertices
-// and 17 M arcs 113 against 177 us, R-MAT scale 20 84 against 201 us.
+// and 17 M arcs 117 against 175 us, R-MAT scale 20 85 against 213 us.
 constexpr int kArcless = 2;  // rows without arcs a lane loads ahead (four spill)
 
 // Whether the tile kernel takes the rows without arcs of a dense numbering.  The

@@ -148,9 +148,8 @@ __global__ void __launch_bounds__(kSmallNT, 1) small_build_kernel(const SmallArg
     // 1: slots.  A row too long for any plan ends the phase: its arcs' atomics on
     // one word and its sort by one block would be in vain (a row of 5 M arcs held
     // a call up by 20 ms).  A slot is looked at one step later, when it has arrived,
-    // and the word that says so at every fourth (1 M arcs 0.79 ms a call, at every
-    // step 0.81; one row of 5 M arcs 3.5
-    // and 3.3, the general path alone 3.1).
+    // and the word that says so at every fourth (1 M arcs 0.77 ms a call, at every
+    // step 0.79; one row of 5 M arcs 3.5 and 3.3, the general path alone 3.1).
     {
         uint32_t mx = 0, bad = 0, s0 = 0, s1 = 0, step = 0;
         uint32_t *too_long = a.word + 8;
