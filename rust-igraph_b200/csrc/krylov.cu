@@ -41,11 +41,14 @@
 namespace prg {
 
 struct KState {
-    double rho[2], alpha[2], omega[2], rhh[2];  // by step parity
+    // By step parity: a kernel's first blocks may be done before its last ones
+    // start, so what it reads of a step it must not write.
+    double rho[2], alpha[2], omega[2], rhh[2];
+    double best[2];    // smallest ||r|| so far (stagnation guard)
+    uint32_t stall[2]; // consecutive steps without a 2x gain over the best ||r||
     double rel;        // inner stop: ||r|| <= max(rel * ||r0||, floor_abs)
     double floor_abs;
     double near;       // rel * ||r0|| below near: aim for floor_abs in this solve
-    double best;       // smallest ||r|| so far (stagnation guard)
     double tol;        // set by the first V1 from ||r0||
     double rnorm;      // last residual norm V1 saw
     double r0norm;
@@ -54,7 +57,6 @@ struct KState {
     int32_t done;      // KDONE_*
     int32_t norm2;     // 0: L1 norms, 1: 2-norms
     uint32_t restarts;
-    uint32_t stall;    // consecutive steps without a 2x gain over the best ||r||
     uint32_t half;     // 1: the solve ended at a half step (the last step ran one matvec)
 };
 
@@ -302,6 +304,10 @@ __global__ void __launch_bounds__(kVT) kv1(uint32_t n, int q, KState *st, const 
                                            T *p, T *pt, const T *v, const float *inv32, const double *dval,
                                            double4 *part1) {
     if (kstopped(st)) return;
+    if (st->half) {  // the step before met the target (kv3)
+        if (kleader()) st->done = KDONE_CONVERGED;
+        return;
+    }
     const double3 red = krecords(part5, gridDim.x, nullptr, 0);
     const double rhr = red.x, rn1 = red.y, rr = red.z;
     const uint32_t k = st->count;
@@ -333,8 +339,9 @@ __global__ void __launch_bounds__(kVT) kv1(uint32_t n, int q, KState *st, const 
         return;
     }
     // stagnation: kStallSteps steps in a row without halving the best norm
-    const double best = k == 0 ? norm : st->best;
-    const uint32_t stall = k == 0 ? 0u : (norm < 0.5 * best ? 0u : st->stall + 1u);
+    const int o = q ^ 1;
+    const double best = k == 0 ? norm : st->best[o];
+    const uint32_t stall = k == 0 ? 0u : (norm < 0.5 * best ? 0u : st->stall[o] + 1u);
     if (stall >= kStallSteps) {
         if (kleader()) {
             st->rnorm = norm;
@@ -342,7 +349,6 @@ __global__ void __launch_bounds__(kVT) kv1(uint32_t n, int q, KState *st, const 
         }
         return;
     }
-    const int o = q ^ 1;
     const double om = k ? st->omega[o] : 0.0, rho0 = k ? st->rho[o] : 0.0, al = k ? st->alpha[o] : 0.0;
     const double rhh = k ? st->rhh[o] : rr;
     // restart (rh = r) when the shadow residual has become nearly orthogonal
@@ -383,8 +389,8 @@ __global__ void __launch_bounds__(kVT) kv1(uint32_t n, int q, KState *st, const 
         st->rho[q] = restart ? rr : rhr;
         st->rhh[q] = restart ? rr : rhh;
         st->rnorm = norm;
-        st->best = fmin(best, norm);
-        st->stall = stall;
+        st->best[q] = fmin(best, norm);
+        st->stall[q] = stall;
         if (write_rh) st->restarts += 1u;
     }
 }
@@ -434,7 +440,7 @@ __global__ void __launch_bounds__(kVT) kv2(uint32_t n, int q, KState *st, const 
 // V3: omega = (t.s)/(t.t); e += alpha p + omega s; r = s - omega t;
 // records (rh.r, |r|_1, r.r) for the next V1.  When M2 skipped (its marker
 // part4[0].w = 1: ||s|| met the target), the step ends at its half:
-// e += alpha p and the solve is converged.
+// e += alpha p and the solve is converged; the next kernel raises done.
 template <class T>
 __global__ void __launch_bounds__(kVT) kv3(uint32_t n, int q, KState *st, const double4 *part4, uint32_t n4,
                                            const double4 *hub_rec, uint32_t nhub, const double4 *part3,
@@ -459,8 +465,7 @@ __global__ void __launch_bounds__(kVT) kv3(uint32_t n, int q, KState *st, const 
             if (threadIdx.x == 0) {
                 st->rnorm = st->norm2 ? sqrt(sr.z) : sr.y;
                 st->count += 1u;
-                st->half = 1u;
-                st->done = KDONE_CONVERGED;
+                st->half = 1u;  // not done: blocks that start later must still add their part
             }
         }
         return;
@@ -613,7 +618,7 @@ static InnerResult bicgstab(const DeviceGraph &g, Workspace &ws, KrylovWs &k, KB
         if (batch > 0) {
             const int prev = slot ^ 1;
             PRG_CUDA(cudaEventSynchronize(k.ev[prev]));
-            if (k.h_st[prev].done != KRUN) stop = true;
+            if (k.h_st[prev].done != KRUN || k.h_st[prev].half) stop = true;
         }
         if (++batch >= max_batches) stop = true;
         PRG_CUDA(cudaGetLastError());
@@ -638,7 +643,7 @@ static InnerResult bicgstab(const DeviceGraph &g, Workspace &ws, KrylovWs &k, KB
             gap_ms += gp;
         }
     }
-    res.done = k.h_st[0].done;
+    res.done = k.h_st[0].half ? KDONE_CONVERGED : k.h_st[0].done;
     res.rnorm = k.h_st[0].rnorm;
     res.half = k.h_st[0].half;
     if (std::getenv("PRG_TRACE"))
