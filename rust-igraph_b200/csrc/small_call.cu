@@ -46,7 +46,6 @@ constexpr uint32_t kSmallRange = 1u << 20;           // ids per bitmap of the bl
 __host__ __device__ constexpr uint32_t small_word(uint32_t i) { return i + (i >> 5); }
 constexpr size_t kSmallSmem = small_word(kSmallRange / 32) * 4;  // also 32 warp buffers
 constexpr uint32_t kSmallSpins = 1u << 21;
-constexpr size_t kSmallJoint = 8 << 20;
 static_assert(kSmallSmem >= (size_t)(kSmallNT / 32) * kSmallWarpBuf * 4, "warp buffers");
 
 struct SmallSide {
@@ -368,7 +367,7 @@ SmallStatus small_call(const SmallCall &c, double *out, SmallResult &r, cudaStre
     // few arcs need few blocks: a barrier over fewer is shorter
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(device_limits().sms, (arcs + n) / 2048));
 
-    // scratch: first what must be zero, then the rest
+    // one allocation: first what must be zero, then the rest
     size_t at = 0;
     auto take = [&](size_t bytes) {
         const size_t o = at;
@@ -377,41 +376,35 @@ SmallStatus small_call(const SmallCall &c, double *out, SmallResult &r, cudaStre
     };
     const size_t o_ctl = take(sizeof(Ctl)), o_word = take(64), o_bar = take(4), o_cnt = take(n * 4ull),
                  o_deg = take(c.directed && !c.w ? n * 4ull : 4), o_cnt2 = take(two ? n * 4ull : 4), zeroed = at;
-    const size_t o_slot = take(arcs * 4), o_ptr = take((n + 1ull) * 4), o_ids = take(arcs * 4), o_bs = take(grid * 4ull),
+    const size_t o_from = take(c.m * 4), o_to = take(c.m * 4), o_w = take(c.w ? c.m * 8 : 8),
+                 o_slot = take(arcs * 4), o_ptr = take((n + 1ull) * 4), o_ids = take(arcs * 4), o_bs = take(grid * 4ull),
                  o_long = take(n * 4ull), o_slot2 = take(two ? arcs * 4 : 4), o_ptr2 = take(two ? (n + 1ull) * 4 : 4),
                  o_ids2 = take(two ? arcs * 4 : 4), o_bs2 = take(grid * 4ull), o_long2 = take(two ? n * 4ull : 4),
                  o_col = take((arcs + kColPad) * 4), o_w64 = take(c.w ? (arcs + kColPad) * 8 : 8), o_dval = take(n * 8ull),
                  o_x = take(n * 8ull), o_t = take(c.reset ? n * 8ull : 8), o_xt0 = take(n * 8ull), o_xt1 = take(n * 8ull),
                  o_rec = take(res_scratch_bytes(kResBlocks));
-    // The edge list may outlive the rest, so it is an allocation of its own where
-    // the rest would be missed (a second allocation takes 3 us).
-    const size_t ids = (c.m * 4 + 255) & ~(size_t)255, edges = 2 * ids + (c.w ? c.m * 8 : 0);
-    const bool joint = at <= kSmallJoint;
-    unsigned char *b = nullptr, *eb = nullptr;
+    unsigned char *b = nullptr;
     Ctl *h = static_cast<Ctl *>(pinned_acquire());
     SmallStatus status = SMALL_DONE;
     auto give_up = [&]() {
         cudaStreamSynchronize(s);
         if (b) cudaFreeAsync(b, s);
-        if (eb && !joint) cudaFreeAsync(eb, s);
         pinned_release(h);
     };
     try {
-        PRG_CUDA(cudaMallocAsync((void **)&b, joint ? at + edges : at, s));
-        if (joint) eb = b + at;
-        else PRG_CUDA(cudaMallocAsync((void **)&eb, edges, s));
+        PRG_CUDA(cudaMallocAsync((void **)&b, at, s));
         PRG_CUDA(cudaMemsetAsync(b, 0, zeroed, s));
-        PRG_CUDA(cudaMemcpyAsync(eb, c.from, c.m * 4, cudaMemcpyHostToDevice, s));
-        PRG_CUDA(cudaMemcpyAsync(eb + ids, c.to, c.m * 4, cudaMemcpyHostToDevice, s));
-        if (c.w) PRG_CUDA(cudaMemcpyAsync(eb + 2 * ids, c.w, c.m * 8, cudaMemcpyHostToDevice, s));
+        PRG_CUDA(cudaMemcpyAsync(b + o_from, c.from, c.m * 4, cudaMemcpyHostToDevice, s));
+        PRG_CUDA(cudaMemcpyAsync(b + o_to, c.to, c.m * 4, cudaMemcpyHostToDevice, s));
+        if (c.w) PRG_CUDA(cudaMemcpyAsync(b + o_w, c.w, c.m * 8, cudaMemcpyHostToDevice, s));
         if (c.reset) PRG_CUDA(cudaMemcpyAsync(b + o_t, c.reset, n * 8ull, cudaMemcpyHostToDevice, s));
         auto u32 = [&](size_t o) { return reinterpret_cast<uint32_t *>(b + o); };
         auto f64 = [&](size_t o) { return reinterpret_cast<double *>(b + o); };
         SmallArgs a;
         std::memset(&a, 0, sizeof(a));
-        a.from = reinterpret_cast<uint32_t *>(eb);
-        a.to = reinterpret_cast<uint32_t *>(eb + ids);
-        a.w = c.w ? reinterpret_cast<double *>(eb + 2 * ids) : nullptr;
+        a.from = u32(o_from);
+        a.to = u32(o_to);
+        a.w = c.w ? f64(o_w) : nullptr;
         a.n = n;
         a.m = (uint32_t)c.m;
         a.longest = res_longest_row(n, arcs);
@@ -510,15 +503,24 @@ SmallStatus small_call(const SmallCall &c, double *out, SmallResult &r, cudaStre
         throw;
     }
     if (status == SMALL_NOT_HERE) {
-        r.edges.block = joint ? b : eb;
-        r.edges.from = reinterpret_cast<uint32_t *>(eb);
-        r.edges.to = reinterpret_cast<uint32_t *>(eb + ids);
-        r.edges.w = c.w ? reinterpret_cast<double *>(eb + 2 * ids) : nullptr;
-        if (!joint) cudaFreeAsync(b, s);
-    } else {
-        cudaFreeAsync(b, s);
-        if (!joint) cudaFreeAsync(eb, s);
+        // the edge list in an allocation of its own: the general path should not
+        // have to do without the rest of this one (nor, where even that fails,
+        // without anything: it uploads again)
+        const size_t ids = (c.m * 4 + 255) & ~(size_t)255, wb = c.w ? c.m * 8 : 0;
+        unsigned char *eb = nullptr;
+        if (cudaMallocAsync((void **)&eb, 2 * ids + wb, s) == cudaSuccess) {
+            cudaMemcpyAsync(eb, b + o_from, c.m * 4, cudaMemcpyDeviceToDevice, s);
+            cudaMemcpyAsync(eb + ids, b + o_to, c.m * 4, cudaMemcpyDeviceToDevice, s);
+            if (c.w) cudaMemcpyAsync(eb + 2 * ids, b + o_w, wb, cudaMemcpyDeviceToDevice, s);
+            r.edges.block = eb;
+            r.edges.from = reinterpret_cast<uint32_t *>(eb);
+            r.edges.to = reinterpret_cast<uint32_t *>(eb + ids);
+            r.edges.w = c.w ? reinterpret_cast<double *>(eb + 2 * ids) : nullptr;
+        } else {
+            cudaGetLastError();
+        }
     }
+    cudaFreeAsync(b, s);
     pinned_release(h);
     return status;
 }
